@@ -105,14 +105,9 @@ static int log2_brick(int b) {
   }
 }
 
-// Map-build work items of one request: kBatchChunk vertex slots each, in rows or bricks.
+// Map-build work items of one request: kBatchChunk vertex slots each, in rows or along the light.
 static int k1_items(const ExactGeo& g, int bl) {
-  long long slots = (long long)g.pd[0] * g.pd[1] * g.pd[2];
-  if (bl) {
-    const long long nb = (long long)((g.pd[0] + (1 << bl) - 1) >> bl) * ((g.pd[1] + (1 << bl) - 1) >> bl) *
-                         ((g.pd[2] + (1 << bl) - 1) >> bl);
-    slots = nb << (3 * bl);
-  }
+  const long long slots = bl ? (long long)light_slots(g, bl) : (long long)g.pd[0] * g.pd[1] * g.pd[2];
   return (int)((slots + kBatchChunk - 1) / kBatchChunk);
 }
 

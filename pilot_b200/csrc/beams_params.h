@@ -43,17 +43,16 @@ struct ExactGeo {
   int ax_off[3];   // offset of field axis d in the table
   int max_off[3];  // offset of map axis d in the table
   int ntab;        // total table entries
-  // K1 vertex order: 0 = x-fastest rows of the vertex grid; b > 0 = cubic
-  // bricks of 2^b vertices per edge in brick order (rays in flight stay in a
-  // narrow cone towards the light, so the field they read stays in L2).
+  // K1 vertex order: 0 = x-fastest rows of the vertex grid; b > 0 = columns
+  // along the light in bricks of 2^b vertices per edge (light_slot_vertex): the
+  // rays in flight stay in a narrow corridor towards the light, so the field
+  // they read stays in L2, and a warp's rays run side by side.
   int light_brick_log2;
-  // Brick order that follows the light: bricks are visited in pencils along
-  // bo_axis[0] (the axis the light travels most along, in map-vertex units),
-  // the two other brick coordinates (bo_axis[1], bo_axis[2]) sheared by
-  // floor(w * bo_shear / 65536) modulo their brick counts, so that a pencil
-  // tracks the light rays through the brick grid; pencils in raster order.
-  // The bricks in flight then sit in a few adjacent pencils and their light
-  // rays cross one narrow region of the field. Any order gives the same map.
+  // That order's axes: columns run along bo_axis[0] (the axis the light travels
+  // most along, in map-vertex units), the two other coordinates (bo_axis[1],
+  // bo_axis[2]) sheared by floor(w * bo_shear / 65536) modulo their counts, so
+  // that a column tracks a light ray through the vertex grid. Any order gives
+  // the same map.
   int bo_axis[3];
   int bo_shear[2];
   // Occupancy of 8^3-cell macro-cells (empty-space skipping): counts per axis.
@@ -119,6 +118,18 @@ struct Counters {
   unsigned int tiles_mark;  // the map-cell marking pass's tile counter (zeroed by its launcher)
   unsigned int reserved;
 };
+
+// Slots of the light-aligned vertex order with groups of 2^bl x 2^bl columns
+// (light_slot_vertex): every vertex once, plus the padding columns of the last
+// groups.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline unsigned light_slots(const ExactGeo& g, int bl) {
+  const unsigned pad = (1u << bl) - 1u;
+  return (unsigned)g.pd[g.bo_axis[0]] * (((unsigned)g.pd[g.bo_axis[1]] + pad) & ~pad) *
+         (((unsigned)g.pd[g.bo_axis[2]] + pad) & ~pad);
+}
 
 // Derives ExactGeo's loop constants from n[] and tf_n.
 inline void geo_loop_constants(ExactGeo& g) {

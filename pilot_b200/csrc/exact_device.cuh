@@ -466,8 +466,8 @@ __device__ __forceinline__ void map_light_sum(const ExactGeo& g, const float4* M
   }
 }
 
-// Shared-memory form of the light-aligned brick order for bricks of 2^bl
-// vertices per edge: {nb_w, nb_u, nb_v, axis_w, axis_u, axis_v, shear_u, shear_v}.
+// Shared-memory form of the marked-vertex listing's brick order, bricks of
+// 2^bl vertices per edge: {nb_w, nb_u, nb_v, axis_w, axis_u, axis_v, shear_u, shear_v}.
 __device__ __forceinline__ void brick_order_setup(const ExactGeo& g, int bl, int* s_bo) {
   int nb[3];
 #pragma unroll
@@ -494,6 +494,50 @@ __device__ __forceinline__ void pencil_brick(int bi, const int* s_bo, int& bx, i
   bx = aw == 0 ? w : (au == 0 ? u : v);
   by = aw == 1 ? w : (au == 1 ? u : v);
   bz = aw == 2 ? w : (au == 2 ? u : v);
+}
+
+// The map build's vertex order. Columns of vertices run along w, the axis the
+// light travels most along, and follow the light: column (u, v) holds at w the
+// vertex (u + floor(w shear_u), v + floor(w shear_v)) modulo the grid, so every
+// vertex is in exactly one column. Columns go in groups of E x E (E = 2^bl),
+// groups in raster order; inside a group chunks of E along w, inside a chunk
+// 2 x 2-column bundles, inside a bundle w, then the four columns. 32
+// consecutive slots are then about 8 vertices along the light by 2 by 2 across:
+// their rays run within a map cell or two of one another, so a warp's 32
+// samples fall into few cells and its loads into few lines (the light march of
+// a 512^3 field with the light along z read 20 lines per load as 8 x 4 vertices
+// in the x, y plane). Slots of columns past the grid hold no vertex.
+// s_lo: {p_w, p_u, p_v, axis_w, axis_u, axis_v, shear_u, shear_v}.
+__device__ __forceinline__ void light_order_setup(const ExactGeo& g, int* s_lo) {
+  for (int k = 0; k < 3; ++k) {
+    s_lo[k] = g.pd[g.bo_axis[k]];
+    s_lo[3 + k] = g.bo_axis[k];
+  }
+  s_lo[6] = g.bo_shear[0];
+  s_lo[7] = g.bo_shear[1];
+}
+
+// Slot of that order -> vertex; false when the slot holds none.
+__device__ __forceinline__ bool light_slot_vertex(unsigned slot, int bl, const int* s_lo, int& x, int& y, int& z) {
+  const volatile int* q = s_lo;  // kept in shared memory, not in registers
+  const unsigned pw = q[0], pu = q[1], pv = q[2];
+  const unsigned group = slot / (pw << (2 * bl)), r = slot - group * (pw << (2 * bl));
+  const unsigned chunk = r >> (3 * bl), rr = r - (chunk << (3 * bl));
+  const unsigned height = min(1u << bl, pw - (chunk << bl));
+  const unsigned bundle = rr / (4u * height), k = rr - bundle * 4u * height;
+  const unsigned gu = (pu + (1u << bl) - 1u) >> bl, half = (1u << (bl - 1)) - 1u;
+  const int w = (int)((chunk << bl) + (k >> 2));
+  const unsigned u0 = ((group % gu) << bl) + ((bundle & half) << 1) + (k & 1u);
+  const unsigned v0 = ((group / gu) << bl) + ((bundle >> (bl - 1)) << 1) + ((k >> 1) & 1u);
+  if (u0 >= pu || v0 >= pv) return false;
+  int u = ((int)u0 + ((w * q[6]) >> 16)) % (int)pu, v = ((int)v0 + ((w * q[7]) >> 16)) % (int)pv;
+  u += (u < 0) ? (int)pu : 0;
+  v += (v < 0) ? (int)pv : 0;
+  const int aw = q[3], au = q[4];
+  x = aw == 0 ? w : (au == 0 ? u : v);
+  y = aw == 1 ? w : (au == 1 ? u : v);
+  z = aw == 2 ? w : (au == 2 ? u : v);
+  return true;
 }
 
 // Quad layout of a point field: Q[z][y][x] = {f(x,y,z), f(x+1,y,z), f(x,y+1,z),

@@ -69,7 +69,8 @@ __global__ void __launch_bounds__(kBatchThreads, 4) k_batch(const ExactGeo* __re
   __shared__ BatchDesc sd;
   __shared__ int s_item, s_req, s_phase, s_skip;
   __shared__ unsigned s_sub;
-  __shared__ int s_bo[8];  // the request's light-aligned brick order
+  __shared__ int s_lo[8];  // the request's light-aligned vertex order
+  __shared__ unsigned s_slots;
   extern __shared__ float4 s_dyn[];
   const int tid = threadIdx.x, lane = tid & 31;
   // shared TF (one colour map for the batch) and its normalised alpha
@@ -107,8 +108,11 @@ __global__ void __launch_bounds__(kBatchThreads, 4) k_batch(const ExactGeo* __re
       __syncthreads();
       const int ntab = phase == 1 ? sg.max_off[0] : sg.ntab;
       for (int i = tid; i < ntab; i += blockDim.x) s_tab[i] = table_entry(sg, i);
-      if (tid == 0 && plan.brick_log2) brick_order_setup(sg, plan.brick_log2, s_bo);
       if (tid == 0) {
+        if (plan.brick_log2) {
+          light_order_setup(sg, s_lo);
+          s_slots = light_slots(sg, plan.brick_log2);
+        }
         s_req = req;
         s_phase = phase;
       }
@@ -126,15 +130,9 @@ __global__ void __launch_bounds__(kBatchThreads, 4) k_batch(const ExactGeo* __re
         const int slot = base + (int)(t << 5) + lane;
         int id = -1, x = 0, y = 0, z = 0;
         if (bl) {
-          const int bi = slot >> (3 * bl), li = slot & ((1 << (3 * bl)) - 1), m = (1 << bl) - 1;
-          // slots past the last brick (the request's last item is padded to a whole item) do nothing
-          const int nb = ((const volatile int*)s_bo)[0] * ((const volatile int*)s_bo)[1] * ((const volatile int*)s_bo)[2];
-          int bx, by, bz;
-          pencil_brick(bi, s_bo, bx, by, bz);
-          x = (bx << bl) + (li & m);
-          y = (by << bl) + ((li >> bl) & m);
-          z = (bz << bl) + (li >> (2 * bl));
-          if (bi < nb && x < sg.pd[0] && y < sg.pd[1] && z < sg.pd[2]) id = (z * sg.pd[1] + y) * sg.pd[0] + x;
+          // slots past the last column (the request's last item is padded to a whole item) do nothing
+          if ((unsigned)slot < s_slots && light_slot_vertex((unsigned)slot, bl, s_lo, x, y, z))
+            id = (z * sg.pd[1] + y) * sg.pd[0] + x;
         } else if (slot < sd.nvert) {
           id = slot;
           x = id % sg.pd[0];

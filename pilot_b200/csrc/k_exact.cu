@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<STITCH, PREC, SKIP,
                                                           const float4* __restrict__ tab,
                                                           const float4* __restrict__ tf,
                                                           const float* __restrict__ tau,
-                                                          void* __restrict__ map, int nvert,
+                                                          void* __restrict__ map, unsigned nslots,
                                                           Counters* __restrict__ cnt,
                                                           const BrickRef* __restrict__ refs, int nrefs,
                                                           int self, const unsigned* __restrict__ gate,
@@ -202,17 +202,13 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<STITCH, PREC, SKIP,
   // inside the march, and the tiles in flight sweep the vertex order as one
   // compact window.
   const int lane = threadIdx.x & 31;
-  // The brick order's parameters live in shared memory and are re-read per
+  // The vertex order's parameters live in shared memory and are re-read per
   // tile, so they occupy no registers across the march (the march is
   // register-bound).
-  __shared__ int s_bo[8];
-  if (threadIdx.x == 0) brick_order_setup(g, g.light_brick_log2, s_bo);
+  __shared__ int s_lo[8];
+  if (threadIdx.x == 0) light_order_setup(g, s_lo);
   __syncthreads();
-  const int ntiles = [&] {
-    if (LIST) return (int)((vlist[0] + 31u) >> 5);
-    const int b0 = g.light_brick_log2;
-    return b0 ? (s_bo[0] * s_bo[1] * s_bo[2]) << (3 * b0 - 5) : (nvert + 31) >> 5;
-  }();
+  const int ntiles = LIST ? (int)((vlist[0] + 31u) >> 5) : (int)((nslots + 31u) >> 5);
   unsigned ns = 0, built = 0;
 
   for (int tile = next_warp_tile(&cnt->tiles_light); tile < ntiles; tile = next_warp_tile(&cnt->tiles_light)) {
@@ -225,22 +221,16 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<STITCH, PREC, SKIP,
       id = (int)vlist[1 + i];
       map_vertex(g, id, V);
     } else if (bl) {
-      // tile -> brick (light-aligned order), lane -> vertex of the brick (x fastest inside the brick)
-      const int bi = tile >> (3 * bl - 5);
-      const int li = ((tile & ((1 << (3 * bl - 5)) - 1)) << 5) + lane;
-      const int m = (1 << bl) - 1;
-      int bx, by, bz;
-      pencil_brick(bi, s_bo, bx, by, bz);
-      const int x = (bx << bl) + (li & m), y = (by << bl) + ((li >> bl) & m);
-      const int z = (bz << bl) + (li >> (2 * bl));
-      if (x >= g.pd[0] || y >= g.pd[1] || z >= g.pd[2]) continue;
+      const unsigned slot = ((unsigned)tile << 5) + lane;
+      int x, y, z;
+      if (slot >= nslots || !light_slot_vertex(slot, bl, s_lo, x, y, z)) continue;
       id = (z * g.pd[1] + y) * g.pd[0] + x;
       V[0] = vtx_coord(g, 0, x);
       V[1] = vtx_coord(g, 1, y);
       V[2] = vtx_coord(g, 2, z);
     } else {
       id = (tile << 5) + lane;
-      if (id >= nvert) continue;
+      if ((unsigned)id >= nslots) continue;
       map_vertex(g, id, V);
     }
     ++built;
@@ -571,6 +561,8 @@ static cudaError_t launch_k1(const ExactGeo& g, const void* quads, const float4*
                              int nrefs, int self, const unsigned* gate = nullptr,
                              const unsigned char* occ = nullptr, const unsigned* vlist = nullptr) {
   const int nvert = g.pd[0] * g.pd[1] * g.pd[2];
+  // vertex slots in the launch's order (the vertices themselves in rows)
+  const unsigned nslots = g.light_brick_log2 ? light_slots(g, g.light_brick_log2) : (unsigned)nvert;
   const size_t smem = (size_t)g.max_off[0] * sizeof(float4) + 2 * (size_t)g.tf_n * sizeof(float);
   const int ntiles = (nvert + kThreads - 1) / kThreads;
   int grid = 0;
@@ -587,13 +579,13 @@ static cudaError_t launch_k1(const ExactGeo& g, const void* quads, const float4*
         e = persistent_grid(k_light_march<float4, false, false, false, true, true>, smem, ntiles, grid);
         if (e != cudaSuccess) return e;
         k_light_march<float4, false, false, false, true, true><<<grid, kThreads, smem, st>>>(
-            g, (const float4*)quads, tab, tf, tau, map, nvert, cnt, refs, nrefs, self, gate, nullptr, vlist);
+            g, (const float4*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, nullptr, vlist);
         return cudaGetLastError();
       }
       e = persistent_grid(k_light_march<float4, false, false, false, true>, smem, ntiles, grid);
       if (e != cudaSuccess) return e;
       k_light_march<float4, false, false, false, true><<<grid, kThreads, smem, st>>>(
-          g, (const float4*)quads, tab, tf, tau, map, nvert, cnt, refs, nrefs, self, gate, nullptr, nullptr);
+          g, (const float4*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, nullptr, nullptr);
       return cudaGetLastError();
     } else {
       return cudaErrorInvalidValue;
@@ -605,12 +597,12 @@ static cudaError_t launch_k1(const ExactGeo& g, const void* quads, const float4*
         e = persistent_grid(k_light_march<QuadT, false, false, true, false, true>, smem, ntiles, grid);
         if (e != cudaSuccess) return e;
         k_light_march<QuadT, false, false, true, false, true><<<grid, kThreads, smem, st>>>(
-            g, (const QuadT*)quads, tab, tf, tau, map, nvert, cnt, refs, nrefs, self, gate, occ, vlist);
+            g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, occ, vlist);
       } else {
         e = persistent_grid(k_light_march<QuadT, false, false, false, false, true>, smem, ntiles, grid);
         if (e != cudaSuccess) return e;
         k_light_march<QuadT, false, false, false, false, true><<<grid, kThreads, smem, st>>>(
-            g, (const QuadT*)quads, tab, tf, tau, map, nvert, cnt, refs, nrefs, self, gate, nullptr, vlist);
+            g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, nullptr, vlist);
       }
       return cudaGetLastError();
     }
@@ -620,12 +612,12 @@ static cudaError_t launch_k1(const ExactGeo& g, const void* quads, const float4*
         e = persistent_grid(k_light_march<QuadT, false, true, true, false, true>, smem, ntiles, grid);
         if (e != cudaSuccess) return e;
         k_light_march<QuadT, false, true, true, false, true><<<grid, kThreads, smem, st>>>(
-            g, (const QuadT*)quads, tab, tf, tau, map, nvert, cnt, refs, nrefs, self, gate, occ, vlist);
+            g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, occ, vlist);
       } else {
         e = persistent_grid(k_light_march<QuadT, false, true, false, false, true>, smem, ntiles, grid);
         if (e != cudaSuccess) return e;
         k_light_march<QuadT, false, true, false, false, true><<<grid, kThreads, smem, st>>>(
-            g, (const QuadT*)quads, tab, tf, tau, map, nvert, cnt, refs, nrefs, self, gate, nullptr, vlist);
+            g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, nullptr, vlist);
       }
       return cudaGetLastError();
     }
@@ -635,7 +627,7 @@ static cudaError_t launch_k1(const ExactGeo& g, const void* quads, const float4*
       e = persistent_grid(k_light_march<QuadT, true, false, false, false, true>, smem, ntiles, grid);
       if (e != cudaSuccess) return e;
       k_light_march<QuadT, true, false, false, false, true><<<grid, kThreads, smem, st>>>(
-          g, (const QuadT*)quads, tab, tf, tau, map, nvert, cnt, refs, nrefs, self, gate, nullptr, vlist);
+          g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, nullptr, vlist);
       return cudaGetLastError();
     }
   } else {
@@ -644,14 +636,13 @@ static cudaError_t launch_k1(const ExactGeo& g, const void* quads, const float4*
   if (occ) {
     e = persistent_grid(k_light_march<QuadT, STITCH, PREC, true>, smem, ntiles, grid);
     if (e != cudaSuccess) return e;
-    k_light_march<QuadT, STITCH, PREC, true><<<grid, kThreads, smem, st>>>(g, (const QuadT*)quads, tab, tf, tau, map,
-                                                                           nvert, cnt, refs, nrefs, self, gate, occ,
+    k_light_march<QuadT, STITCH, PREC, true><<<grid, kThreads, smem, st>>>(g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, occ,
                                                                            nullptr);
   } else {
     e = persistent_grid(k_light_march<QuadT, STITCH, PREC, false>, smem, ntiles, grid);
     if (e != cudaSuccess) return e;
     k_light_march<QuadT, STITCH, PREC, false><<<grid, kThreads, smem, st>>>(g, (const QuadT*)quads, tab, tf, tau,
-                                                                            map, nvert, cnt, refs, nrefs, self, gate,
+                                                                            map, nslots, cnt, refs, nrefs, self, gate,
                                                                             nullptr, nullptr);
   }
   return cudaGetLastError();
