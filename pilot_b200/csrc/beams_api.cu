@@ -182,14 +182,14 @@ beams_status make_geo_vol(beams_renderer* r, const beams_volume& v, const beams_
   int off = 0;
   for (int d = 0; d < 3; ++d) {
     g.ax_off[d] = off;
-    off += g.n[d] - 1;
+    off += g.n[d];  // n - 1 cells and the closing entry (table_entry)
   }
   for (int d = 0; d < 3; ++d) {
     g.max_off[d] = off;
     off += r->map_m[d];
   }
   g.ntab = off;
-  geo_loop_constants(g);
+  geo_loop_constants(g, true);
   g.slab_fp64 = r->slab_fp64;
   g.use_map = r->use_map ? 1 : 0;
   g.assoc_cells = (v.assoc == BEAMS_ASSOC_CELLS) ? 1 : 0;
@@ -355,13 +355,14 @@ beams_status prepare_layouts(beams_renderer* r, const ExactGeo& g, int& launches
     if (e != cudaSuccess) return cuda_fail(r, e, "cell table build");
     ++launches;
     if (g.rect) {
-      // explicit coordinates: the field axes' entries {lo, hi, hi - lo, RN(1 / (hi - lo))}
+      // explicit coordinates: the field axes' entries
       std::vector<float4> fe((size_t)g.max_off[0]);
-      for (int d = 0; d < 3; ++d)
-        for (int c = 0; c + 1 < g.n[d]; ++c) {
-          const float lo = r->coords[d][c], hi = r->coords[d][c + 1], w = hi - lo;
-          fe[(size_t)g.ax_off[d] + c] = make_float4(lo, hi, w, 1.f / w);
-        }
+      for (int d = 0; d < 3; ++d) {
+        for (int c = 0; c + 1 < g.n[d]; ++c)
+          fe[(size_t)g.ax_off[d] + c] = field_entry(r->coords[d][c], r->coords[d][c + 1], (unsigned)c * g.fs[d]);
+        fe[(size_t)g.ax_off[d] + g.n[d] - 1] =
+            closing_entry(r->coords[d].back(), (unsigned)(g.n[d] - 2) * g.fs[d]);
+      }
       e = cudaMemcpyAsync(r->d_tab, fe.data(), fe.size() * sizeof(float4), cudaMemcpyHostToDevice, r->stream);
       if (e == cudaSuccess) e = cudaStreamSynchronize(r->stream);
       if (e != cudaSuccess) return cuda_fail(r, e, "coordinate table upload");

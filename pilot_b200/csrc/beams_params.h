@@ -1,7 +1,12 @@
 // beams_params.h — kernel parameter blocks, derived on the host from the scene
 // exactly as the reference derives them (float32 arithmetic, no contraction).
 #pragma once
+#include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
+
+#include <cmath>
+#include <cstring>
 
 namespace beams {
 
@@ -50,7 +55,7 @@ struct ExactGeo {
   int light_brick_log2;
   // That order's axes: columns run along bo_axis[0] (the axis the light travels
   // most along, in map-vertex units), the two other coordinates (bo_axis[1],
-  // bo_axis[2]) sheared by floor(w * bo_shear / 65536) modulo their counts, so
+  // bo_axis[2]) sheared by round(w * bo_shear / 65536) modulo their counts, so
   // that a column tracks a light ray through the vertex grid. Any order gives
   // the same map.
   int bo_axis[3];
@@ -66,15 +71,15 @@ struct ExactGeo {
   // search instead of from the uniform spacing; org/h/invh then only describe
   // the average spacing. 0: coord(d, i) = org[d] + h[d] * float(i).
   int rect;
-  // Loop constants the exact light march takes from the kernel's parameter
-  // space (the constant bank) instead of holding them in registers (set by
-  // geo_loop_constants): per field axis the cell guess's upper clamp n - 2 as
-  // a float, the quad strides (n0 - 1) and (n0 - 1)(n1 - 1), and the TF's last
-  // index as a float. The 257^3-vertex map of a 512^3 noise field: 2.59 ->
-  // 2.38 ms against the same values derived in the kernel.
-  float cmaxf[3];
-  unsigned qxs, qzs;
-  float n1f;
+  // The light march's cell guess scale per field axis: 1 / h, lowered where
+  // floor((maxp - org) * seed) would exceed n - 1, so that a guess always indexes
+  // the cell table (geo_loop_constants).
+  float seed[3];
+  float n1f;  // the TF's last index
+  // Strides of the field layout the marches read, in entries along x, y, z: the
+  // quads' {1, n0 - 1, (n0 - 1)(n1 - 1)}, or the plain field's (set by
+  // geo_loop_constants); cell (x, y, z) is entry fs . (x, y, z).
+  unsigned fs[3];
   // Pixel window {x0, y0, w, h} the (non-listed) view march covers; the whole
   // image unless a brick's projection is known to lie inside a smaller one
   // (every pixel outside it misses the volume).
@@ -119,23 +124,115 @@ struct Counters {
   unsigned int reserved;
 };
 
+__host__ __device__ inline unsigned float_bits(float x) {
+#ifdef __CUDA_ARCH__
+  return __float_as_uint(x);
+#else
+  unsigned u;
+  std::memcpy(&u, &x, 4);
+  return u;
+#endif
+}
+__host__ __device__ inline float bits_float(unsigned u) {
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(u);
+#else
+  float x;
+  std::memcpy(&x, &u, 4);
+  return x;
+#endif
+}
+
+// Map axes' cell table entry: {lo, w, rh, rl} of the cell [lo, hi], w = hi - lo,
+// rh = RN(1/w) and rl = RN((1 - w rh) / w) (the residual is exact), so rh + rl
+// is 1/w to 48 bits.
+__host__ __device__ inline float4 cell_entry(float lo, float hi) {
+  const float w = hi - lo, rh = 1.f / w;
+  return make_float4(lo, w, rh, fmaf(-w, rh, 1.f) / w);
+}
+
+// Whether fma(x, rh, x rl) is the correctly rounded x / w for every x, given
+// |rh + rl - 1/w| <= 7 * 2^-48 / w. The sum is x / w to 2^-45 before its one
+// rounding, so it can only round wrongly when a midpoint of two floats lies
+// within 2^-45 of x / w. With w = W 2^b, x = X 2^a, the midpoint M 2^c (W, X 24
+// bits, M odd, 25 bits) that means 0 < |X 2^k - M W| < 16, k = 24 (X >= W) or 25.
+// For each such difference D, M W = -D modulo 2^k fixes M modulo 2^k / (W's
+// trailing zeros) and X = (M W + D) / 2^k, so the few numerators at risk are
+// solved for and tried. M is odd, so D has exactly W's trailing zeros: from four
+// on (cells some 16 widths or more from coordinate 0) there are none.
+__host__ __device__ inline bool two_term_division_exact(float w, float rh, float rl) {
+  const unsigned bits = float_bits(w), ex = bits >> 23;
+  if (ex < 64u || ex > 190u) return false;  // far from any overflow or underflow (and w > 0)
+  const unsigned W = (bits & 0x7fffffu) | 0x800000u;
+  int z = 0;
+  while (z < 4 && !((W >> z) & 1u)) ++z;
+  if (z == 4) return true;
+  unsigned inv = W >> z;  // the odd part's inverse modulo 2^32 (Newton)
+  for (int i = 0; i < 5; ++i) inv *= 2u - (W >> z) * inv;
+  for (int k = 24; k <= 25; ++k)
+    for (int D = 1 << z; D < 16; D += 2 << z)
+      for (int sign = -1; sign <= 1; sign += 2) {
+        const unsigned step = 1u << (k - z), M0 = (0u - (unsigned)(sign * (D >> z))) * inv & (step - 1u);
+        for (unsigned M = M0; M < (1u << 25); M += step) {
+          if (M <= (1u << 24)) continue;
+          const long long X = ((long long)((unsigned long long)M * W) + sign * D) >> k;  // exact
+          if (X < (1 << 23) || X >= (1 << 24)) continue;
+          const float x = bits_float((ex << 23) | ((unsigned)X & 0x7fffffu));
+          if (fmaf(x, rh, x * rl) != x / w) return false;
+        }
+      }
+  return true;
+}
+
+// Field axes' cell table entry: {lo, offset, rh, rl} of the cell [lo, hi]; offset
+// (its bits) = the cell's term of the quad index. rl is the one of seven
+// neighbouring values, nearest to (1 - w rh) / w first, with which fma(x, rh, x
+// rl) is the correctly rounded quotient x / w for every x, or NaN when there is
+// none (the marches then divide).
+__host__ __device__ inline float4 field_entry(float lo, float hi, unsigned offset) {
+  const float w = hi - lo, rh = 1.f / w;
+  const float r0 = fmaf(-w, rh, 1.f) / w;
+  float rl = NAN;
+  for (int i = 0; i < 7; ++i) {
+    const int by = (i & 1) ? (i + 1) / 2 : -(i / 2);  // 0, 1, -1, 2, -2, 3, -3 ulp
+    const unsigned b = float_bits(r0) + (unsigned)by;
+    const float t = bits_float(b);
+    if (r0 == 0.f && i > 0) break;
+    if (two_term_division_exact(w, rh, t)) {
+      rl = t;
+      break;
+    }
+  }
+  return make_float4(lo, bits_float(offset), rh, rl);
+}
+// The entry after an axis's last cell: the last coordinate, and that cell's offset.
+__host__ __device__ inline float4 closing_entry(float lo, unsigned offset) {
+  return make_float4(lo, bits_float(offset), 1.f, 0.f);
+}
+
 // Slots of the light-aligned vertex order with groups of 2^bl x 2^bl columns
 // (light_slot_vertex): every vertex once, plus the padding columns of the last
 // groups.
-#ifdef __CUDACC__
-__host__ __device__
-#endif
-inline unsigned light_slots(const ExactGeo& g, int bl) {
+__host__ __device__ inline unsigned light_slots(const ExactGeo& g, int bl) {
   const unsigned pad = (1u << bl) - 1u;
   return (unsigned)g.pd[g.bo_axis[0]] * (((unsigned)g.pd[g.bo_axis[1]] + pad) & ~pad) *
          (((unsigned)g.pd[g.bo_axis[2]] + pad) & ~pad);
 }
 
-// Derives ExactGeo's loop constants from n[] and tf_n.
-inline void geo_loop_constants(ExactGeo& g) {
-  for (int d = 0; d < 3; ++d) g.cmaxf[d] = (float)(g.n[d] - 2);
-  g.qxs = (unsigned)(g.n[0] - 1);
-  g.qzs = g.qxs * (unsigned)(g.n[1] - 1);
+// Derives seed, n1f and fs. Coordinates that are not finite in float32 (an origin
+// past its range) have no inside: their bounds become NaN, which no position
+// passes, so no guess is ever formed from them.
+inline void geo_loop_constants(ExactGeo& g, bool quads) {
+  g.fs[0] = 1u;
+  g.fs[1] = (unsigned)(quads ? g.n[0] - 1 : g.n[0]);
+  g.fs[2] = g.fs[1] * (unsigned)(quads ? g.n[1] - 1 : g.n[1]);
+  for (int d = 0; d < 3; ++d) {
+    const float room = g.maxp[d] - g.org[d];
+    if (!(std::isfinite(g.org[d]) && std::isfinite(room))) g.minp[d] = g.maxp[d] = NAN;
+    g.seed[d] = (std::isfinite(g.invh[d]) && std::isfinite(room)) ? g.invh[d] : 0.f;
+    if ((double)room * g.seed[d] >= (double)g.n[d])  // the product of two floats is exact
+      g.seed[d] = (float)((g.n[d] - 1) / (double)room);
+  }
   g.n1f = (float)(g.tf_n - 1);
 }
 

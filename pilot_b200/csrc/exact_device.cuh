@@ -159,23 +159,21 @@ __device__ __forceinline__ void light_origin(const ExactGeo& g, const float V[3]
   }
 }
 
-// Entry i of the cell tables: {lo, hi, hi - lo, RN(1 / (hi - lo))} of field
-// cell i (axes in order) or, past max_off[0], of map cell i - max_off[0].
+// Entry i of the cell tables: per field axis its n - 1 cells (field_entry) and a
+// closing entry whose lo is the last coordinate (so a cell's upper coordinate is
+// the next entry's lo, and a guess one past the last cell reads a valid entry);
+// past max_off[0] the map axes' cells (cell_entry).
 __device__ __forceinline__ float4 table_entry(const ExactGeo& g, int i) {
-  float lo, hi;
   if (i < g.max_off[0]) {
     const int d = (i >= g.ax_off[2]) ? 2 : (i >= g.ax_off[1] ? 1 : 0);
     const int c = i - g.ax_off[d];
-    lo = coord(g, d, c);
-    hi = coord(g, d, c + 1);
-  } else {
-    const int d = (i >= g.max_off[2]) ? 2 : (i >= g.max_off[1] ? 1 : 0);
-    const int c = i - g.max_off[d];
-    lo = vtx_coord(g, d, c);
-    hi = vtx_coord(g, d, c + 1);
+    const float lo = coord(g, d, c);
+    return c < g.n[d] - 1 ? field_entry(lo, coord(g, d, c + 1), (unsigned)c * g.fs[d])
+                          : closing_entry(lo, (unsigned)(c - 1) * g.fs[d]);
   }
-  const float w = hi - lo;
-  return make_float4(lo, hi, w, 1.f / w);
+  const int d = (i >= g.max_off[2]) ? 2 : (i >= g.max_off[1] ? 1 : 0);
+  const int c = i - g.max_off[d];
+  return cell_entry(vtx_coord(g, d, c), vtx_coord(g, d, c + 1));
 }
 
 // (int)x for x in [0, 2^23), computed on the FMA pipe instead of the
@@ -186,50 +184,37 @@ __device__ __forceinline__ int trunc_small(float x) {
   return __float_as_int(__fadd_rz(x, 8388608.f)) - 0x4B000000;
 }
 
-// Correctly rounded division x / w given r = RN(1/w), after Markstein's
-// theorem (P. Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990): with r the
-// correctly rounded reciprocal and q a faithful quotient, the residual
-// e = x - q*w is exact under fma and RN(q + e*r) is the correctly rounded
-// quotient. One refinement makes q faithful, the second rounds it. Valid for
-// normal operands whose quotient neither overflows nor underflows, which
-// holds for the parametric coordinates here (|x| <= 2w, w a cell width);
-// beams_selftest(BEAMS_SELFTEST_DIVISION) checks it against IEEE division.
-__device__ __forceinline__ float div_rn_markstein(float x, float w, float r) {
-  float q = x * r;
-  float e = fmaf(-q, w, x);
-  q = fmaf(e, r, q);
-  e = fmaf(-q, w, x);
-  return fmaf(e, r, q);
+// Correctly rounded division x / w for the map cell entry e = {lo, w, rh, rl}. q =
+// fma(x, rh, x rl) is x / w to 2^-47 before its one rounding, hence faithful;
+// then the residual x - q w is exact under fma and, by Markstein's theorem (P.
+// Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34(1), 1990: rh the correctly rounded
+// reciprocal, q faithful), RN(q + residual rh) is the correctly rounded
+// quotient. Valid for normal operands whose quotient neither overflows nor
+// underflows, which holds for the parametric coordinates here (|x| <= 2w, w a
+// cell width); beams_selftest_division checks it against IEEE division.
+__device__ __forceinline__ float div_cell(float x, const float4& e) {
+  const float q = fmaf(x, e.z, x * e.w);
+  return fmaf(fmaf(-q, e.y, x), e.z, q);
 }
+// The same for a field cell entry, whose rl makes the two-term product itself the
+// correctly rounded quotient (field_entry), in two operations; NaN when it cannot.
+__device__ __forceinline__ float div_field(float x, const float4& e) { return fmaf(x, e.z, x * e.w); }
 
-// Cell tables: T[c] = {coord(c), coord(c+1), coord(c+1)-coord(c), RN(1/(coord(c+1)-coord(c)))}.
-//
 // Light-march cell search: RectilinearMeshOracle's binary search
 // (RectilinearMeshOracle.h:154-176) returns the smallest cell c with
 // val <= coord(c+1). The seed (val - org) / h is that cell for counting
 // coordinates except within an ulp of a cell face, where the bounded walk
 // below settles it. At c == 0 a point on the lower face stays in cell 0 and
 // inside the volume val <= coord(cmax+1), so one test per side suffices.
-__device__ __forceinline__ int find_cell_bsearch_t(const float4* T, int cmax, float org, float invh,
-                                                   float val, float4& e) {
-  int c = trunc_small(fminf(fmaxf((val - org) * invh, 0.f), (float)cmax));
-  e = T[c];
-  if (val <= e.x || val > e.y) {
-    while (c > 0 && val <= e.x) e = T[--c];
-    while (c < cmax && val > e.y) e = T[++c];
-  }
-  return c;
-}
-
 // The bounded walk that settles a seeded light-march cell guess (the smallest
 // c with val <= coord(c+1), RectilinearMeshOracle.h:154-176), for the rare
 // sample within an ulp of a cell face; kept out of line (noinline) so that the
 // march's common path carries none of its code.
 static __device__ __noinline__ int walk_cell_bsearch(const float4* T, int cmax, float val, int c) {
-  float4 e = T[c];
-  while (c > 0 && val <= e.x) e = T[--c];
-  while (c < cmax && val > e.y) e = T[++c];
+  c = min(c, cmax);
+  while (c > 0 && val <= T[c].x) --c;
+  while (c < cmax && val > T[c + 1].x) ++c;
   return c;
 }
 static __device__ __noinline__ int3 walk_cells_bsearch(const float4* T0, const float4* T1, const float4* T2, int m0,
@@ -249,7 +234,7 @@ __device__ __forceinline__ int find_cell_bsearch_rect(const float4* T, int cmax,
   int lo = 0, hi = cmax;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
-    if (val <= T[mid].y) hi = mid;
+    if (val <= T[mid + 1].x) hi = mid;
     else lo = mid + 1;
   }
   e = T[lo];
@@ -271,20 +256,17 @@ __device__ __forceinline__ int find_cell_walk_rect(const float4* T, int cmax, fl
 __device__ __forceinline__ int find_cell_walk_t(const float4* T, int cmax, float org, float invh, float p,
                                                 float4& e) {
   int c = trunc_small(fminf(fmaxf((p - org) * invh, 0.f), (float)cmax));
+  while (c > 0 && p < T[c].x) --c;
+  while (c < cmax && p >= T[c + 1].x) ++c;
   e = T[c];
-  if (p < e.x || p >= e.y) {
-    while (c > 0 && p < e.x) e = T[--c];
-    while (c < cmax && p >= e.y) e = T[++c];
-  }
   return c;
 }
 
 // The view march's walk (the unique c with coord(c) <= p < coord(c+1)) that
 // settles seeded guesses off by a face, out of line like walk_cells_bsearch.
 static __device__ __noinline__ int walk_cell_view(const float4* T, int cmax, float p, int c) {
-  float4 e = T[c];
-  while (c > 0 && p < e.x) e = T[--c];
-  while (c < cmax && p >= e.y) e = T[++c];
+  while (c > 0 && p < T[c].x) --c;
+  while (c < cmax && p >= T[c + 1].x) ++c;
   return c;
 }
 static __device__ __noinline__ int3 walk_cells_view(const float4* T0, const float4* T1, const float4* T2, int m0,
@@ -306,8 +288,9 @@ __device__ __forceinline__ void locate_view_cell(const ExactGeo& g, const float4
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     c[k] = trunc_small(fminf(fmaxf((p[k] - g.org[k]) * g.invh[k], 0.f), (float)(g.n[k] - 2)));
-    e[k] = s_tab[g.ax_off[k] + c[k]];
-    off = off | (p[k] < e[k].x) | (p[k] >= e[k].y);
+    const float4* T = s_tab + g.ax_off[k] + c[k];
+    e[k] = T[0];
+    off = off | (p[k] < e[k].x) | (p[k] >= T[1].x);
   }
   if (off) {
     const int3 cc = walk_cells_view(s_tab + g.ax_off[0], s_tab + g.ax_off[1], s_tab + g.ax_off[2], g.n[0] - 2,
@@ -324,7 +307,7 @@ __device__ __forceinline__ void locate_view_cell(const ExactGeo& g, const float4
       c[k] = g.n[k] - 2;
       e[k] = s_tab[g.ax_off[k] + c[k]];
     } else {
-      inv[k] = e[k].w;  // 1.f / (coord(c+1) - coord(c)), IEEE
+      inv[k] = e[k].z;  // 1.f / (coord(c+1) - coord(c)), IEEE
     }
     bl[k] = e[k].x;
   }
@@ -396,9 +379,10 @@ __device__ __forceinline__ bool ray_setup(const ExactGeo& g, int x, int y, float
   return slab_t<float>(o, d, g.bmin, g.bmax, minD, maxD);
 }
 
+// A position with a NaN coordinate is outside.
 __device__ __forceinline__ bool inside_vol(const ExactGeo& g, const float p[3]) {
-  return !(p[0] < g.minp[0] || p[0] > g.maxp[0] || p[1] < g.minp[1] || p[1] > g.maxp[1] ||
-           p[2] < g.minp[2] || p[2] > g.maxp[2]);
+  return p[0] >= g.minp[0] && p[0] <= g.maxp[0] && p[1] >= g.minp[1] && p[1] <= g.maxp[1] && p[2] >= g.minp[2] &&
+         p[2] <= g.maxp[2];
 }
 
 template <typename MapT> __device__ __forceinline__ float ld_map(const MapT* p);
@@ -421,7 +405,7 @@ __device__ __forceinline__ float map_interp_t(const ExactGeo& g, const float4* M
     const float t = (p[d] - g.morig[d]) * g.minv[d];
     c[d] = trunc_small(fminf(fmaxf(t, 0.f), (float)(g.pd[d] - 2)));
     const float4 e = MT[g.max_off[d] + c[d]];
-    pc[d] = div_rn_markstein(p[d] - e.x, e.z, e.w);
+    pc[d] = div_cell(p[d] - e.x, e);
   }
   const unsigned px = (unsigned)g.pd[0], pxy = (unsigned)g.pd[0] * (unsigned)g.pd[1];
   const MapT* m = map + ((unsigned)c[2] * pxy + (unsigned)c[1] * px + (unsigned)c[0]);
@@ -449,7 +433,7 @@ __device__ __forceinline__ void map_light_sum(const ExactGeo& g, const float4* M
     const float t = (p[d] - g.morig[d]) * g.minv[d];
     c[d] = trunc_small(fminf(fmaxf(t, 0.f), (float)(g.pd[d] - 2)));
     const float4 e = MT[g.max_off[d] + c[d]];
-    pc[d] = div_rn_markstein(p[d] - e.x, e.z, e.w);
+    pc[d] = div_cell(p[d] - e.x, e);
   }
   const unsigned px = (unsigned)g.pd[0], pxy = (unsigned)g.pd[0] * (unsigned)g.pd[1];
   const size_t nv = (size_t)pxy * (unsigned)g.pd[2];
@@ -498,10 +482,10 @@ __device__ __forceinline__ void pencil_brick(int bi, const int* s_bo, int& bx, i
 
 // The map build's vertex order. Columns of vertices run along w, the axis the
 // light travels most along, and follow the light: column (u, v) holds at w the
-// vertex (u + floor(w shear_u), v + floor(w shear_v)) modulo the grid, so every
+// vertex (u + round(w shear_u), v + round(w shear_v)) modulo the grid, so every
 // vertex is in exactly one column. Columns go in groups of E x E (E = 2^bl),
 // groups in raster order; inside a group chunks of E along w, inside a chunk
-// 2 x 2-column bundles, inside a bundle w, then the four columns. 32
+// 2 x 2-column bundles, inside a bundle its four columns one after the other. 32
 // consecutive slots are then about 8 vertices along the light by 2 by 2 across:
 // their rays run within a map cell or two of one another, so a warp's 32
 // samples fall into few cells and its loads into few lines (the light march of
@@ -524,13 +508,13 @@ __device__ __forceinline__ bool light_slot_vertex(unsigned slot, int bl, const i
   const unsigned group = slot / (pw << (2 * bl)), r = slot - group * (pw << (2 * bl));
   const unsigned chunk = r >> (3 * bl), rr = r - (chunk << (3 * bl));
   const unsigned height = min(1u << bl, pw - (chunk << bl));
-  const unsigned bundle = rr / (4u * height), k = rr - bundle * 4u * height;
-  const unsigned gu = (pu + (1u << bl) - 1u) >> bl, half = (1u << (bl - 1)) - 1u;
-  const int w = (int)((chunk << bl) + (k >> 2));
-  const unsigned u0 = ((group % gu) << bl) + ((bundle & half) << 1) + (k & 1u);
-  const unsigned v0 = ((group / gu) << bl) + ((bundle >> (bl - 1)) << 1) + ((k >> 1) & 1u);
+  const unsigned column = rr / height, wi = rr - column * height;
+  const unsigned bundle = column >> 2, gu = (pu + (1u << bl) - 1u) >> bl, half = (1u << (bl - 1)) - 1u;
+  const int w = (int)((chunk << bl) + wi);
+  const unsigned u0 = ((group % gu) << bl) + ((bundle & half) << 1) + (column & 1u);
+  const unsigned v0 = ((group / gu) << bl) + ((bundle >> (bl - 1)) << 1) + ((column >> 1) & 1u);
   if (u0 >= pu || v0 >= pv) return false;
-  int u = ((int)u0 + ((w * q[6]) >> 16)) % (int)pu, v = ((int)v0 + ((w * q[7]) >> 16)) % (int)pv;
+  int u = ((int)u0 + ((w * q[6] + 32768) >> 16)) % (int)pu, v = ((int)v0 + ((w * q[7] + 32768) >> 16)) % (int)pv;
   u += (u < 0) ? (int)pu : 0;
   v += (v < 0) ? (int)pv : 0;
   const int aw = q[3], au = q[4];
@@ -616,45 +600,6 @@ __device__ __forceinline__ bool occupied(const ExactGeo& g, const unsigned char*
     m[d] = trunc_small(f) >> kMacroLog2;
   }
   return __ldg(occ + ((size_t)m[2] * g.occ_n[1] + m[1]) * g.occ_n[0] + m[0]) != 0;
-}
-
-// The light march of TransmittanceMap.h:279-332 from L to an arbitrary point P
-// (K1 runs it to map vertices): opacity accumulated over the same sample
-// sequence. T0..T2: field cell tables; s_a: TF alpha / max alpha.
-__device__ __forceinline__ float point_opacity(const ExactGeo& g, const float4* __restrict__ quads, const float4* T0,
-                                               const float4* T1, const float4* T2, const float* s_a, const float L[3],
-                                               const float P[3]) {
-  const float v[3] = {P[0] - L[0], P[1] - L[1], P[2] - L[2]};
-  const float rs = 1.f / sqrtf(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-  const float dir[3] = {v[0] * rs, v[1] * rs, v[2] * rs};
-  float tmin, tmax;
-  segment_aabb(g, L, P, tmin, tmax);
-  const float st[3] = {L[0] + tmin * dir[0], L[1] + tmin * dir[1], L[2] + tmin * dir[2]};
-  float s[3] = {st[0], st[1], st[2]};
-  const float len2 = (tmax - tmin) * (tmax - tmin);
-  const int n1 = g.tf_n - 1;
-  const unsigned qx = (unsigned)(g.n[0] - 1), qz = (unsigned)(g.n[0] - 1) * (unsigned)(g.n[1] - 1);
-  float o = 0.f;
-  for (int b = g.light_budget; b > 0; --b) {
-    const float q0 = s[0] - st[0], q1 = s[1] - st[1], q2 = s[2] - st[2];
-    if (!(q0 * q0 + q1 * q1 + q2 * q2 <= len2)) break;
-    s[0] = s[0] + g.step * dir[0];
-    s[1] = s[1] + g.step * dir[1];
-    s[2] = s[2] + g.step * dir[2];
-    if (!inside_vol(g, s)) break;
-    float4 e0, e1, e2;
-    const int c0 = find_cell_bsearch_t(T0, g.n[0] - 2, g.org[0], g.invh[0], s[0], e0);
-    const int c1 = find_cell_bsearch_t(T1, g.n[1] - 2, g.org[1], g.invh[1], s[1], e1);
-    const int c2 = find_cell_bsearch_t(T2, g.n[2] - 2, g.org[2], g.invh[2], s[2], e2);
-    float vals[8];
-    QuadLoad<float4>::cell(quads, (unsigned)c2 * qz + (unsigned)c1 * qx + (unsigned)c0, qx, qz, vals);
-    float scalar = hex_interp(vals, div_rn_markstein(s[0] - e0.x, e0.z, e0.w), div_rn_markstein(s[1] - e1.x, e1.z, e1.w),
-                              div_rn_markstein(s[2] - e2.x, e2.z, e2.w));
-    scalar = (scalar - g.min_scalar) * g.inv_delta;
-    o = o + (1.f - o) * s_a[tf_index_clamped(scalar * (float)n1, n1)];
-    if (o == 1.f) break;
-  }
-  return o;
 }
 
 // Warp-aggregated counter increment (one atomic per warp). Must be reached by

@@ -21,7 +21,7 @@
 // Per item a block keeps the request's geometry and cell tables in shared
 // memory (recomputed there when the request changes, so no table buffers or
 // table launches exist). Results equal the single-request kernels': the light
-// march per vertex is march_vertex (the K1 march) and the view march is
+// march per vertex is light_march (the K1 march) and the view march is
 // view_march_pixel. Compiled with -fmad=false like every kernel file.
 #include <cuda_runtime.h>
 
@@ -122,6 +122,7 @@ __global__ void __launch_bounds__(kBatchThreads, 4) k_batch(const ExactGeo* __re
       // a chunk of kBatchChunk vertex slots; warps take 32-slot tiles from the block's counter
       const int bl = plan.brick_log2;
       const int base = li * kBatchChunk;
+      const LightField<float4> F(sg, sd.quads, s_tab, s_a, sd.occ);
       for (;;) {
         unsigned t = 0;
         if (lane == 0) t = atomicAdd(&s_sub, 1u);
@@ -145,9 +146,10 @@ __global__ void __launch_bounds__(kBatchThreads, 4) k_batch(const ExactGeo* __re
           light_origin(sg, V, L);
           Accum<false> acc;
           unsigned ns = 0;
-          march_vertex<float4, false, SKIP, false, SKIP && MODE != 0, true>(sg, sd.quads, s_tab + sg.ax_off[0], s_tab + sg.ax_off[1],
-                                            s_tab + sg.ax_off[2], s_a, nullptr, sd.occ, V, L,
-                                            [](const float*) { return 0.f; }, acc, ns);
+          float dir[3];
+          const LightRay ray = light_ray(sg, V, L, dir);
+          acc.init(0.f);
+          light_march<float4, false, SKIP>(sg, F, ray, ray.sure, acc, ns);
           acc.store(sd.map, id);
         }
       }

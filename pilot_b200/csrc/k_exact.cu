@@ -42,11 +42,11 @@ __device__ __forceinline__ void load_tables(float4* s_tab, const float4* __restr
 // STITCH: the multi-brick Phase 3 — the march starts from the cross-brick
 // prefix (stitch_prefix) instead of zero, as GenerateEstimator is re-run on
 // the prefix opacities (LightedVolumeRenderer.cxx:1241-1252).
-// Blocks per SM: 6 (40 registers) for the plain and the stitching exact march,
-// which issue one sample at a time (the 257^3-vertex map of a 512^3 noise
-// field: 2.70 ms against 2.78 ms at 4 blocks; the 2x2x2-brick frame 0.7% faster
-// than at 4); the skipping, precision and rectilinear marches keep 4 (at 6 they
-// spill: the 640^3 precision build went 6.4 -> 9.5 ms).
+// Blocks per SM: 6 (40 registers) for the plain and the stitching exact march
+// (the 257^3-vertex map of a 512^3 noise field, mean of eight light directions:
+// 2.39 ms against 2.63 ms at 4 blocks, where the loads' latency shows); the
+// skipping, precision and rectilinear marches keep 4 (at 6 they spill: the 640^3
+// precision build went 6.4 -> 9.5 ms).
 template <bool STITCH, bool PREC, bool SKIP, bool RECT>
 constexpr int k1_blocks_per_sm() {
   return (PREC || SKIP || RECT) ? 4 : 6;
@@ -195,9 +195,7 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<STITCH, PREC, SKIP,
   }
   __syncthreads();
 
-  const float4* T0 = s_tab + g.ax_off[0];
-  const float4* T1 = s_tab + g.ax_off[1];
-  const float4* T2 = s_tab + g.ax_off[2];
+  const LightField<QuadT> F(g, quads, s_tab, PREC ? s_tau : s_a, occ);
   // Warps take 32-vertex tiles from a launch-wide counter: no block barriers
   // inside the march, and the tiles in flight sweep the vertex order as one
   // compact window.
@@ -235,12 +233,17 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<STITCH, PREC, SKIP,
     }
     ++built;
     light_origin(g, V, L);
+    float dir[3];
+    const LightRay ray = light_ray(g, V, L, dir);
     Accum<PREC> acc;
-    march_vertex<QuadT, PREC, SKIP, RECT>(g, quads, T0, T1, T2, s_a, s_tau, occ, V, L,
-                                    [&](const float dir[3]) {
-                                      return STITCH ? stitch_prefix(refs, nrefs, self, L, V, dir) : 0.f;
-                                    },
-                                    acc, ns);
+    acc.init(STITCH ? stitch_prefix(refs, nrefs, self, L, V, dir) : 0.f);
+    if constexpr (RECT) {
+      light_march_rect(g, quads, s_tab, s_a, ray, acc, ns);
+    } else {
+      // the lanes leave the untested steps together
+      const int sure = SKIP ? ray.sure : __reduce_min_sync(__activemask(), ray.sure);
+      light_march<QuadT, PREC, SKIP>(g, F, ray, sure, acc, ns);
+    }
     acc.store(map, id);
   }
   warp_add(&cnt->light_samples, ns);
@@ -405,7 +408,7 @@ __global__ void __launch_bounds__(kThreads) k_view_march_cells(const ExactGeo g,
               e = T[c[k]];
             } else {
               c[k] = find_cell_walk_t(T, g.n[k] - 2, g.org[k], g.invh[k], p[k], e);
-              inv[k] = e.w;
+              inv[k] = e.z;
             }
             bl[k] = e.x;
           }
@@ -447,8 +450,8 @@ __global__ void __launch_bounds__(kThreads) k_view_march_cells(const ExactGeo g,
 // ---------------------------------------------------------------------------
 // layout builders
 // ---------------------------------------------------------------------------
-// Cell tables: field axes then map axes, each entry {lo, hi, hi-lo, RN(1/(hi-lo))}
-// with lo/hi the same float expressions the marches compare against.
+// Cell tables: field axes then map axes, each entry by
+// table_entry, with lo/hi the same float expressions the marches compare against.
 __global__ void k_build_tables(const ExactGeo g, float4* __restrict__ tab) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.ntab) return;
@@ -798,7 +801,8 @@ __global__ void k_build_occupancy(const ExactGeo g, const QuadT* __restrict__ qu
 }
 
 void occupancy_dims(const int n[3], int occ_n[3]) {
-  for (int d = 0; d < 3; ++d) occ_n[d] = ((n[d] - 1) + (1 << kMacroLog2) - 1) >> kMacroLog2;
+  // the macro-cell of a guess one past the last cell (the volume's max face) included
+  for (int d = 0; d < 3; ++d) occ_n[d] = ((n[d] - 1) >> kMacroLog2) + 1;
 }
 
 cudaError_t launch_build_occupancy(const ExactGeo& g, int quad_dtype, const void* quads, const float4* tf,
@@ -940,8 +944,8 @@ __global__ void k_selftest_division(float org, float h, int ncells, int samples,
     const unsigned k = (unsigned)(i - (long long)c * samples);
     const float lo = org + h * (float)c;
     const float hi = org + h * (float)(c + 1);
-    const float w = hi - lo;
-    const float r = 1.f / w;
+    const float4 e = cell_entry(lo, hi), ef = field_entry(lo, hi, 0u);
+    const float w = e.y;
     // x spans [-w/2, 3w/2]: a Weyl sequence over the interval plus exact end points.
     float x;
     if (k == 0) x = 0.f;
@@ -952,8 +956,9 @@ __global__ void k_selftest_division(float org, float h, int ncells, int samples,
       x = (u * 2.f - 0.5f) * w;
     }
     const float ref = x / w;  // IEEE (prec-div)
-    const float got = div_rn_markstein(x, w, r);
-    nb += (__float_as_uint(ref) != __float_as_uint(got)) ? 1u : 0u;
+    const float got = div_cell(x, e);
+    const float gotf = div_field(x, ef);  // NaN: the marches divide
+    nb += (__float_as_uint(ref) != __float_as_uint(got) || (gotf == gotf && ref != gotf)) ? 1u : 0u;
     nc += 1u;
   }
   const unsigned sb = __reduce_add_sync(0xffffffffu, nb), sc = __reduce_add_sync(0xffffffffu, nc);

@@ -124,9 +124,7 @@ __global__ void __launch_bounds__(kThreadsP, 3) k_probe_check(const ExactGeo g, 
   }
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const float4* T0 = s_tab + g.ax_off[0];
-  const float4* T1 = s_tab + g.ax_off[1];
-  const float4* T2 = s_tab + g.ax_off[2];
+  const LightField<float4> F(g, quads, s_tab, s_a, nullptr);
   for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < nprobe; q += nwarps) {
     const int x = (q % pg.nqx) * pg.P + pg.h, y = (q / pg.nqx) * pg.P + pg.h;
     const int m = count[q];
@@ -144,8 +142,10 @@ __global__ void __launch_bounds__(kThreadsP, 3) k_probe_check(const ExactGeo g, 
           light_origin(g, P, L);
           Accum<false> acc;
           unsigned ns = 0;
-          march_vertex<float4, false, false>(g, quads, T0, T1, T2, s_a, nullptr, nullptr, P, L,
-                                             [](const float*) { return 0.f; }, acc, ns);
+          float dir[3];
+          const LightRay ray = light_ray(g, P, L, dir);
+          acc.init(0.f);
+          light_march<float4, false, false>(g, F, ray, ray.sure, acc, ns);
           const float tr = 1.f - acc.o;
           s0 = clamp01(tc.x * (tr * g.light_color[0]));
           s1 = clamp01(tc.y * (tr * g.light_color[1]));

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "exact_device.cuh"
+#include "light_march.cuh"
 #include "kernels.h"
 #include "mlp_common.cuh"
 #include "mlp_host.h"
@@ -38,20 +39,9 @@ __device__ __forceinline__ float uniform01(unsigned seed, unsigned i, unsigned k
 
 // ---- data: exact transmittance at random points ---------------------------------
 // Normalised colour-map alpha of the field at P (one light-march sample).
-__device__ float alpha_at(const ExactGeo& g, const float4* __restrict__ quads, const float4* T0, const float4* T1,
-                          const float4* T2, const float* s_a, const float P[3]) {
-  const unsigned qx = (unsigned)(g.n[0] - 1), qz = (unsigned)(g.n[0] - 1) * (unsigned)(g.n[1] - 1);
-  float4 e0, e1, e2;
-  const int c0 = find_cell_bsearch_t(T0, g.n[0] - 2, g.org[0], g.invh[0], P[0], e0);
-  const int c1 = find_cell_bsearch_t(T1, g.n[1] - 2, g.org[1], g.invh[1], P[1], e1);
-  const int c2 = find_cell_bsearch_t(T2, g.n[2] - 2, g.org[2], g.invh[2], P[2], e2);
-  float vals[8];
-  QuadLoad<float4>::cell(quads, (unsigned)c2 * qz + (unsigned)c1 * qx + (unsigned)c0, qx, qz, vals);
-  float scalar = hex_interp(vals, div_rn_markstein(P[0] - e0.x, e0.z, e0.w), div_rn_markstein(P[1] - e1.x, e1.z, e1.w),
-                            div_rn_markstein(P[2] - e2.x, e2.z, e2.w));
-  scalar = (scalar - g.min_scalar) * g.inv_delta;
-  const int n1 = g.tf_n - 1;
-  return s_a[tf_index_clamped(scalar * (float)n1, n1)];
+__device__ __noinline__ float alpha_at(const ExactGeo& g, const LightField<float4>& F, const float P[3]) {
+  return sample_value(g, F, P, guess(P[0], g.org[0], g.seed[0]), guess(P[1], g.org[1], g.seed[1]),
+                      guess(P[2], g.org[2], g.seed[2]));
 }
 
 // sample i: position (world) in xyz, light index in w; target transmittance.
@@ -69,6 +59,7 @@ __global__ void __launch_bounds__(256) k_gen_data(const ExactGeo g, const float4
   for (int i = threadIdx.x; i < g.max_off[0]; i += blockDim.x) s_tab[i] = tab[i];
   for (int i = threadIdx.x; i < g.tf_n; i += blockDim.x) s_a[i] = (g.max_alpha > 0.f) ? tf[i].w / g.max_alpha : 0.f;
   __syncthreads();
+  const LightField<float4> F(g, quads, s_tab, s_a, nullptr);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int li = (int)(hash32(seed + 7919u * (unsigned)i) % (unsigned)nlights);
     float P[3];
@@ -78,15 +69,19 @@ __global__ void __launch_bounds__(256) k_gen_data(const ExactGeo g, const float4
 #pragma unroll
       for (int a = 0; a < 3; ++a)
         P[a] = g.minp[a] + uniform01(seed, (unsigned)i, k + (unsigned)a) * (g.maxp[a] - g.minp[a]);
-      if (tries == 1 || alpha_at(g, quads, s_tab + g.ax_off[0], s_tab + g.ax_off[1], s_tab + g.ax_off[2], s_a, P) > 0.f)
+      if (tries == 1 || alpha_at(g, F, P) > 0.f)
         break;
     }
     const float4 Lw = lights[li];
     const float L[3] = {Lw.x, Lw.y, Lw.z};
-    const float o = point_opacity(g, quads, s_tab + g.ax_off[0], s_tab + g.ax_off[1], s_tab + g.ax_off[2], s_a,
-                                  L, P);
+    float dir[3];
+    const LightRay ray = light_ray(g, P, L, dir);
+    Accum<false> acc;
+    acc.init(0.f);
+    unsigned ns = 0;
+    light_march<float4, false, false>(g, F, ray, ray.sure, acc, ns);
     samples[i] = make_float4(P[0], P[1], P[2], (float)li);
-    target[i] = 1.f - o;
+    target[i] = 1.f - acc.o;
   }
 }
 

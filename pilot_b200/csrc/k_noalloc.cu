@@ -11,7 +11,7 @@
 // the caller's input and output buffers.
 //
 // The kernels run the same march code as beams_render's K1 and K2
-// (march_vertex, view_march_pixel) on the plain float32 field with the cell
+// (light_march, view_march_pixel) on the plain float32 field with the cell
 // tables computed into shared memory, so the image equals beams_render's bit
 // for bit.
 // Compiled with -fmad=false like every kernel file.
@@ -58,7 +58,7 @@ cudaError_t scratch_address(float** out) {
 // Errors go to the thread-local text that beams_last_error(NULL) returns.
 beams_status nf(beams_status s, const char* msg) { return fail(nullptr, s, msg); }
 
-// The cell tables {lo, hi, hi - lo, RN(1/(hi - lo))} computed into shared
+// The cell tables (table_entry) computed into shared
 // memory from the generated coordinates (the entries beams_render builds once
 // per volume into device memory), n entries from the start.
 __device__ void stage_tables(const ExactGeo& g, int n, float4* s_tab) {
@@ -66,7 +66,7 @@ __device__ void stage_tables(const ExactGeo& g, int n, float4* s_tab) {
 }
 
 // K1: one thread per map vertex, the light march of k_light_march
-// (march_vertex, TransmittanceMap.h:279-332) on the plain field, into the
+// (light_march, TransmittanceMap.h:279-332) on the plain field, into the
 // scratch map. Alpha / max alpha as GetMaxAlpha (TransmittanceMap.h:515-525).
 __global__ void __launch_bounds__(256) k_noalloc_light_march(const ExactGeo g, const FieldF32* __restrict__ field,
                                                              const float4* __restrict__ tf,
@@ -91,8 +91,10 @@ __global__ void __launch_bounds__(256) k_noalloc_light_march(const ExactGeo g, c
   light_origin(g, V, L);
   Accum<false> acc;
   unsigned ns = 0;
-  march_vertex<FieldF32, false, false>(g, field, s_tab + g.ax_off[0], s_tab + g.ax_off[1], s_tab + g.ax_off[2], s_a,
-                                       nullptr, nullptr, V, L, [](const float*) { return 0.f; }, acc, ns);
+  float dir[3];
+  const LightRay ray = light_ray(g, V, L, dir);
+  acc.init(0.f);
+  light_march<FieldF32, false, false>(g, LightField<FieldF32>(g, field, s_tab, s_a, nullptr), ray, ray.sure, acc, ns);
   map[id] = acc.o;
 }
 
@@ -182,7 +184,7 @@ extern "C" beams_status beams_render_noalloc(const beams_volume* vol, const floa
     int off = 0;
     for (int d = 0; d < 3; ++d) {
       g.ax_off[d] = off;
-      off += g.n[d] - 1;
+      off += g.n[d];
     }
     for (int d = 0; d < 3; ++d) {
       g.max_off[d] = off;
@@ -190,7 +192,7 @@ extern "C" beams_status beams_render_noalloc(const beams_volume* vol, const floa
     }
     g.ntab = off;
   }
-  geo_loop_constants(g);
+  geo_loop_constants(g, false);
   float ext[3];
   for (int d = 0; d < 3; ++d) ext[d] = (float)(g.bmax[d] - g.bmin[d]);
   g.extent_mag = std::sqrt(ext[0] * ext[0] + ext[1] * ext[1] + ext[2] * ext[2]);

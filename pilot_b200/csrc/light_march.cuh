@@ -1,8 +1,8 @@
 // light_march.cuh — one light ray of the map build: the march of
 // TransmittanceMapGenerator::operator() (beams/rendering/TransmittanceMap.h:279-332)
-// from the light towards a map vertex (one sample at a time, or two deep in the
-// exact form's skipping march). Shared by K1 (k_exact.cu), the batched kernel
-// (k_batch.cu) and the learned form's probe check (k_mlp_probe.cu).
+// from the light towards a map vertex. Shared by K1 (k_exact.cu), the batched
+// kernel (k_batch.cu), the allocation-free entry point (k_noalloc.cu) and the
+// learned form's training data and probe check (k_mlp_train.cu, k_mlp_probe.cu).
 // Compiled with -fmad=false (see exact_device.cuh).
 #pragma once
 #include <cuda_fp16.h>
@@ -24,8 +24,8 @@ template <bool PREC> struct Accum;
 template <> struct Accum<false> {
   float o;
   __device__ __forceinline__ void init(float o0) { o = o0; }
-  __device__ __forceinline__ bool add(const float* s_a, const float*, int idx) {
-    o = o + (1.f - o) * s_a[idx];
+  __device__ __forceinline__ bool add(float a) {
+    o = o + (1.f - o) * a;
     return o == 1.f;
   }
   __device__ __forceinline__ void store(void* map, int id) const { ((float*)map)[id] = o; }
@@ -38,8 +38,7 @@ template <> struct Accum<true> {
     comp = 0.f;
     cut = false;
   }
-  __device__ __forceinline__ bool add(const float*, const float* s_tau, int idx) {
-    const float ti = s_tau[idx];
+  __device__ __forceinline__ bool add(float ti) {
     if (ti == __int_as_float(0x7f800000)) {
       cut = true;
       return true;
@@ -57,195 +56,260 @@ template <> struct Accum<true> {
   }
 };
 
-// March from L towards vertex V. prefix(dir) gives the starting opacity (0,
-// or the cross-brick prefix of the multi-brick Phase 3). ns counts the samples
-// marched. With SKIP, occ is the macro-cell occupancy (see occupied()).
-// PIPE: sample k+1 is located and its loads issued before sample k is
-// composited (two samples' loads in flight per ray). That pays only in the
-// exact form's skipping march; elsewhere the march issues one sample at a time,
-// which needs fewer registers and instructions (the 257^3-vertex map of a
-// 512^3 noise field went 2.97 -> 2.78 ms at 4 blocks per SM, 2.70 ms at 6).
-template <typename QuadT, bool PREC, bool SKIP, bool RECT = false, bool PIPE = SKIP && !PREC, bool REG_CONSTS = PREC,
-          typename Prefix>
-__device__ __forceinline__ void march_vertex(const ExactGeo& g, const QuadT* __restrict__ quads, const float4* T0,
-                                             const float4* T1, const float4* T2, const float* s_a,
-                                             const float* s_tau, const unsigned char* __restrict__ occ,
-                                             const float V[3], const float L[3], Prefix prefix, Accum<PREC>& acc,
-                                             unsigned& ns) {
-  const int cm0 = g.n[0] - 2, cm1 = g.n[1] - 2, cm2 = g.n[2] - 2;
-  // Loop constants: with REG_CONSTS derived here (held in registers), else read
-  // at each use from g's loop-constant fields, which in a kernel's parameter
-  // block cost no registers (the exact light march: 2.59 -> 2.38 ms at six
-  // blocks per SM). The precision march (1.5% faster so) and the batch kernel,
-  // whose geometry lives in shared memory, derive them.
-  unsigned qx, qz;  // FieldF32, and quads with REG_CONSTS
-  QuadLoad<QuadT>::strides(g, qx, qz);
-  const int n1 = g.tf_n - 1;
+// A light ray from L to V: the first position (where the segment enters the
+// volume), the step, and the squared length the distance test compares with.
+struct LightRay {
+  float st[3], sd[3];
+  float len2;
+  int sure;  // the first `sure` steps pass every test (see light_ray)
+};
+
+// sure: steps certain to pass the budget, distance and inside tests, so the
+// march need not make them (11 of its instructions). With u = 2^-24:
+//  * distance: after k steps the float position lies within k (step (1 + 4u) +
+//    2 sqrt(3) u M) of the start (M bounds every |coordinate| on the segment),
+//    so |s - st|^2 <= len2 holds, rounding included, while k < (1 - 4u) (tmax -
+//    tmin) / (that per-step bound);
+//  * inside: adding a constant to a float, rounding included, is monotonic, so
+//    steps 1..k are inside when step 1 is (tested here) and step k is; per axis
+//    k steps move the position by at most k (|sd| + u B), B = max |bound|, so
+//    step k is inside while k (that) < the room from st to the bound ahead.
+// Every u term is doubled or more, the approximate divisions err by 2 ulp
+// against the 1e-5 taken off, and two more steps are kept back.
+__device__ __forceinline__ LightRay light_ray(const ExactGeo& g, const float V[3], const float L[3], float dir[3]) {
+  LightRay r;
   const float v[3] = {V[0] - L[0], V[1] - L[1], V[2] - L[2]};
   const float rs = 1.f / sqrtf(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-  const float dir[3] = {v[0] * rs, v[1] * rs, v[2] * rs};
   float tmin, tmax;
   segment_aabb(g, L, V, tmin, tmax);
-  const float st[3] = {L[0] + tmin * dir[0], L[1] + tmin * dir[1], L[2] + tmin * dir[2]};
-  float s[3] = {st[0], st[1], st[2]};
-  const float len2 = (tmax - tmin) * (tmax - tmin);
-  const float sdx = g.step * dir[0], sdy = g.step * dir[1], sdz = g.step * dir[2];
-  // The sample positions do not depend on the opacity, so with PIPE sample
-  // k+1 is located and its loads issued before sample k is composited. The
-  // break conditions are evaluated in the reference's order for every sample;
-  // only o == 1 ends the march early, after which a prefetched sample is
-  // discarded.
-  // Empty macro-cells (occ == 0: every value there has TF alpha 0) are
-  // stepped over without a field fetch: such a sample leaves the state
-  // unchanged (Accum), so only its position update and break checks run. sk
-  // counts the samples skipped before the one returned; they are counted as
-  // marched once that sample is composited (or the ray ends on its own).
-  int b = g.light_budget;
-  // The first `fast` iterations are certain to pass the budget and distance
-  // tests, so they skip them. With u = 2^-24, after k steps the float position
-  // lies within k (step (1 + 4u) + 2 sqrt(3) u M) of the start (M bounds every
-  // |coordinate| on the segment), so |s - st|^2 <= len2 holds, rounding
-  // included, while k < (1 - 4u) (tmax - tmin) / (that per-step bound); the
-  // constants below double each u term, and two more steps are kept back.
-  int fast = 0;
-  {
-    const float dl = tmax - tmin;
-    if (dl > 0.f) {
-      const float M = fmaxf(fmaxf(fabsf(st[0]), fabsf(st[1])), fabsf(st[2])) + dl + g.step;
-      const float kf = (dl * 0.99999f) / (g.step * 1.00001f + 4e-7f * M);
-      if (kf > 2.f) fast = min((int)fminf(kf, 1e9f) - 2, b);
-    }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    dir[d] = v[d] * rs;
+    r.st[d] = L[d] + tmin * dir[d];
+    r.sd[d] = g.step * dir[d];
   }
-  b -= fast;
-  auto gen = [&](float v8[8], float pc[3], unsigned& sk) -> bool {
-    sk = 0;
+  const float dl = tmax - tmin;
+  r.len2 = dl * dl;
+  r.sure = 0;
+  if (dl > 0.f) {
+    const float M = fmaxf(fmaxf(fabsf(r.st[0]), fabsf(r.st[1])), fabsf(r.st[2])) + dl + g.step;
+    float k = __fdividef(dl * 0.99999f, g.step * 1.00001f + 4e-7f * M);
+    bool in = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const float room = r.sd[d] > 0.f ? g.maxp[d] - r.st[d] : r.st[d] - g.minp[d];
+      const float B = fmaxf(fabsf(g.minp[d]), fabsf(g.maxp[d]));
+      k = fminf(k, __fdividef(room * 0.99999f, fabsf(r.sd[d]) * 1.00001f + 1.2e-7f * B));
+      const float s1 = r.st[d] + r.sd[d];
+      in = in && s1 >= g.minp[d] && s1 <= g.maxp[d];
+    }
+    if (in && k > 3.f) r.sure = min((int)fminf(k, 1e6f) - 2, g.light_budget);
+  }
+  return r;
+}
+
+// What the march reads of one field: quads (or the plain field), the cell tables
+// and the TF table in shared memory, by 32-bit shared addresses biased so that
+// the bits of a cell guess (0x4B000000 + cell, see guess) index them directly.
+constexpr unsigned kGuessBias = 0x4B000000u;  // the bits of 2^23
+
+template <typename QuadT>
+struct LightField {
+  const QuadT* q;
+  const float4* T[3];
+  unsigned tab[3], val;  // biased shared addresses of T[d] and of the value table
+  const unsigned char* occ;
+  unsigned ox, oz, obias;
+
+  // vals: s_a (exact) or s_tau (precision).
+  __device__ __forceinline__ LightField(const ExactGeo& g, const QuadT* quads, const float4* s_tab, const float* vals,
+                                        const unsigned char* occupancy)
+      : q(quads), occ(occupancy) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      T[d] = s_tab + g.ax_off[d];
+      tab[d] = (unsigned)__cvta_generic_to_shared(T[d]) - (kGuessBias << 4);
+    }
+    val = (unsigned)__cvta_generic_to_shared(vals) - (kGuessBias << 2);
+    ox = (unsigned)g.occ_n[0];
+    oz = ox * (unsigned)g.occ_n[1];
+    obias = 0u - (kGuessBias >> kMacroLog2) * (1u + ox + oz);
+  }
+};
+
+// The guessed cell of s >= org on one axis as the bits 0x4B000000 + c: one
+// fused multiply-add rounded toward zero leaves floor((s - org) seed) in the
+// low mantissa bits of [2^23, 2^24). ExactGeo::seed keeps c <= n - 1 over the
+// volume, so c indexes the table (its closing entry included) unclamped.
+__device__ __forceinline__ unsigned guess(float s, float org, float seed) {
+  return __float_as_uint(__fmaf_rz(s - org, seed, 8388608.f));
+}
+__device__ __forceinline__ float4 ld_shared4(unsigned a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float ld_shared1(unsigned a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+
+// Three-way minimum and maximum (one instruction each); NaN if any operand is.
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// Corner values and parametric coordinates of the cell of s, whose guess is b. A
+// guess is the found cell unless s lies within an ulp of a cell face. The
+// parametric coordinates tell: s > lo exactly when its coordinate is > 0, and a
+// coordinate < 1 implies s < hi, so one minimum and one maximum test the three
+// axes (a NaN quotient fails); the rest takes the walk, out of line, and IEEE
+// divisions. The loads go out before the test; a wrong guess loads some cell in
+// vain.
+template <typename QuadT>
+__device__ __forceinline__ void sample_fetch(const ExactGeo& g, const LightField<QuadT>& F, const float s[3],
+                                             unsigned b0, unsigned b1, unsigned b2, float v[8], float p[3]) {
+  {
+    const float4 e0 = ld_shared4(F.tab[0] + (b0 << 4)), e1 = ld_shared4(F.tab[1] + (b1 << 4)),
+                 e2 = ld_shared4(F.tab[2] + (b2 << 4));
+    QuadLoad<QuadT>::cell(F.q, float_bits(e0.y) + float_bits(e1.y) + float_bits(e2.y), g.fs[1], g.fs[2], v);
+    // pcoords = (p - min) / (max - min) (RectilinearMeshOracle.h:189-192)
+    p[0] = div_field(s[0] - e0.x, e0);
+    p[1] = div_field(s[1] - e1.x, e1);
+    p[2] = div_field(s[2] - e2.x, e2);
+  }
+  if (!(min3(p[0], p[1], p[2]) > 0.f && max3(p[0], p[1], p[2]) < 1.f)) {
+    const int3 c = walk_cells_bsearch(F.T[0], F.T[1], F.T[2], g.n[0] - 2, g.n[1] - 2, g.n[2] - 2, s[0], s[1], s[2],
+                                      (int)(b0 - kGuessBias), (int)(b1 - kGuessBias), (int)(b2 - kGuessBias));
+    const float4 *e0 = F.T[0] + c.x, *e1 = F.T[1] + c.y, *e2 = F.T[2] + c.z;
+    QuadLoad<QuadT>::cell(F.q, float_bits(e0->y) + float_bits(e1->y) + float_bits(e2->y), g.fs[1], g.fs[2], v);
+    p[0] = (s[0] - e0->x) / (e0[1].x - e0->x);
+    p[1] = (s[1] - e1->x) / (e1[1].x - e1->x);
+    p[2] = (s[2] - e2->x) / (e2[1].x - e2->x);
+  }
+}
+template <typename QuadT>
+__device__ __forceinline__ float sample_finish(const ExactGeo& g, const LightField<QuadT>& F, const float v[8],
+                                               const float p[3]) {
+  float scalar = hex_interp(v, p[0], p[1], p[2]);
+  // TF index (TransmittanceMap.h:322-326): truncate, clamp to [0, n1], NaN -> 0.
+  // Saturating the normalised scalar to [0, 1] first gives the same index.
+  scalar = __saturatef((scalar - g.min_scalar) * g.inv_delta);
+  return ld_shared1(F.val + (__float_as_uint(__fadd_rz(scalar * g.n1f, 8388608.f)) << 2));
+}
+template <typename QuadT>
+__device__ __forceinline__ float sample_value(const ExactGeo& g, const LightField<QuadT>& F, const float s[3],
+                                              unsigned b0, unsigned b1, unsigned b2) {
+  float v[8], p[3];
+  sample_fetch(g, F, s, b0, b1, b2, v, p);
+  return sample_finish(g, F, v, p);
+}
+
+// The light march of one ray. ns counts the samples marched (skipped ones
+// included). sure: at most ray.sure. With SKIP, samples in empty macro-cells
+// (occ == 0: every value there has TF alpha 0, which leaves the state
+// unchanged, see Accum) take no field fetch.
+template <typename QuadT, bool PREC, bool SKIP>
+__device__ __forceinline__ void light_march(const ExactGeo& g, const LightField<QuadT>& F, const LightRay& ray,
+                                            int sure, Accum<PREC>& acc, unsigned& ns) {
+  float s[3] = {ray.st[0], ray.st[1], ray.st[2]};
+  if constexpr (!SKIP) {
+#pragma unroll 1
+    for (int k = 0; k < sure; ++k) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) s[d] = s[d] + ray.sd[d];
+      // stop when the accumulated value can no longer change (see Accum)
+      if (acc.add(sample_value(g, F, s, guess(s[0], g.org[0], g.seed[0]), guess(s[1], g.org[1], g.seed[1]),
+                               guess(s[2], g.org[2], g.seed[2])))) {
+        ns += (unsigned)k + 1u;
+        return;
+      }
+    }
+    unsigned n = (unsigned)sure;
+    for (int b = g.light_budget - sure; b > 0; --b) {
+      const float q0 = s[0] - ray.st[0], q1 = s[1] - ray.st[1], q2 = s[2] - ray.st[2];
+      if (!(q0 * q0 + q1 * q1 + q2 * q2 <= ray.len2)) break;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) s[d] = s[d] + ray.sd[d];
+      if (!inside_vol(g, s)) break;
+      ++n;
+      if (acc.add(sample_value(g, F, s, guess(s[0], g.org[0], g.seed[0]), guess(s[1], g.org[1], g.seed[1]),
+                               guess(s[2], g.org[2], g.seed[2]))))
+        break;
+    }
+    ns += n;
+  } else {
+    int k = 0;  // samples marched
     for (;;) {
-      if (fast > 0) {
-        --fast;
-      } else {
-        if (b-- <= 0) return false;
-        const float q0 = s[0] - st[0], q1 = s[1] - st[1], q2 = s[2] - st[2];
-        if (!(q0 * q0 + q1 * q1 + q2 * q2 <= len2)) return false;
-      }
-      s[0] = s[0] + sdx;
-      s[1] = s[1] + sdy;
-      s[2] = s[2] + sdz;
-      if (!inside_vol(g, s)) return false;
-      if (SKIP && !occupied(g, occ, s)) {
-        ++sk;
-        continue;
-      }
-      float4 e0, e1, e2;
-      int c0, c1, c2;
-      if constexpr (RECT) {
-        c0 = find_cell_bsearch_rect(T0, cm0, s[0], e0);
-        c1 = find_cell_bsearch_rect(T1, cm1, s[1], e1);
-        c2 = find_cell_bsearch_rect(T2, cm2, s[2], e2);
-      } else {
-        // s is inside the volume (tested above), so s - org >= 0 exactly and the
-        // seeded guesses need no lower clamp. A guess is the found cell unless s
-        // lies within an ulp of a cell face: one branch tests the three axes and
-        // the rare walk runs out of line, so the common path carries none of its
-        // code (the 257^3-vertex map of a 512^3 noise field: 2.66 -> 2.59 ms;
-        // the same walks inline behind one branch ran 2.75 ms, and three
-        // separate per-axis branches 2.66 ms)
-        c0 = trunc_small(fminf((s[0] - g.org[0]) * g.invh[0], REG_CONSTS ? (float)cm0 : g.cmaxf[0]));
-        c1 = trunc_small(fminf((s[1] - g.org[1]) * g.invh[1], REG_CONSTS ? (float)cm1 : g.cmaxf[1]));
-        c2 = trunc_small(fminf((s[2] - g.org[2]) * g.invh[2], REG_CONSTS ? (float)cm2 : g.cmaxf[2]));
-        e0 = T0[c0];
-        e1 = T1[c1];
-        e2 = T2[c2];
-        if ((s[0] <= e0.x) | (s[0] > e0.y) | (s[1] <= e1.x) | (s[1] > e1.y) | (s[2] <= e2.x) | (s[2] > e2.y)) {
-          if constexpr (PREC) {
-            // the precision march keeps the walks inline (out of line its
-            // 640^3 skipping build ran 1.5% slower)
-            while (c0 > 0 && s[0] <= e0.x) e0 = T0[--c0];
-            while (c0 < cm0 && s[0] > e0.y) e0 = T0[++c0];
-            while (c1 > 0 && s[1] <= e1.x) e1 = T1[--c1];
-            while (c1 < cm1 && s[1] > e1.y) e1 = T1[++c1];
-            while (c2 > 0 && s[2] <= e2.x) e2 = T2[--c2];
-            while (c2 < cm2 && s[2] > e2.y) e2 = T2[++c2];
-          } else {
-            const int3 cc = walk_cells_bsearch(T0, T1, T2, cm0, cm1, cm2, s[0], s[1], s[2], c0, c1, c2);
-            c0 = cc.x;
-            c1 = cc.y;
-            c2 = cc.z;
-            e0 = T0[c0];
-            e1 = T1[c1];
-            e2 = T2[c2];
+      unsigned b0, b1, b2;
+      for (;;) {  // on to the next sample in an occupied macro-cell
+        if (k >= sure) {
+          const float q0 = s[0] - ray.st[0], q1 = s[1] - ray.st[1], q2 = s[2] - ray.st[2];
+          if (k >= g.light_budget || !(q0 * q0 + q1 * q1 + q2 * q2 <= ray.len2)) {
+            ns += (unsigned)k;
+            return;
           }
         }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) s[d] = s[d] + ray.sd[d];
+        if (k >= sure && !inside_vol(g, s)) {
+          ns += (unsigned)k;
+          return;
+        }
+        ++k;
+        b0 = guess(s[0], g.org[0], g.seed[0]);
+        b1 = guess(s[1], g.org[1], g.seed[1]);
+        b2 = guess(s[2], g.org[2], g.seed[2]);
+        // the macro-cell comes from the guess; its occupancy covers a guess off by one
+        if (__ldg(F.occ + ((b2 >> kMacroLog2) * F.oz + ((b1 >> kMacroLog2) * F.ox + ((b0 >> kMacroLog2) + F.obias)))))
+          break;
       }
-      if constexpr (REG_CONSTS || std::is_same<QuadT, FieldF32>::value)
-        QuadLoad<QuadT>::cell(quads, (unsigned)c2 * qz + (unsigned)c1 * qx + (unsigned)c0, qx, qz, v8);
-      else  // the quad strides straight from the parameter space
-        QuadLoad<QuadT>::cell(quads, (unsigned)c2 * g.qzs + (unsigned)c1 * g.qxs + (unsigned)c0, g.qxs, g.qzs, v8);
-      // pcoords = (p - min) / (max - min) (RectilinearMeshOracle.h:189-192)
-      pc[0] = div_rn_markstein(s[0] - e0.x, e0.z, e0.w);
-      pc[1] = div_rn_markstein(s[1] - e1.x, e1.z, e1.w);
-      pc[2] = div_rn_markstein(s[2] - e2.x, e2.z, e2.w);
-      return true;
-    }
-  };
-  // TF index of a normalised scalar (TransmittanceMap.h:322-326)
-  auto tf_idx = [&](float scalar) {
-    return REG_CONSTS ? tf_index_clamped(scalar * (float)n1, n1) : tf_index_clamped_f(scalar * g.n1f, g.n1f);
-  };
-  acc.init(prefix(dir));
-  float va[8], pa[3];
-  unsigned ska;
-  if constexpr (!PIPE) {
-    // Every gen() call takes one step (fast or b), so the samples marched are
-    // the steps taken less a failing last one: the precision march counts them
-    // so at the end (its 640^3 build 6.06 -> 5.96 ms); the exact march counts
-    // per sample, which runs faster there (2.38 against 2.42 ms).
-    const int steps0 = fast + b;
-    for (;;) {
-      if (!gen(va, pa, ska)) {
-        if constexpr (PREC) ns += (unsigned)(steps0 - (fast + b) - 1);
-        else ns += ska;  // skipped samples before the end of the ray
-        break;
-      }
-      float scalar = hex_interp(va, pa[0], pa[1], pa[2]);
-      scalar = (scalar - g.min_scalar) * g.inv_delta;
-      if constexpr (!PREC) ns += 1 + ska;
-      // Stop when the accumulated value can no longer change (see Accum).
-      if (acc.add(s_a, s_tau, tf_idx(scalar))) {
-        if constexpr (PREC) ns += (unsigned)(steps0 - (fast + b));
-        break;
+      if (acc.add(sample_value(g, F, s, b0, b1, b2))) {
+        ns += (unsigned)k;
+        return;
       }
     }
-    return;
   }
-  static_assert(!PIPE || SKIP, "the two-sample pipeline is written for the skipping march");
-  float vb[8], pb[3];
-  unsigned skb;
-  bool ok = gen(va, pa, ska);
-  if (!ok) ns += ska;
-  while (ok) {
-    const bool okb = gen(vb, pb, skb);
-    bool done;
-    {
-      float scalar = hex_interp(va, pa[0], pa[1], pa[2]);
-      scalar = (scalar - g.min_scalar) * g.inv_delta;
-      done = acc.add(s_a, s_tau, tf_idx(scalar));
-      ns += 1 + ska;
+}
+
+// The same for explicit rectilinear coordinates, where no guess from a uniform
+// spacing is close: binary-search cell location over the cell tables.
+__device__ __forceinline__ void light_march_rect(const ExactGeo& g, const float4* __restrict__ quads,
+                                                 const float4* s_tab, const float* s_a, const LightRay& ray,
+                                                 Accum<false>& acc, unsigned& ns) {
+  float s[3] = {ray.st[0], ray.st[1], ray.st[2]};
+  const int n1 = g.tf_n - 1;
+  for (int b = g.light_budget; b > 0; --b) {
+    const float q0 = s[0] - ray.st[0], q1 = s[1] - ray.st[1], q2 = s[2] - ray.st[2];
+    if (!(q0 * q0 + q1 * q1 + q2 * q2 <= ray.len2)) break;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) s[d] = s[d] + ray.sd[d];
+    if (!inside_vol(g, s)) break;
+    float pc[3];
+    unsigned qi = 0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const float4* T = s_tab + g.ax_off[d];
+      float4 e;
+      const int c = find_cell_bsearch_rect(T, g.n[d] - 2, s[d], e);
+      qi += float_bits(e.y);
+      pc[d] = div_field(s[d] - e.x, e);
+      if (pc[d] != pc[d]) pc[d] = (s[d] - e.x) / (T[c + 1].x - e.x);
     }
-    // Stop when the accumulated value can no longer change (see Accum).
-    if (done) break;
-    if (!okb) {
-      ns += skb;
-      break;
-    }
-    ok = gen(va, pa, ska);
-    {
-      float scalar = hex_interp(vb, pb[0], pb[1], pb[2]);
-      scalar = (scalar - g.min_scalar) * g.inv_delta;
-      done = acc.add(s_a, s_tau, tf_idx(scalar));
-      ns += 1 + skb;
-    }
-    if (done) break;
-    if (!ok) ns += ska;
+    float v[8];
+    QuadLoad<float4>::cell(quads, qi, g.fs[1], g.fs[2], v);
+    float scalar = hex_interp(v, pc[0], pc[1], pc[2]);
+    scalar = (scalar - g.min_scalar) * g.inv_delta;
+    ++ns;
+    if (acc.add(s_a[tf_index_clamped(scalar * (float)n1, n1)])) break;
   }
 }
 

@@ -119,7 +119,7 @@ __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT*
             e = T[c[k]];
           } else {
             c[k] = find_cell_walk_rect(T, g.n[k] - 2, p[k], e);
-            inv[k] = e.w;  // 1.f / (coord(c+1) - coord(c)), IEEE
+            inv[k] = e.z;  // 1.f / (coord(c+1) - coord(c)), IEEE
           }
           bl[k] = e.x;
         }
