@@ -27,11 +27,13 @@ struct BatchVolume {
   beams_volume vol{};
   void* owned = nullptr;         // device copy of a host field
   float4* quads = nullptr;       // float32 4-corner quads
-  unsigned char* occ = nullptr;  // macro-cell occupancy under occ_tf (empty-space skipping)
+  void* ranges = nullptr;        // value ranges of the quads' macro-cells
+  unsigned char* occ = nullptr;  // their distances under occ_tf (empty-space skipping)
   unsigned long long occ_tf = ~0ull;
   ~BatchVolume() {
     if (owned) cudaFree(owned);
     if (quads) cudaFree(quads);
+    if (ranges) cudaFree(ranges);
     if (occ) cudaFree(occ);
   }
 };
@@ -152,7 +154,9 @@ beams_status beams_batch_set_volumes(beams_renderer* r, const beams_volume* vols
     }
     const size_t nq = (size_t)(vols[i].dims[0] - 1) * (vols[i].dims[1] - 1) * vols[i].dims[2];
     if (e == cudaSuccess) e = cudaMalloc((void**)&bv->quads, nq * sizeof(float4));
-    if (e == cudaSuccess) e = launch_build_quads(bv->vol.data, BEAMS_F32, bv->quads, BEAMS_F32, vols[i].dims, r->stream);
+    if (e == cudaSuccess) e = cudaMalloc(&bv->ranges, macro_bytes(vols[i].dims));
+    if (e == cudaSuccess)
+      e = launch_build_quads(bv->vol.data, BEAMS_F32, bv->quads, BEAMS_F32, vols[i].dims, bv->ranges, r->stream);
     if (e != cudaSuccess) {
       for (auto* v : b->vols) delete v;
       b->vols.clear();
@@ -226,7 +230,8 @@ beams_status beams_render_batch(beams_renderer* r, const beams_request* reqs, in
     r->cutoff = q.termination_alpha;
     r->use_map = true;
     s = make_geo_vol(r, b->vols[q.volume]->vol, &q.camera, geos[i]);
-    if (s == BEAMS_OK && (size_t)(geos[i].ntab + 2 * r->tf_n) * 16 > 200 * 1024)
+    // (the tables' six entries past the axes' cells are not counted against the limit)
+    if (s == BEAMS_OK && (size_t)(geos[i].ntab - 6 + 2 * r->tf_n) * 16 > 200 * 1024)
       s = fail(r, BEAMS_ERR_UNSUPPORTED, "render_batch: volume/map axes too long for the shared cell tables");
     const bool direct = q.out_on_device && (((uintptr_t)q.rgba_out & 15) == 0);
     sig.push_back(q.volume);
@@ -253,8 +258,8 @@ beams_status beams_render_batch(beams_renderer* r, const beams_request* reqs, in
       ExactGeo g;
       s = make_geo_vol(r, bv->vol, nullptr, g);
       if (s != BEAMS_OK) return s;
-      if (!bv->occ) e = cudaMalloc((void**)&bv->occ, (size_t)g.occ_n[0] * g.occ_n[1] * g.occ_n[2]);
-      if (e == cudaSuccess) e = launch_build_occupancy(g, BEAMS_F32, bv->quads, r->d_tf, bv->occ, r->stream);
+      if (!bv->occ) e = cudaMalloc((void**)&bv->occ, occupancy_bytes(g.n));
+      if (e == cudaSuccess) e = launch_build_occupancy(g, bv->ranges, r->d_tf, bv->occ, r->stream);
       if (e != cudaSuccess) return cuda_fail(r, e, "render_batch: occupancy build");
       bv->occ_tf = r->tf_version;
     }

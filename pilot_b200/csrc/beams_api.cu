@@ -179,6 +179,11 @@ beams_status make_geo_vol(beams_renderer* r, const beams_volume& v, const beams_
     for (int l = 0; l < g.n_lights; ++l)
       for (int d = 0; d < 3; ++d) g.light_colors[l][d] = r->lights[l].color[d] * r->lights[l].intensity;
   }
+  bool tame = true;  // the colour map's entries are finite (beams_set_color_map)
+  for (int i = 0; i < r->tf_n; ++i) tame = tame && r->tf[4 * i + 3] >= 0.f;
+  for (int l = 0; l < g.n_lights; ++l)
+    for (int d = 0; d < 3; ++d) tame = tame && std::fabs(g.light_colors[l][d]) <= 1e30f;
+  g.tame = tame ? 1 : 0;
   int off = 0;
   for (int d = 0; d < 3; ++d) {
     g.ax_off[d] = off;
@@ -186,7 +191,7 @@ beams_status make_geo_vol(beams_renderer* r, const beams_volume& v, const beams_
   }
   for (int d = 0; d < 3; ++d) {
     g.max_off[d] = off;
-    off += r->map_m[d];
+    off += g.pd[d];  // M cells and the last one again (table_entry)
   }
   g.ntab = off;
   geo_loop_constants(g, true);
@@ -327,7 +332,7 @@ static beams_status prepare_layouts_for(beams_renderer* r, const ExactGeo& g, in
     const size_t nq = (size_t)(g.n[0] - 1) * (g.n[1] - 1) * g.n[2];
     beams_status s = ensure_buffer(r, (void**)d_quads, quads_cap, nq * sizeof(float4), "allocating quad field");
     if (s != BEAMS_OK) return s;
-    cudaError_t e = launch_build_quads(d_field, BEAMS_F32, *d_quads, BEAMS_F32, g.n, r->stream);
+    cudaError_t e = launch_build_quads(d_field, BEAMS_F32, *d_quads, BEAMS_F32, g.n, nullptr, r->stream);
     if (e != cudaSuccess) return cuda_fail(r, e, "quad field build");
     ++launches;
     *quads_version = version;
@@ -376,25 +381,28 @@ beams_status prepare_layouts(beams_renderer* r, const ExactGeo& g, int& launches
     const size_t qbytes = (qd == BEAMS_F32) ? sizeof(float4) : 8;
     beams_status s = ensure_buffer(r, (void**)&r->d_quads, &r->quads_cap, nq * qbytes, "allocating quad field");
     if (s != BEAMS_OK) return s;
-    cudaError_t e = launch_build_quads(r->d_field, r->vol.dtype, r->d_quads, qd, g.n, r->stream);
+    // the macro-cells' ranges with them: they describe these quads, whatever becomes of the field
+    s = ensure_buffer(r, (void**)&r->d_ranges, &r->ranges_cap, macro_bytes(g.n), "allocating macro-cell ranges");
+    if (s != BEAMS_OK) return s;
+    r->quads_version = 0;  // not these quads until both launches are queued
+    cudaError_t e = launch_build_quads(r->d_field, r->vol.dtype, r->d_quads, qd, g.n, r->d_ranges, r->stream);
     if (e != cudaSuccess) return cuda_fail(r, e, "quad field build");
-    ++launches;
+    launches += 2;
     r->quads_version = qkey;
   }
   return BEAMS_OK;
 }
 
-// Occupancy of the current quads under the current colour map (rebuilt when either changes).
+// Empty space of the current quads under the current colour map (rebuilt when either changes).
 beams_status prepare_occupancy(beams_renderer* r, const ExactGeo& g, int& launches) {
   const int qd = quad_dtype(r);
   const unsigned long long key[2] = {r->volume_version * 4ull + (unsigned long long)qd, r->tf_version};
   if (key[0] == r->occ_key[0] && key[1] == r->occ_key[1]) return BEAMS_OK;
-  const size_t nm = (size_t)g.occ_n[0] * g.occ_n[1] * g.occ_n[2];
-  beams_status s = ensure_buffer(r, (void**)&r->d_occ, &r->occ_cap, nm, "allocating occupancy grid");
+  beams_status s = ensure_buffer(r, (void**)&r->d_occ, &r->occ_cap, occupancy_bytes(g.n), "allocating occupancy grid");
   if (s != BEAMS_OK) return s;
-  cudaError_t e = launch_build_occupancy(g, qd, r->d_quads, r->d_tf, r->d_occ, r->stream);
+  cudaError_t e = launch_build_occupancy(g, r->d_ranges, r->d_tf, r->d_occ, r->stream);
   if (e != cudaSuccess) return cuda_fail(r, e, "occupancy build");
-  ++launches;
+  launches += 4;
   r->occ_key[0] = key[0];
   r->occ_key[1] = key[1];
   return BEAMS_OK;

@@ -43,8 +43,8 @@ struct ExactGeo {
   int slab_fp64;
   int use_map;
   int assoc_cells;
-  // Cell tables: per axis, one float4 {lo, hi, RN(1/(hi-lo)), 0} per cell, field
-  // axes first (n-1 cells each), then map axes (M cells each).
+  // Cell tables: one float4 entry per cell and one more per axis, field axes
+  // first (n entries each), then map axes (M + 1 each); see table_entry.
   int ax_off[3];   // offset of field axis d in the table
   int max_off[3];  // offset of map axis d in the table
   int ntab;        // total table entries
@@ -60,7 +60,7 @@ struct ExactGeo {
   // the same map.
   int bo_axis[3];
   int bo_shear[2];
-  // Occupancy of 8^3-cell macro-cells (empty-space skipping): counts per axis.
+  // Macro-cells of 8^3 cells (empty-space skipping): counts per axis.
   int occ_n[3];
   // The multi-light extension: n_lights maps, map l at map + l * (M+1)^3, the
   // view march shading by sum_l T_l * light_colors[l] (n_lights <= 1: light 0 only).
@@ -80,6 +80,9 @@ struct ExactGeo {
   // quads' {1, n0 - 1, (n0 - 1)(n1 - 1)}, or the plain field's (set by
   // geo_loop_constants); cell (x, y, z) is entry fs . (x, y, z).
   unsigned fs[3];
+  // 1: no shading can be NaN (colour map and light colours finite, alphas >= 0),
+  // so a sample of alpha 0 adds nothing and clamping is saturation.
+  int tame;
   // Pixel window {x0, y0, w, h} the (non-listed) view march covers; the whole
   // image unless a brick's projection is known to lie inside a smaller one
   // (every pixel outside it misses the volume).
@@ -143,14 +146,6 @@ __host__ __device__ inline float bits_float(unsigned u) {
 #endif
 }
 
-// Map axes' cell table entry: {lo, w, rh, rl} of the cell [lo, hi], w = hi - lo,
-// rh = RN(1/w) and rl = RN((1 - w rh) / w) (the residual is exact), so rh + rl
-// is 1/w to 48 bits.
-__host__ __device__ inline float4 cell_entry(float lo, float hi) {
-  const float w = hi - lo, rh = 1.f / w;
-  return make_float4(lo, w, rh, fmaf(-w, rh, 1.f) / w);
-}
-
 // Whether fma(x, rh, x rl) is the correctly rounded x / w for every x, given
 // |rh + rl - 1/w| <= 7 * 2^-48 / w. The sum is x / w to 2^-45 before its one
 // rounding, so it can only round wrongly when a midpoint of two floats lies
@@ -184,8 +179,9 @@ __host__ __device__ inline bool two_term_division_exact(float w, float rh, float
   return true;
 }
 
-// Field axes' cell table entry: {lo, offset, rh, rl} of the cell [lo, hi]; offset
-// (its bits) = the cell's term of the quad index. rl is the one of seven
+// Cell table entry {lo, offset, rh, rl} of the cell [lo, hi], w = hi - lo: offset
+// (its bits) = the cell's term of the quad (field axes) or vertex (map axes)
+// index, rh = RN(1/w), and rl is the one of seven
 // neighbouring values, nearest to (1 - w rh) / w first, with which fma(x, rh, x
 // rl) is the correctly rounded quotient x / w for every x, or NaN when there is
 // none (the marches then divide).
@@ -205,9 +201,10 @@ __host__ __device__ inline float4 field_entry(float lo, float hi, unsigned offse
   }
   return make_float4(lo, bits_float(offset), rh, rl);
 }
-// The entry after an axis's last cell: the last coordinate, and that cell's offset.
+// The entry after a field axis's last cell: the last coordinate, that cell's
+// offset (a load in bounds) and NaN, so that no position looks inside it.
 __host__ __device__ inline float4 closing_entry(float lo, unsigned offset) {
-  return make_float4(lo, bits_float(offset), 1.f, 0.f);
+  return make_float4(lo, bits_float(offset), NAN, NAN);
 }
 
 // Slots of the light-aligned vertex order with groups of 2^bl x 2^bl columns

@@ -162,7 +162,7 @@ __device__ __forceinline__ void light_origin(const ExactGeo& g, const float V[3]
 // Entry i of the cell tables: per field axis its n - 1 cells (field_entry) and a
 // closing entry whose lo is the last coordinate (so a cell's upper coordinate is
 // the next entry's lo, and a guess one past the last cell reads a valid entry);
-// past max_off[0] the map axes' cells (cell_entry).
+// past max_off[0] the map axes' cells, the last one twice (see map_cell).
 __device__ __forceinline__ float4 table_entry(const ExactGeo& g, int i) {
   if (i < g.max_off[0]) {
     const int d = (i >= g.ax_off[2]) ? 2 : (i >= g.ax_off[1] ? 1 : 0);
@@ -172,8 +172,9 @@ __device__ __forceinline__ float4 table_entry(const ExactGeo& g, int i) {
                           : closing_entry(lo, (unsigned)(c - 1) * g.fs[d]);
   }
   const int d = (i >= g.max_off[2]) ? 2 : (i >= g.max_off[1] ? 1 : 0);
-  const int c = i - g.max_off[d];
-  return cell_entry(vtx_coord(g, d, c), vtx_coord(g, d, c + 1));
+  const int c = min(i - g.max_off[d], g.pd[d] - 2);
+  const unsigned stride = d == 0 ? 1u : (d == 1 ? (unsigned)g.pd[0] : (unsigned)g.pd[0] * (unsigned)g.pd[1]);
+  return field_entry(vtx_coord(g, d, c), vtx_coord(g, d, c + 1), (unsigned)c * stride);
 }
 
 // (int)x for x in [0, 2^23), computed on the FMA pipe instead of the
@@ -184,21 +185,8 @@ __device__ __forceinline__ int trunc_small(float x) {
   return __float_as_int(__fadd_rz(x, 8388608.f)) - 0x4B000000;
 }
 
-// Correctly rounded division x / w for the map cell entry e = {lo, w, rh, rl}. q =
-// fma(x, rh, x rl) is x / w to 2^-47 before its one rounding, hence faithful;
-// then the residual x - q w is exact under fma and, by Markstein's theorem (P.
-// Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", IBM J. Res. Dev. 34(1), 1990: rh the correctly rounded
-// reciprocal, q faithful), RN(q + residual rh) is the correctly rounded
-// quotient. Valid for normal operands whose quotient neither overflows nor
-// underflows, which holds for the parametric coordinates here (|x| <= 2w, w a
-// cell width); beams_selftest_division checks it against IEEE division.
-__device__ __forceinline__ float div_cell(float x, const float4& e) {
-  const float q = fmaf(x, e.z, x * e.w);
-  return fmaf(fmaf(-q, e.y, x), e.z, q);
-}
-// The same for a field cell entry, whose rl makes the two-term product itself the
-// correctly rounded quotient (field_entry), in two operations; NaN when it cannot.
+// Correctly rounded division x / w for the cell entry e = {lo, offset, rh, rl} of
+// width w in two operations (see field_entry); NaN when two terms do not suffice.
 __device__ __forceinline__ float div_field(float x, const float4& e) { return fmaf(x, e.z, x * e.w); }
 
 // Light-march cell search: RectilinearMeshOracle's binary search
@@ -265,6 +253,7 @@ __device__ __forceinline__ int find_cell_walk_t(const float4* T, int cmax, float
 // The view march's walk (the unique c with coord(c) <= p < coord(c+1)) that
 // settles seeded guesses off by a face, out of line like walk_cells_bsearch.
 static __device__ __noinline__ int walk_cell_view(const float4* T, int cmax, float p, int c) {
+  c = min(c, cmax);
   while (c > 0 && p < T[c].x) --c;
   while (c < cmax && p >= T[c + 1].x) ++c;
   return c;
@@ -275,53 +264,11 @@ static __device__ __noinline__ int3 walk_cells_view(const float4* T0, const floa
   return make_int3(walk_cell_view(T0, m0, v0, c0), walk_cell_view(T1, m1, v1, c1), walk_cell_view(T2, m2, v2, c2));
 }
 
-// The view march's cell location on a uniform grid when a sample leaves its
-// cell (RectilinearLocator::LocateCell, LightedVolumeRenderer.cxx:119-165):
-// seeded guesses, one branch testing the three axes, the rare walk out of line.
-// On a max face the cell is the last one and inv[k] is left as it was (the
-// reference keeps the previous invSpacing there); bl[k] = the cell's lower
-// coordinate.
-__device__ __forceinline__ void locate_view_cell(const ExactGeo& g, const float4* s_tab, const float p[3], int c[3],
-                                                 float inv[3], float bl[3]) {
-  float4 e[3];
-  bool off = false;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    c[k] = trunc_small(fminf(fmaxf((p[k] - g.org[k]) * g.invh[k], 0.f), (float)(g.n[k] - 2)));
-    const float4* T = s_tab + g.ax_off[k] + c[k];
-    e[k] = T[0];
-    off = off | (p[k] < e[k].x) | (p[k] >= T[1].x);
-  }
-  if (off) {
-    const int3 cc = walk_cells_view(s_tab + g.ax_off[0], s_tab + g.ax_off[1], s_tab + g.ax_off[2], g.n[0] - 2,
-                                    g.n[1] - 2, g.n[2] - 2, p[0], p[1], p[2], c[0], c[1], c[2]);
-    c[0] = cc.x;
-    c[1] = cc.y;
-    c[2] = cc.z;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) e[k] = s_tab[g.ax_off[k] + c[k]];
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    if (p[k] == g.maxp[k]) {
-      c[k] = g.n[k] - 2;
-      e[k] = s_tab[g.ax_off[k] + c[k]];
-    } else {
-      inv[k] = e[k].z;  // 1.f / (coord(c+1) - coord(c)), IEEE
-    }
-    bl[k] = e[k].x;
-  }
-}
-
 // TF index of the light march (TransmittanceMap.h:322-326): truncate, clamp to
 // [0, n1]; saturating, NaN -> 0. Clamping in float first gives the same index:
 // (-1, 0) truncates to 0 either way and [n1, n1+1) to n1.
 __device__ __forceinline__ int tf_index_clamped(float fi, int n1) {
   return trunc_small(fminf(fmaxf(fi, 0.f), (float)n1));
-}
-// The same with the top index given as a float (n1f = (float)n1).
-__device__ __forceinline__ int tf_index_clamped_f(float fi, float n1f) {
-  return trunc_small(fminf(fmaxf(fi, 0.f), n1f));
 }
 
 // Pinhole camera ray through pixel centre (x, y).
@@ -388,67 +335,6 @@ __device__ __forceinline__ bool inside_vol(const ExactGeo& g, const float p[3]) 
 template <typename MapT> __device__ __forceinline__ float ld_map(const MapT* p);
 template <> __device__ __forceinline__ float ld_map<float>(const float* p) { return __ldg(p); }
 template <> __device__ __forceinline__ float ld_map<__half>(const __half* p) { return __half2float(__ldg(p)); }
-
-// TransmittanceLocator::LocateCell + GetEstimateUsingVerticesT
-// (TransmittanceMap.h:93-112, :200-229): the map value interpolated at p
-// (opacity in the exact form, transmittance in the precision form).
-// MT = map cell tables.
-template <typename MapT>
-__device__ __forceinline__ float map_interp_t(const ExactGeo& g, const float4* MT, const MapT* __restrict__ map,
-                                              const float p[3]) {
-  int c[3];
-  float pc[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    // the reference clamps t to [0, pd-2] when t >= pd-1 and truncates; the
-    // cell is the same as truncating min(max(t, 0), pd-2)
-    const float t = (p[d] - g.morig[d]) * g.minv[d];
-    c[d] = trunc_small(fminf(fmaxf(t, 0.f), (float)(g.pd[d] - 2)));
-    const float4 e = MT[g.max_off[d] + c[d]];
-    pc[d] = div_cell(p[d] - e.x, e);
-  }
-  const unsigned px = (unsigned)g.pd[0], pxy = (unsigned)g.pd[0] * (unsigned)g.pd[1];
-  const MapT* m = map + ((unsigned)c[2] * pxy + (unsigned)c[1] * px + (unsigned)c[0]);
-  float v[8];
-  v[0] = ld_map(m);
-  v[1] = ld_map(m + 1);
-  v[2] = ld_map(m + 1 + px);
-  v[3] = ld_map(m + px);
-  v[4] = ld_map(m + pxy);
-  v[5] = ld_map(m + pxy + 1);
-  v[6] = ld_map(m + pxy + 1 + px);
-  v[7] = ld_map(m + pxy + px);
-  return hex_interp(v, pc[0], pc[1], pc[2]);
-}
-
-// The multi-light shading term at p: sum over the maps of (1 - opacity_l) *
-// light_colors[l], in light order. The cell and parametric coordinates are the
-// same for every map (one map grid), so they are located once.
-__device__ __forceinline__ void map_light_sum(const ExactGeo& g, const float4* MT, const float* __restrict__ map,
-                                              const float p[3], float est[3]) {
-  int c[3];
-  float pc[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const float t = (p[d] - g.morig[d]) * g.minv[d];
-    c[d] = trunc_small(fminf(fmaxf(t, 0.f), (float)(g.pd[d] - 2)));
-    const float4 e = MT[g.max_off[d] + c[d]];
-    pc[d] = div_cell(p[d] - e.x, e);
-  }
-  const unsigned px = (unsigned)g.pd[0], pxy = (unsigned)g.pd[0] * (unsigned)g.pd[1];
-  const size_t nv = (size_t)pxy * (unsigned)g.pd[2];
-  const float* m = map + ((unsigned)c[2] * pxy + (unsigned)c[1] * px + (unsigned)c[0]);
-  for (int l = 0; l < g.n_lights; ++l, m += nv) {
-    const float v[8] = {__ldg(m), __ldg(m + 1), __ldg(m + 1 + px), __ldg(m + px),
-                        __ldg(m + pxy), __ldg(m + pxy + 1), __ldg(m + pxy + 1 + px), __ldg(m + pxy + px)};
-    const float tr = 1.f - hex_interp(v, pc[0], pc[1], pc[2]);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const float t = tr * g.light_colors[l][d];
-      est[d] = (l == 0) ? t : est[d] + t;
-    }
-  }
-}
 
 // Shared-memory form of the marked-vertex listing's brick order, bricks of
 // 2^bl vertices per edge: {nb_w, nb_u, nb_v, axis_w, axis_u, axis_v, shear_u, shear_v}.
@@ -588,19 +474,6 @@ template <> struct QuadLoad<float4> {
     v[4] = b.x; v[5] = b.y; v[6] = b.w; v[7] = b.z;
   }
 };
-
-// Whether the macro-cell holding p may hold a non-zero TF alpha. The macro
-// index comes from the approximate cell (p - org) / h; the occupancy of macro
-// m covers cells [8m - 1, 8m + 8], so a cell search off by one stays covered.
-__device__ __forceinline__ bool occupied(const ExactGeo& g, const unsigned char* __restrict__ occ, const float p[3]) {
-  int m[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const float f = fminf(fmaxf((p[d] - g.org[d]) * g.invh[d], 0.f), (float)(g.n[d] - 2));
-    m[d] = trunc_small(f) >> kMacroLog2;
-  }
-  return __ldg(occ + ((size_t)m[2] * g.occ_n[1] + m[1]) * g.occ_n[0] + m[0]) != 0;
-}
 
 // Warp-aggregated counter increment (one atomic per warp). Must be reached by
 // all 32 lanes of the warp (kernels keep out-of-range lanes alive with v = 0);

@@ -20,6 +20,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "cell_tables.cuh"
 #include "exact_device.cuh"
 #include "kernels.h"
 #include "mlp_common.cuh"
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(256, 2) k_view_march_mlp(const ExactGeo g, con
   const int tiles_x = (g.width + 7) >> 3;
   const int nprobe = probe.nqx * probe.nqy;
   const int ntiles = pass.probes_only ? (nprobe + 31) >> 5 : tiles_x * ((g.height + 3) >> 2);
-  const unsigned qx = (unsigned)(g.n[0] - 1), qz = (unsigned)(g.n[0] - 1) * (unsigned)(g.n[1] - 1);
+  const CellTables cells(g, s_tab);
   const int n1 = g.tf_n - 1;
   unsigned lit = 0, hit = 0, evals = 0, rows = 0;
   for (int tile = next_warp_tile_mlp(&cnt->tiles_view); tile < ntiles; tile = next_warp_tile_mlp(&cnt->tiles_view)) {
@@ -280,8 +281,7 @@ __global__ void __launch_bounds__(256, 2) k_view_march_mlp(const ExactGeo g, con
     }
     const float sdx = g.sd * d[0], sdy = g.sd * d[1], sdz = g.sd * d[2];
     float bl[3] = {0.f, 0.f, 0.f}, inv[3] = {0.f, 0.f, 0.f};
-    bool newCell = true;
-    float tx = 0.f, ty = 0.f, tz = 0.f;
+    float tx = 2.f, ty = 2.f, tz = 2.f;  // outside any cell: the first sample locates its cell
     float s0 = 0.f, s1m0 = 0.f, s2m3 = 0.f, s3 = 0.f, s4 = 0.f, s5m4 = 0.f, s6m7 = 0.f, s7 = 0.f;
     float Tprev = 1.f;
     bool have_prev = false;
@@ -300,14 +300,12 @@ __global__ void __launch_bounds__(256, 2) k_view_march_mlp(const ExactGeo g, con
           done = true;
           break;
         }
-        const float mint = mn(tx, mn(ty, tz));
-        const float maxt = mx(tx, mx(ty, tz));
-        if (maxt > 1.f || mint < 0.f) newCell = true;
-        if (newCell) {
-          int c[3];
-          locate_view_cell(g, s_tab, p, c, inv, bl);
+        if (!(min3(tx, ty, tz) >= 0.f && max3(tx, ty, tz) <= 1.f)) {
+          const unsigned off =
+              locate_view_cell(g, cells, p, guess(p[0], g.org[0], g.seed[0]), guess(p[1], g.org[1], g.seed[1]),
+                               guess(p[2], g.org[2], g.seed[2]), inv, bl, tx, ty, tz);
           float v[8];
-          QuadLoad<QuadT>::cell(quads, (unsigned)c[2] * qz + (unsigned)c[1] * qx + (unsigned)c[0], qx, qz, v);
+          QuadLoad<QuadT>::cell(quads, off, g.fs[1], g.fs[2], v);
           s0 = v[0];
           s3 = v[3];
           s4 = v[4];
@@ -316,10 +314,6 @@ __global__ void __launch_bounds__(256, 2) k_view_march_mlp(const ExactGeo g, con
           s5m4 = v[5] - v[4];
           s1m0 = v[1] - v[0];
           s2m3 = v[2] - v[3];
-          tx = (p[0] - bl[0]) * inv[0];
-          ty = (p[1] - bl[1]) * inv[1];
-          tz = (p[2] - bl[2]) * inv[2];
-          newCell = false;
         }
         const float l76 = s7 + tx * s6m7;
         const float l45 = s4 + tx * s5m4;

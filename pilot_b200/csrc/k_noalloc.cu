@@ -188,7 +188,7 @@ extern "C" beams_status beams_render_noalloc(const beams_volume* vol, const floa
     }
     for (int d = 0; d < 3; ++d) {
       g.max_off[d] = off;
-      off += map_cells;
+      off += map_cells + 1;
     }
     g.ntab = off;
   }

@@ -9,8 +9,11 @@
 namespace beams {
 
 cudaError_t launch_build_tables(const ExactGeo& g, float4* tab, cudaStream_t st);
+// The quads of a field and (ranges non-null: macro_bytes(n) of device memory) the
+// value ranges of its macro-cells, which launch_build_occupancy reads.
 cudaError_t launch_build_quads(const void* field, int in_dtype, void* quads, int quad_dtype, const int n[3],
-                               cudaStream_t st);
+                               void* ranges, cudaStream_t st);
+size_t macro_bytes(const int n[3]);
 cudaError_t launch_light_march_prec(const ExactGeo& g, int quad_dtype, const void* quads, const float4* tab,
                                     const float4* tf, const float* tau, __half* map, Counters* cnt, cudaStream_t st,
                                     const unsigned char* occ = nullptr, const unsigned* vlist = nullptr);
@@ -29,10 +32,14 @@ cudaError_t launch_light_march_f32(const ExactGeo& g, const float4* quads, const
 size_t marked_list_bytes(const int pd[3]);
 cudaError_t launch_list_marked_vertices(const ExactGeo& g, const unsigned char* cell_mask, const unsigned* gate,
                                         unsigned* list, cudaStream_t st);
-// Empty-space occupancy of 8^3-cell macro-cells for the light march's skip.
+// Empty space: per 8^3-cell macro-cell its distance in macro-cells to the nearest
+// one that is not empty under the colour map (0: not empty itself), from the
+// ranges of launch_build_quads. occ spans occupancy_bytes(n) (the distances, then
+// scratch). Four kernels.
 void occupancy_dims(const int n[3], int occ_n[3]);
-cudaError_t launch_build_occupancy(const ExactGeo& g, int quad_dtype, const void* quads, const float4* tf,
-                                   unsigned char* occ, cudaStream_t st);
+size_t occupancy_bytes(const int n[3]);
+cudaError_t launch_build_occupancy(const ExactGeo& g, const void* ranges, const float4* tf, unsigned char* occ,
+                                   cudaStream_t st);
 // Learned form's lazy fallback (k_mlp_probe.cu): when the list of failing tiles
 // is non-empty, clears the cell mask (one byte per map cell, rounded up to a
 // 16-byte multiple) and marks the map cells that the listed tiles' view rays

@@ -9,6 +9,7 @@
 
 #include <type_traits>
 
+#include "cell_tables.cuh"
 #include "exact_device.cuh"
 
 namespace beams {
@@ -109,63 +110,18 @@ __device__ __forceinline__ LightRay light_ray(const ExactGeo& g, const float V[3
 }
 
 // What the march reads of one field: quads (or the plain field), the cell tables
-// and the TF table in shared memory, by 32-bit shared addresses biased so that
-// the bits of a cell guess (0x4B000000 + cell, see guess) index them directly.
-constexpr unsigned kGuessBias = 0x4B000000u;  // the bits of 2^23
-
+// and the value table in shared memory, and the macro-cells' distances.
 template <typename QuadT>
 struct LightField {
   const QuadT* q;
-  const float4* T[3];
-  unsigned tab[3], val;  // biased shared addresses of T[d] and of the value table
+  CellTables cells;
+  unsigned val;  // biased shared address of the value table: s_a (exact) or s_tau (precision)
   const unsigned char* occ;
-  unsigned ox, oz, obias;
 
-  // vals: s_a (exact) or s_tau (precision).
   __device__ __forceinline__ LightField(const ExactGeo& g, const QuadT* quads, const float4* s_tab, const float* vals,
                                         const unsigned char* occupancy)
-      : q(quads), occ(occupancy) {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      T[d] = s_tab + g.ax_off[d];
-      tab[d] = (unsigned)__cvta_generic_to_shared(T[d]) - (kGuessBias << 4);
-    }
-    val = (unsigned)__cvta_generic_to_shared(vals) - (kGuessBias << 2);
-    ox = (unsigned)g.occ_n[0];
-    oz = ox * (unsigned)g.occ_n[1];
-    obias = 0u - (kGuessBias >> kMacroLog2) * (1u + ox + oz);
-  }
+      : q(quads), cells(g, s_tab), val((unsigned)__cvta_generic_to_shared(vals) - (kGuessBias << 2)), occ(occupancy) {}
 };
-
-// The guessed cell of s >= org on one axis as the bits 0x4B000000 + c: one
-// fused multiply-add rounded toward zero leaves floor((s - org) seed) in the
-// low mantissa bits of [2^23, 2^24). ExactGeo::seed keeps c <= n - 1 over the
-// volume, so c indexes the table (its closing entry included) unclamped.
-__device__ __forceinline__ unsigned guess(float s, float org, float seed) {
-  return __float_as_uint(__fmaf_rz(s - org, seed, 8388608.f));
-}
-__device__ __forceinline__ float4 ld_shared4(unsigned a) {
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ float ld_shared1(unsigned a) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
-  return v;
-}
-
-// Three-way minimum and maximum (one instruction each); NaN if any operand is.
-__device__ __forceinline__ float min3(float a, float b, float c) {
-  float r;
-  asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float r;
-  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
 
 // Corner values and parametric coordinates of the cell of s, whose guess is b. A
 // guess is the found cell unless s lies within an ulp of a cell face. The
@@ -178,8 +134,8 @@ template <typename QuadT>
 __device__ __forceinline__ void sample_fetch(const ExactGeo& g, const LightField<QuadT>& F, const float s[3],
                                              unsigned b0, unsigned b1, unsigned b2, float v[8], float p[3]) {
   {
-    const float4 e0 = ld_shared4(F.tab[0] + (b0 << 4)), e1 = ld_shared4(F.tab[1] + (b1 << 4)),
-                 e2 = ld_shared4(F.tab[2] + (b2 << 4));
+    const float4 e0 = ld_shared4(F.cells.tab[0] + (b0 << 4)), e1 = ld_shared4(F.cells.tab[1] + (b1 << 4)),
+                 e2 = ld_shared4(F.cells.tab[2] + (b2 << 4));
     QuadLoad<QuadT>::cell(F.q, float_bits(e0.y) + float_bits(e1.y) + float_bits(e2.y), g.fs[1], g.fs[2], v);
     // pcoords = (p - min) / (max - min) (RectilinearMeshOracle.h:189-192)
     p[0] = div_field(s[0] - e0.x, e0);
@@ -187,9 +143,9 @@ __device__ __forceinline__ void sample_fetch(const ExactGeo& g, const LightField
     p[2] = div_field(s[2] - e2.x, e2);
   }
   if (!(min3(p[0], p[1], p[2]) > 0.f && max3(p[0], p[1], p[2]) < 1.f)) {
-    const int3 c = walk_cells_bsearch(F.T[0], F.T[1], F.T[2], g.n[0] - 2, g.n[1] - 2, g.n[2] - 2, s[0], s[1], s[2],
+    const int3 c = walk_cells_bsearch(F.cells.T[0], F.cells.T[1], F.cells.T[2], g.n[0] - 2, g.n[1] - 2, g.n[2] - 2, s[0], s[1], s[2],
                                       (int)(b0 - kGuessBias), (int)(b1 - kGuessBias), (int)(b2 - kGuessBias));
-    const float4 *e0 = F.T[0] + c.x, *e1 = F.T[1] + c.y, *e2 = F.T[2] + c.z;
+    const float4 *e0 = F.cells.T[0] + c.x, *e1 = F.cells.T[1] + c.y, *e2 = F.cells.T[2] + c.z;
     QuadLoad<QuadT>::cell(F.q, float_bits(e0->y) + float_bits(e1->y) + float_bits(e2->y), g.fs[1], g.fs[2], v);
     p[0] = (s[0] - e0->x) / (e0[1].x - e0->x);
     p[1] = (s[1] - e1->x) / (e1[1].x - e1->x);
@@ -215,8 +171,9 @@ __device__ __forceinline__ float sample_value(const ExactGeo& g, const LightFiel
 
 // The light march of one ray. ns counts the samples marched (skipped ones
 // included). sure: at most ray.sure. With SKIP, samples in empty macro-cells
-// (occ == 0: every value there has TF alpha 0, which leaves the state
-// unchanged, see Accum) take no field fetch.
+// (every value there has TF alpha 0, which leaves the state unchanged, see
+// Accum) take no field fetch, and the march steps through empty neighbours
+// without looking them up (see macro_distance).
 template <typename QuadT, bool PREC, bool SKIP>
 __device__ __forceinline__ void light_march(const ExactGeo& g, const LightField<QuadT>& F, const LightRay& ray,
                                             int sure, Accum<PREC>& acc, unsigned& ns) {
@@ -247,10 +204,17 @@ __device__ __forceinline__ void light_march(const ExactGeo& g, const LightField<
     }
     ns += n;
   } else {
+    // steps that cannot move further than one macro-cell (see macro_distance)
+    float cells = 0.f;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      cells = fmaxf(cells,
+                    (fabsf(ray.sd[d]) * 1.00001f + 1.2e-7f * fmaxf(fabsf(g.minp[d]), fabsf(g.maxp[d]))) * g.invh[d]);
+    const float per_macro = __fdividef(0.999f * (float)(1 << kMacroLog2), cells);
     int k = 0;  // samples marched
     for (;;) {
       unsigned b0, b1, b2;
-      for (;;) {  // on to the next sample in an occupied macro-cell
+      for (;;) {  // on to the next sample in a macro-cell that is not empty
         if (k >= sure) {
           const float q0 = s[0] - ray.st[0], q1 = s[1] - ray.st[1], q2 = s[2] - ray.st[2];
           if (k >= g.light_budget || !(q0 * q0 + q1 * q1 + q2 * q2 <= ray.len2)) {
@@ -268,9 +232,14 @@ __device__ __forceinline__ void light_march(const ExactGeo& g, const LightField<
         b0 = guess(s[0], g.org[0], g.seed[0]);
         b1 = guess(s[1], g.org[1], g.seed[1]);
         b2 = guess(s[2], g.org[2], g.seed[2]);
-        // the macro-cell comes from the guess; its occupancy covers a guess off by one
-        if (__ldg(F.occ + ((b2 >> kMacroLog2) * F.oz + ((b1 >> kMacroLog2) * F.ox + ((b0 >> kMacroLog2) + F.obias)))))
-          break;
+        const int far = macro_distance(g, F.occ, b0, b1, b2);
+        if (far == 0) break;
+        const int more = min((int)((float)(far - 1) * per_macro), sure - k);
+        for (int i = 0; i < more; ++i) {
+#pragma unroll
+          for (int d = 0; d < 3; ++d) s[d] = s[d] + ray.sd[d];
+        }
+        k += max(more, 0);
       }
       if (acc.add(sample_value(g, F, s, b0, b1, b2))) {
         ns += (unsigned)k;

@@ -5,6 +5,7 @@
 #pragma once
 #include <type_traits>
 
+#include "cell_tables.cuh"
 #include "exact_device.cuh"
 
 namespace beams {
@@ -59,9 +60,85 @@ struct CellMarker {
   }
 };
 
-// SKIP: samples in macro-cells whose occupancy is 0 (every value there maps to
-// an in-range TF entry of alpha 0) only advance and count as lit: their
-// premultiplied alpha is 0, so they change neither colour nor alpha.
+// What the view march reads through 32-bit shared addresses, biased like
+// CellTables': the colour map and the map axes' cell tables.
+struct ViewTables {
+  CellTables cells;
+  unsigned tf;
+  unsigned map[3];
+  __device__ __forceinline__ ViewTables(const ExactGeo& g, const float4* s_tab, const float4* s_tf)
+      : cells(g, s_tab), tf((unsigned)__cvta_generic_to_shared(s_tf) - (kGuessBias << 4)) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      map[d] = (unsigned)__cvta_generic_to_shared(s_tab + g.max_off[d]) - (kGuessBias << 4);
+  }
+};
+
+// The cell of the map a shaded sample at p interpolates
+// (TransmittanceLocator::LocateCell, TransmittanceMap.h:93-112): index of its
+// first vertex and parametric coordinates. The reference clamps t to [0, pd - 2]
+// when t >= pd - 1 and truncates; p is inside the volume, so t is in [0, pd - 1],
+// and the table's entry pd - 1 repeats the last cell.
+__device__ __forceinline__ unsigned map_cell(const ExactGeo& g, const ViewTables& T, const float4* s_tab,
+                                             const float p[3], float pc[3]) {
+  unsigned idx = 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const float t = (p[d] - g.morig[d]) * g.minv[d];
+    const float4 e = ld_shared4(T.map[d] + (__float_as_uint(__fadd_rz(t, 8388608.f)) << 4));
+    idx += __float_as_uint(e.y);
+    pc[d] = div_field(p[d] - e.x, e);
+  }
+  const float sum = pc[0] + pc[1] + pc[2];
+  if (sum != sum) {  // an entry whose two-term division is not exact (see field_entry)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int c = min(trunc_small((p[d] - g.morig[d]) * g.minv[d]), g.pd[d] - 2);
+      const float4* e = s_tab + g.max_off[d] + c;
+      pc[d] = (p[d] - e->x) / (vtx_coord(g, d, c + 1) - e->x);
+    }
+  }
+  return idx;
+}
+
+// Map value interpolated in that cell (GetEstimateUsingVerticesT,
+// TransmittanceMap.h:200-229): opacity in the exact form, transmittance in the
+// precision form.
+template <typename MapT>
+__device__ __forceinline__ float map_value(const ExactGeo& g, const MapT* __restrict__ map, unsigned idx,
+                                           const float pc[3]) {
+  const unsigned px = (unsigned)g.pd[0], pxy = (unsigned)g.pd[0] * (unsigned)g.pd[1];
+  const MapT *m0 = map + idx, *m1 = map + (idx + px), *m2 = map + (idx + pxy), *m3 = map + (idx + pxy + px);
+  const float v[8] = {ld_map(m0), ld_map(m0 + 1), ld_map(m1 + 1), ld_map(m1),
+                      ld_map(m2), ld_map(m2 + 1), ld_map(m3 + 1), ld_map(m3)};
+  return hex_interp(v, pc[0], pc[1], pc[2]);
+}
+
+// How many steps of the march from p (inside the volume, distance dist) are
+// certain to stay inside the volume and below maxD, so that they need no tests.
+// Positions and dist move by repeated addition of a constant, which is monotonic
+// in floats, so the first and the last step decide; k additions move coordinate d
+// by at most k (|sd_d| + u B) with u = 2^-24 and B = max |bound|, and dist by at
+// most k (sd + u maxD). The u terms are doubled, the approximate divisions err by
+// 2 ulp against the 1e-5 taken off, and two steps are kept back.
+__device__ __forceinline__ int sure_steps(const ExactGeo& g, const float p[3], const float sd[3], float dist,
+                                          float maxD, int budget) {
+  float k = __fdividef((maxD - dist) * 0.99999f, g.sd * 1.00001f + 1.2e-7f * maxD);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const float room = sd[d] > 0.f ? g.maxp[d] - p[d] : p[d] - g.minp[d];
+    const float B = fmaxf(fabsf(g.minp[d]), fabsf(g.maxp[d]));
+    k = fminf(k, __fdividef(room * 0.99999f, fabsf(sd[d]) * 1.00001f + 1.2e-7f * B));
+  }
+  return k > 3.f ? min((int)fminf(k, 1e9f) - 2, budget) : 0;
+}
+
+// SKIP: a sample that enters a cell of an empty macro-cell (every value there
+// maps to an in-range TF entry of alpha 0, occ != 0 = the distance in macro-cells
+// to the nearest one that is not empty) only advances and counts as lit: its
+// premultiplied alpha is 0, so it changes neither colour nor alpha. Macro-cells
+// nearer than that distance are empty too, so the march advances without further
+// tests for as many steps as cannot leave them.
 template <typename QuadT, bool USE_MAP, typename MapT, typename Rec = NoRecord, bool SKIP = false, bool MULTI = false,
           bool RECT = false>
 __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT* __restrict__ quads,
@@ -83,109 +160,155 @@ __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT*
     p[1] = o[1] + dist * d[1];
     p[2] = o[2] + dist * d[2];
   }
-  const float sdx = g.sd * d[0], sdy = g.sd * d[1], sdz = g.sd * d[2];
-  unsigned qx, qz;
-  QuadLoad<QuadT>::strides(g, qx, qz);
-  float bl[3] = {0.f, 0.f, 0.f};
-  bool newCell = true;
-  float tx = 0.f, ty = 0.f, tz = 0.f;
-  float s0 = 0.f, s1m0 = 0.f, s2m3 = 0.f, s3 = 0.f, s4 = 0.f, s5m4 = 0.f, s6m7 = 0.f, s7 = 0.f;
-  int c[3] = {0, 0, 0};
-  float inv[3] = {0.f, 0.f, 0.f};
-  const int n1 = g.tf_n - 1;
-  while (inside_vol(g, p) && dist < maxD && budget-- > 0) {
-    if (SKIP && !occupied(g, occ, p)) {
-      ++lit;
-      dist += g.sd;
-      p[0] = p[0] + sdx;
-      p[1] = p[1] + sdy;
-      p[2] = p[2] + sdz;
-      tx = (p[0] - bl[0]) * inv[0];
-      ty = (p[1] - bl[1]) * inv[1];
-      tz = (p[2] - bl[2]) * inv[2];
-      continue;  // colour unchanged, so the cutoff test cannot newly pass
-    }
-    const float mint = mn(tx, mn(ty, tz));
-    const float maxt = mx(tx, mx(ty, tz));
-    if (maxt > 1.f || mint < 0.f) newCell = true;
-    if (newCell) {
-      if constexpr (RECT) {
+  if (!(inside_vol(g, p) && dist < maxD && budget > 0)) return;
+  const float sd[3] = {g.sd * d[0], g.sd * d[1], g.sd * d[2]};
+  // steps after this one certain to pass the loop's tests
+  int left = sure_steps(g, p, sd, dist, maxD, budget - 1);
+  budget -= left + 1;
+  float per_macro = 0.f;  // steps that cannot move further than one macro-cell
+  if (SKIP) {
+    float cells = 0.f;  // cells a step moves at most, over the axes
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const float4* T = s_tab + g.ax_off[k];
-          float4 e;
-          if (p[k] == g.maxp[k]) {
-            c[k] = g.n[k] - 2;  // the reference leaves invSpacing[k] unchanged here
-            e = T[c[k]];
-          } else {
-            c[k] = find_cell_walk_rect(T, g.n[k] - 2, p[k], e);
-            inv[k] = e.z;  // 1.f / (coord(c+1) - coord(c)), IEEE
+    for (int k = 0; k < 3; ++k)
+      cells = fmaxf(cells, (fabsf(sd[k]) * 1.00001f + 1.2e-7f * fmaxf(fabsf(g.minp[k]), fabsf(g.maxp[k]))) * g.invh[k]);
+    per_macro = __fdividef(0.999f * (float)(1 << kMacroLog2), cells);
+  }
+  const ViewTables T(g, s_tab, s_tf);
+  // no cell yet: t is NaN until a cell is located (inv starts at 0 for the max-face rule)
+  const float none = __int_as_float(0x7fffffff);
+  float bl[3] = {none, none, none}, inv[3] = {0.f, 0.f, 0.f};
+  float tx = none, ty = none, tz = none;
+  float s0 = 0.f, s1m0 = 0.f, s2m3 = 0.f, s3 = 0.f, s4 = 0.f, s5m4 = 0.f, s6m7 = 0.f, s7 = 0.f;
+  for (;;) {
+    bool skipped = false;
+    if (!(min3(tx, ty, tz) >= 0.f && max3(tx, ty, tz) <= 1.f)) {
+      const unsigned b0 = guess(p[0], g.org[0], g.seed[0]), b1 = guess(p[1], g.org[1], g.seed[1]),
+                     b2 = guess(p[2], g.org[2], g.seed[2]);
+      if (SKIP) {
+        const int far = macro_distance(g, occ, b0, b1, b2);
+        if (far) {
+          skipped = true;
+          const int more = min((int)((float)(far - 1) * per_macro), left);
+          left -= more;
+          lit += (unsigned)more + 1u;
+          for (int i = 0; i < more; ++i) {
+            dist += g.sd;
+            p[0] = p[0] + sd[0];
+            p[1] = p[1] + sd[1];
+            p[2] = p[2] + sd[2];
           }
-          bl[k] = e.x;
         }
-      } else {
-        locate_view_cell(g, s_tab, p, c, inv, bl);
       }
-      float v[8];
-      QuadLoad<QuadT>::cell(quads, (unsigned)c[2] * qz + (unsigned)c[1] * qx + (unsigned)c[0], qx, qz, v);
-      s0 = v[0];
-      s3 = v[3];
-      s4 = v[4];
-      s7 = v[7];
-      s6m7 = v[6] - v[7];
-      s5m4 = v[5] - v[4];
-      s1m0 = v[1] - v[0];
-      s2m3 = v[2] - v[3];
-      tx = (p[0] - bl[0]) * inv[0];
-      ty = (p[1] - bl[1]) * inv[1];
-      tz = (p[2] - bl[2]) * inv[2];
-      newCell = false;
+      if (!skipped) {
+        unsigned off;
+        if constexpr (RECT) {
+          off = 0;
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const float4* A = s_tab + g.ax_off[k];
+            float4 e;
+            if (p[k] == g.maxp[k]) {
+              e = A[g.n[k] - 2];  // the reference leaves invSpacing[k] unchanged here
+            } else {
+              find_cell_walk_rect(A, g.n[k] - 2, p[k], e);
+              inv[k] = e.z;  // 1.f / (coord(c+1) - coord(c)), IEEE
+            }
+            bl[k] = e.x;
+            off += __float_as_uint(e.y);
+          }
+          tx = (p[0] - bl[0]) * inv[0];
+          ty = (p[1] - bl[1]) * inv[1];
+          tz = (p[2] - bl[2]) * inv[2];
+        } else {
+          off = locate_view_cell(g, T.cells, p, b0, b1, b2, inv, bl, tx, ty, tz);
+        }
+        float v[8];
+        QuadLoad<QuadT>::cell(quads, off, g.fs[1], g.fs[2], v);
+        s0 = v[0];
+        s3 = v[3];
+        s4 = v[4];
+        s7 = v[7];
+        s6m7 = v[6] - v[7];
+        s5m4 = v[5] - v[4];
+        s1m0 = v[1] - v[0];
+        s2m3 = v[2] - v[3];
+      }
     }
-    const float l76 = s7 + tx * s6m7;
-    const float l45 = s4 + tx * s5m4;
-    const float top = l45 + ty * (l76 - l45);
-    const float l01 = s0 + tx * s1m0;
-    const float l32 = s3 + tx * s2m3;
-    const float bot = l01 + ty * (l32 - l01);
-    float fs = bot + tz * (top - bot);
-    fs = (fs - g.min_scalar) * g.inv_delta;
-    const float fi = fs * (float)n1;
-    if (fi > -1.f && fi < (float)(n1 + 1)) {
-      const float4 tfc = s_tf[trunc_small(fmaxf(fi, 0.f))];  // (int)fi: fi in (-1, n1 + 1)
-      float sc0 = tfc.x, sc1 = tfc.y, sc2 = tfc.z;
-      const float sa = tfc.w * (1.f - color.w);
-      if (rec) (*rec)(p, tfc, sa);
-      if (USE_MAP && MULTI) {
-        float est[3];
-        map_light_sum(g, s_tab, (const float*)map, p, est);
-        sc0 = sc0 * est[0];
-        sc1 = sc1 * est[1];
-        sc2 = sc2 * est[2];
-      } else if (USE_MAP) {
-        // exact form: 1 - opacity (TransmittanceMap.h:195); precision form: stored transmittance
-        const float mv = map_interp_t<MapT>(g, s_tab, map, p);
-        const float tr = (sizeof(MapT) == 2) ? mv : 1.f - mv;
-        sc0 = sc0 * (tr * g.light_color[0]);
-        sc1 = sc1 * (tr * g.light_color[1]);
-        sc2 = sc2 * (tr * g.light_color[2]);
+    if (!skipped) {
+      const float l76 = s7 + tx * s6m7;
+      const float l45 = s4 + tx * s5m4;
+      const float top = l45 + ty * (l76 - l45);
+      const float l01 = s0 + tx * s1m0;
+      const float l32 = s3 + tx * s2m3;
+      const float bot = l01 + ty * (l32 - l01);
+      float fs = bot + tz * (top - bot);
+      fs = (fs - g.min_scalar) * g.inv_delta;
+      const float fi = fs * g.n1f;
+      if (fi > -1.f && fi < g.n1f + 1.f) {
+        const float4 tfc = ld_shared4(T.tf + (__float_as_uint(__fadd_rz(fmaxf(fi, 0.f), 8388608.f)) << 4));
+        const float sa = tfc.w * (1.f - color.w);
+        if (rec) (*rec)(p, tfc, sa);
+        // a sample of alpha 0 adds 0 times its shading, which is 0 unless the shading is not finite
+        if (sa != 0.f || !g.tame) {
+          float sc0 = tfc.x, sc1 = tfc.y, sc2 = tfc.z;
+          if (USE_MAP) {
+            float pc[3];
+            const unsigned idx = map_cell(g, T, s_tab, p, pc);
+            if (MULTI) {
+              // the multi-light extension: sum over the maps of (1 - opacity_l) *
+              // light_colors[l], in light order, over one map grid
+              const size_t nv = (size_t)g.pd[0] * (unsigned)g.pd[1] * (unsigned)g.pd[2];
+              float e0 = 0.f, e1 = 0.f, e2 = 0.f;
+              for (int l = 0; l < g.n_lights; ++l) {
+                const float tr = 1.f - map_value(g, (const float*)map + l * nv, idx, pc);
+                const float t0 = tr * g.light_colors[l][0], t1 = tr * g.light_colors[l][1],
+                            t2 = tr * g.light_colors[l][2];
+                e0 = (l == 0) ? t0 : e0 + t0;
+                e1 = (l == 0) ? t1 : e1 + t1;
+                e2 = (l == 0) ? t2 : e2 + t2;
+              }
+              sc0 = sc0 * e0;
+              sc1 = sc1 * e1;
+              sc2 = sc2 * e2;
+            } else {
+              // exact form: 1 - opacity (TransmittanceMap.h:195); precision form: stored transmittance
+              const float mv = map_value(g, map, idx, pc);
+              const float tr = (sizeof(MapT) == 2) ? mv : 1.f - mv;
+              sc0 = sc0 * (tr * g.light_color[0]);
+              sc1 = sc1 * (tr * g.light_color[1]);
+              sc2 = sc2 * (tr * g.light_color[2]);
+            }
+          }
+          if (g.tame) {  // no NaN: clamp01 is a saturation
+            sc0 = __saturatef(sc0);
+            sc1 = __saturatef(sc1);
+            sc2 = __saturatef(sc2);
+          } else {
+            sc0 = clamp01(sc0);
+            sc1 = clamp01(sc1);
+            sc2 = clamp01(sc2);
+          }
+          color.x = color.x + sc0 * sa;
+          color.y = color.y + sc1 * sa;
+          color.z = color.z + sc2 * sa;
+        }
+        color.w = sa + color.w;
+        ++lit;
       }
-      sc0 = clamp01(sc0);
-      sc1 = clamp01(sc1);
-      sc2 = clamp01(sc2);
-      color.x = color.x + sc0 * sa;
-      color.y = color.y + sc1 * sa;
-      color.z = color.z + sc2 * sa;
-      color.w = sa + color.w;
-      ++lit;
     }
     dist += g.sd;
-    p[0] = p[0] + sdx;
-    p[1] = p[1] + sdy;
-    p[2] = p[2] + sdz;
+    p[0] = p[0] + sd[0];
+    p[1] = p[1] + sd[1];
+    p[2] = p[2] + sd[2];
+    if (!skipped && color.w >= g.cutoff) return;
+    if (left > 0) {
+      --left;
+    } else if (!(inside_vol(g, p) && dist < maxD && budget-- > 0)) {
+      return;
+    }
     tx = (p[0] - bl[0]) * inv[0];
     ty = (p[1] - bl[1]) * inv[1];
     tz = (p[2] - bl[2]) * inv[2];
-    if (color.w >= g.cutoff) break;
   }
 }
 
