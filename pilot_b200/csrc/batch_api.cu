@@ -27,13 +27,12 @@ struct BatchVolume {
   beams_volume vol{};
   void* owned = nullptr;         // device copy of a host field
   float4* quads = nullptr;       // float32 4-corner quads
-  void* ranges = nullptr;        // value ranges of the quads' macro-cells
+  void* ranges = nullptr;        // value ranges of the quads' macro-cells, behind the quads
   unsigned char* occ = nullptr;  // their distances under occ_tf (empty-space skipping)
   unsigned long long occ_tf = ~0ull;
   ~BatchVolume() {
     if (owned) cudaFree(owned);
     if (quads) cudaFree(quads);
-    if (ranges) cudaFree(ranges);
     if (occ) cudaFree(occ);
   }
 };
@@ -153,8 +152,9 @@ beams_status beams_batch_set_volumes(beams_renderer* r, const beams_volume* vols
       bv->vol.on_device = 1;
     }
     const size_t nq = (size_t)(vols[i].dims[0] - 1) * (vols[i].dims[1] - 1) * vols[i].dims[2];
-    if (e == cudaSuccess) e = cudaMalloc((void**)&bv->quads, nq * sizeof(float4));
-    if (e == cudaSuccess) e = cudaMalloc(&bv->ranges, macro_bytes(vols[i].dims));
+    const size_t tail = (nq * sizeof(float4) + 255) & ~(size_t)255;
+    if (e == cudaSuccess) e = cudaMalloc((void**)&bv->quads, tail + macro_bytes(vols[i].dims));
+    bv->ranges = (char*)bv->quads + tail;
     if (e == cudaSuccess)
       e = launch_build_quads(bv->vol.data, BEAMS_F32, bv->quads, BEAMS_F32, vols[i].dims, bv->ranges, r->stream);
     if (e != cudaSuccess) {

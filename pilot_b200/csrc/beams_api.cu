@@ -379,12 +379,13 @@ beams_status prepare_layouts(beams_renderer* r, const ExactGeo& g, int& launches
   if (r->vol.assoc == BEAMS_ASSOC_POINTS && r->quads_version != qkey) {
     const size_t nq = (size_t)(g.n[0] - 1) * (g.n[1] - 1) * g.n[2];
     const size_t qbytes = (qd == BEAMS_F32) ? sizeof(float4) : 8;
-    beams_status s = ensure_buffer(r, (void**)&r->d_quads, &r->quads_cap, nq * qbytes, "allocating quad field");
-    if (s != BEAMS_OK) return s;
-    // the macro-cells' ranges with them: they describe these quads, whatever becomes of the field
-    s = ensure_buffer(r, (void**)&r->d_ranges, &r->ranges_cap, macro_bytes(g.n), "allocating macro-cell ranges");
-    if (s != BEAMS_OK) return s;
+    // the macro-cells' ranges behind them: they describe these quads, whatever becomes of the field
+    const size_t tail = (nq * qbytes + 255) & ~(size_t)255;
     r->quads_version = 0;  // not these quads until both launches are queued
+    beams_status s = ensure_buffer(r, (void**)&r->d_quads, &r->quads_cap, tail + macro_bytes(g.n),
+                                   "allocating quad field");
+    if (s != BEAMS_OK) return s;
+    r->d_ranges = (char*)r->d_quads + tail;
     cudaError_t e = launch_build_quads(r->d_field, r->vol.dtype, r->d_quads, qd, g.n, r->d_ranges, r->stream);
     if (e != cudaSuccess) return cuda_fail(r, e, "quad field build");
     launches += 2;

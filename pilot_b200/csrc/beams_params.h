@@ -147,25 +147,26 @@ __host__ __device__ inline float bits_float(unsigned u) {
 }
 
 // Whether fma(x, rh, x rl) is the correctly rounded x / w for every x, given
-// |rh + rl - 1/w| <= 7 * 2^-48 / w. The sum is x / w to 2^-45 before its one
-// rounding, so it can only round wrongly when a midpoint of two floats lies
-// within 2^-45 of x / w. With w = W 2^b, x = X 2^a, the midpoint M 2^c (W, X 24
-// bits, M odd, 25 bits) that means 0 < |X 2^k - M W| < 16, k = 24 (X >= W) or 25.
-// For each such difference D, M W = -D modulo 2^k fixes M modulo 2^k / (W's
-// trailing zeros) and X = (M W + D) / 2^k, so the few numerators at risk are
-// solved for and tried. M is odd, so D has exactly W's trailing zeros: from four
-// on (cells some 16 widths or more from coordinate 0) there are none.
-__host__ __device__ inline bool two_term_division_exact(float w, float rh, float rl) {
+// |rh + rl - 1/w| <= (reach / 2 - 1) 2^-48 / w. x rl adds 2^-48 of its own, so the
+// sum is x / w to reach 2^-49 before its one rounding and can only round wrongly
+// when a midpoint of two floats lies that near to x / w. With w = W 2^b, x = X 2^a,
+// the midpoint M 2^c (W, X 24 bits, M odd, 25 bits) that means 0 < |X 2^k - M W| <
+// reach, k = 24 (X >= W) or 25. For each such difference D, M W = -D modulo 2^k
+// fixes M modulo 2^k / (W's trailing zeros) and X = (M W + D) / 2^k, so the few
+// numerators at risk are solved for and tried. M is odd, so D has exactly W's
+// trailing zeros: with enough of them (cells some widths from coordinate 0) there
+// are none.
+__host__ __device__ inline bool two_term_division_exact(float w, float rh, float rl, int reach) {
   const unsigned bits = float_bits(w), ex = bits >> 23;
   if (ex < 64u || ex > 190u) return false;  // far from any overflow or underflow (and w > 0)
   const unsigned W = (bits & 0x7fffffu) | 0x800000u;
   int z = 0;
-  while (z < 4 && !((W >> z) & 1u)) ++z;
-  if (z == 4) return true;
+  while ((1 << z) < reach && !((W >> z) & 1u)) ++z;
+  if ((1 << z) >= reach) return true;
   unsigned inv = W >> z;  // the odd part's inverse modulo 2^32 (Newton)
   for (int i = 0; i < 5; ++i) inv *= 2u - (W >> z) * inv;
   for (int k = 24; k <= 25; ++k)
-    for (int D = 1 << z; D < 16; D += 2 << z)
+    for (int D = 1 << z; D < reach; D += 2 << z)
       for (int sign = -1; sign <= 1; sign += 2) {
         const unsigned step = 1u << (k - z), M0 = (0u - (unsigned)(sign * (D >> z))) * inv & (step - 1u);
         for (unsigned M = M0; M < (1u << 25); M += step) {
@@ -194,7 +195,8 @@ __host__ __device__ inline float4 field_entry(float lo, float hi, unsigned offse
     const unsigned b = float_bits(r0) + (unsigned)by;
     const float t = bits_float(b);
     if (r0 == 0.f && i > 0) break;
-    if (two_term_division_exact(w, rh, t)) {
+    // r0 itself is 1/w - rh to 2^-48, three ulp away to 7 * 2^-48
+    if (two_term_division_exact(w, rh, t, i == 0 ? 4 : 16)) {
       rl = t;
       break;
     }

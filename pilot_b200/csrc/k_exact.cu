@@ -478,57 +478,52 @@ struct Make16 {
 };
 
 // The quads of one volume, and the value ranges its macro-cells' emptiness is
-// read from. A block takes eight rows of quads of one slice (a macro-cell row):
-// each thread walks down the eleven field rows around them at its x, keeping the
-// previous row, so the field is read 11/8 times (from L2 past the first) and
-// every quad is one coalesced store; the emptiness of macro-cell m looks at cells
-// [8m - 1, 8m + 8], hence at the points [8m - 1, 8m + 9] of each axis: the column
-// ranges over those rows go through shared memory into one range per macro-cell
-// and slice. Bound by the quads' stores (a 512^3 float32 field: 2.1 GB). The
-// ranges cost nothing beside them, where reading them back from the quads took
-// 1.24 ms for that field.
+// read from. A block takes eight rows of quads of one slice (a macro-cell row): a
+// warp reads the eleven field rows around them at 32 neighbouring x (the field is
+// read 11/8 times, past the first from L2), makes the eight rows of 31 quads with
+// the next lane's values and stores each row coalesced. The emptiness of
+// macro-cell m looks at cells [8m - 1, 8m + 8], hence at the points [8m - 1, 8m + 9]
+// of each axis: the column ranges over those rows go through shared memory into
+// one range per macro-cell and slice. Rows and columns past the volume repeat its
+// last ones, which no range notices.
 constexpr int kLayoutThreads = 128;
 
 template <typename In, typename OutT, typename Maker, bool RANGES>
-__global__ void __launch_bounds__(kLayoutThreads) k_build_quads(const In* __restrict__ f, OutT* __restrict__ q, int nx,
-                                                                int ny, float2* __restrict__ part, int mx, int my) {
+__global__ void __launch_bounds__(kLayoutThreads, 10) k_build_quads(const In* __restrict__ f, OutT* __restrict__ q,
+                                                                    int nx, int ny, float2* __restrict__ part, int mx,
+                                                                    int my) {
   extern __shared__ float2 s_col[];  // per x: {min, max} over the rows
-  const int by = blockIdx.x, z = blockIdx.y;
-  const size_t slice = (size_t)z * ny;
+  const int by = blockIdx.x, z = blockIdx.y, lane = threadIdx.x & 31;
   const int y0 = (by << kMacroLog2) - 1;
-  for (int x = threadIdx.x; x < ((nx + 31) & ~31); x += kLayoutThreads) {
-    const bool in = x < nx;
-    typename Maker::V prev{}, prevn{};
-    float lo = __int_as_float(0x7f800000), hi = -lo;
-    typename Maker::V row[11];
+  const In* slice = f + (size_t)z * ny * nx;
+  const int rows = min(8, ny - 2 - y0);  // rows of quads here: y0 + 1 .. y0 + rows
+  for (int xb = (threadIdx.x >> 5) * 31; xb < nx - 1; xb += 31 * (kLayoutThreads / 32)) {
+    const int x = min(xb + lane, nx - 1);
+    typename Maker::V v[11];
 #pragma unroll
-    for (int r = 0; r < 11; ++r) {
-      const int y = y0 + r;
-      row[r] = (in && y >= 0 && y < ny) ? Maker::get(f + (slice + y) * nx + x) : typename Maker::V{};
-    }
+    for (int r = 0; r < 11; ++r) v[r] = Maker::get(slice + (unsigned)min(max(y0 + r, 0), ny - 1) * (unsigned)nx + x);
+    if (RANGES) {
+      float lo = __int_as_float(0x7f800000), hi = -lo;
+      bool nan = false;
 #pragma unroll
-    for (int r = 0; r < 11; ++r) {
-      const int y = y0 + r;
-      const bool ok = in && y >= 0 && y < ny;
-      const typename Maker::V cur = row[r];
-      typename Maker::V next = __shfl_down_sync(0xffffffffu, cur, 1);
-      if ((threadIdx.x & 31) == 31 && x + 1 < nx && ok) next = Maker::get(f + (slice + y) * nx + x + 1);
-      if (RANGES && ok) {
-        const float v = Maker::value(cur);
-        lo = fminf(lo, v);
-        hi = fmaxf(hi, v);
-        if (v != v) {  // never empty
-          lo = -__int_as_float(0x7f800000);
-          hi = -lo;
-        }
+      for (int r = 0; r < 11; ++r) {
+        const float a = Maker::value(v[r]);
+        lo = fminf(lo, a);
+        hi = fmaxf(hi, a);
+        nan = nan || a != a;
       }
-      // rows y - 1 and y make the quads of row y - 1
-      if (r >= 2 && r <= 9 && ok && x + 1 < nx) q[((size_t)z * (ny - 1) + (y - 1)) * (nx - 1) + x] =
-          Maker::make(prev, prevn, cur, next);
-      prev = cur;
-      prevn = next;
+      const float inf = __int_as_float(0x7f800000);
+      s_col[x] = nan ? make_float2(-inf, inf) : make_float2(lo, hi);  // NaN: never empty
     }
-    if (RANGES && in) s_col[x] = make_float2(lo, hi);
+    OutT* out = q + ((size_t)z * (ny - 1) + (y0 + 1)) * (nx - 1) + x;
+    const bool store = lane < 31 && xb + lane < nx - 1;
+    typename Maker::V below = __shfl_down_sync(0xffffffffu, v[1], 1);
+#pragma unroll
+    for (int r = 1; r <= 8; ++r) {
+      const typename Maker::V above = __shfl_down_sync(0xffffffffu, v[r + 1], 1);
+      if (store && r <= rows) out[(size_t)(r - 1) * (nx - 1)] = Maker::make(v[r], below, v[r + 1], above);
+      below = above;
+    }
   }
   if (!RANGES) return;
   __syncthreads();

@@ -179,10 +179,10 @@ struct beams_renderer {
   float4* d_tab = nullptr;
   size_t tab_cap = 0;
   unsigned long long tab_key[4] = {0, 0, 0, 0};  // volume_version, map m[3] packed
-  // value ranges of the quads' macro-cells and, under the colour map, their
-  // distances to the nearest that is not empty (empty-space skipping)
+  // value ranges of the quads' macro-cells (behind the quads in their buffer) and,
+  // under the colour map, their distances to the nearest that is not empty
+  // (empty-space skipping)
   void* d_ranges = nullptr;
-  size_t ranges_cap = 0;
   unsigned char* d_occ = nullptr;
   size_t occ_cap = 0;
   unsigned long long occ_key[2] = {~0ull, ~0ull};  // quads key, tf_version
@@ -229,7 +229,6 @@ struct beams_renderer {
     if (d_quads) cudaFree(d_quads);
     if (d_tab) cudaFree(d_tab);
     if (d_occ) cudaFree(d_occ);
-    if (d_ranges) cudaFree(d_ranges);
     if (d_tau) cudaFree(d_tau);
     if (d_rgba) cudaFree(d_rgba);
     if (d_depth) cudaFree(d_depth);
