@@ -42,14 +42,14 @@ __device__ __forceinline__ void load_tables(float4* s_tab, const float4* __restr
 // STITCH: the multi-brick Phase 3 — the march starts from the cross-brick
 // prefix (stitch_prefix) instead of zero, as GenerateEstimator is re-run on
 // the prefix opacities (LightedVolumeRenderer.cxx:1241-1252).
-// Blocks per SM: 6 (40 registers) for the plain and the stitching exact march
-// (the 257^3-vertex map of a 512^3 noise field, mean of eight light directions:
-// 2.39 ms against 2.63 ms at 4 blocks, where the loads' latency shows); the
-// skipping, precision and rectilinear marches keep 4 (at 6 they spill: the 640^3
-// precision build went 6.4 -> 9.5 ms).
-template <bool STITCH, bool PREC, bool SKIP, bool RECT>
+// Blocks per SM: 6 (40 registers), where the loads' latency is covered best (the
+// 257^3-vertex map of a 512^3 noise field, mean of eight light directions: 2.39 ms
+// against 2.63 ms at 4; skipping, 256^3 noise 0.40 against 0.44 ms, 384^3
+// bfloat16 0.99 against 1.04 ms); the rectilinear march, and the listed ones with
+// both ways to march a ray, spill there and keep 4.
+template <bool RECT, bool LIST>
 constexpr int k1_blocks_per_sm() {
-  return (PREC || SKIP || RECT) ? 4 : 6;
+  return RECT || LIST ? 4 : 6;
 }
 
 // A masked map build (the exact form's lazy map, the learned form's fallback,
@@ -167,10 +167,23 @@ __global__ void __launch_bounds__(256) k_list_marked_vertices(const ExactGeo g, 
   }
 }
 
+// Maps of at most this many rays are marched kSplit lanes a ray (light_march_split):
+// with a lane a ray they leave most of the GPU idle while the longest rays run
+// (the 33^3-vertex map of a 64^3 field takes 56 us, split 31 us; 49^3 vertices 65 and
+// 55 us; 65^3 87 and 97 us. Without skipping, on a 256^3 field: 91 and 47, 90 and 74,
+// 108 and 118 us). The precision form's sums cost more in the split march (41^3
+// vertices 62 and 53 us, 49^3 65 and 70 us).
+constexpr int kSplit = 4;
+template <bool PREC>
+constexpr unsigned split_rays() {
+  return PREC ? 100000u : 160000u;
+}
+
 // LIST: the vertices come from a work list (k_list_marked_vertices) instead of
-// the whole map's vertex order.
-template <typename QuadT, bool STITCH, bool PREC, bool SKIP, bool RECT = false, bool LIST = false>
-__global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<STITCH, PREC, SKIP, RECT>()) k_light_march(const ExactGeo g, const QuadT* __restrict__ quads,
+// the whole map's vertex order. SPLIT: kSplit lanes a ray (a list decides by its
+// own length).
+template <typename QuadT, bool STITCH, bool PREC, bool SKIP, bool RECT = false, bool LIST = false, bool SPLIT = false>
+__global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<RECT, LIST>()) k_light_march(const ExactGeo g, const QuadT* __restrict__ quads,
                                                           const float4* __restrict__ tab,
                                                           const float4* __restrict__ tf,
                                                           const float* __restrict__ tau,
@@ -206,45 +219,65 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<STITCH, PREC, SKIP,
   __shared__ int s_lo[8];
   if (threadIdx.x == 0) light_order_setup(g, s_lo);
   __syncthreads();
-  const int ntiles = LIST ? (int)((vlist[0] + 31u) >> 5) : (int)((nslots + 31u) >> 5);
+  const unsigned nrays = LIST ? vlist[0] : nslots;
+  const bool split = !RECT && (SPLIT || (LIST && nrays <= split_rays<PREC>()));
+  const int ntiles = split ? (int)((nrays + 32 / kSplit - 1) / (32 / kSplit)) : (int)((nrays + 31u) >> 5);
+  const int bl = g.light_brick_log2;
   unsigned ns = 0, built = 0;
 
-  for (int tile = next_warp_tile(&cnt->tiles_light); tile < ntiles; tile = next_warp_tile(&cnt->tiles_light)) {
-    int id;
-    float V[3], L[3];
-    const int bl = g.light_brick_log2;
+  // ray -> vertex; false when it has none
+  auto vertex = [&](unsigned i, int& id, float V[3]) -> bool {
+    if (i >= nrays) return false;
     if (LIST) {
-      const unsigned i = ((unsigned)tile << 5) + lane;
-      if (i >= vlist[0]) continue;
       id = (int)vlist[1 + i];
       map_vertex(g, id, V);
     } else if (bl) {
-      const unsigned slot = ((unsigned)tile << 5) + lane;
       int x, y, z;
-      if (slot >= nslots || !light_slot_vertex(slot, bl, s_lo, x, y, z)) continue;
+      if (!light_slot_vertex(i, bl, s_lo, x, y, z)) return false;
       id = (z * g.pd[1] + y) * g.pd[0] + x;
       V[0] = vtx_coord(g, 0, x);
       V[1] = vtx_coord(g, 1, y);
       V[2] = vtx_coord(g, 2, z);
     } else {
-      id = (tile << 5) + lane;
-      if ((unsigned)id >= nslots) continue;
+      id = (int)i;
       map_vertex(g, id, V);
     }
-    ++built;
-    light_origin(g, V, L);
-    float dir[3];
-    const LightRay ray = light_ray(g, V, L, dir);
+    return true;
+  };
+
+  for (int tile = next_warp_tile(&cnt->tiles_light); tile < ntiles; tile = next_warp_tile(&cnt->tiles_light)) {
+    int id = 0;
+    float V[3] = {0.f, 0.f, 0.f}, L[3], dir[3];
     Accum<PREC> acc;
-    acc.init(STITCH ? stitch_prefix(refs, nrefs, self, L, V, dir) : 0.f);
-    if constexpr (RECT) {
-      light_march_rect(g, quads, s_tab, s_a, ray, acc, ns);
-    } else {
-      // the lanes leave the untested steps together
-      const int sure = SKIP ? ray.sure : __reduce_min_sync(__activemask(), ray.sure);
-      light_march<QuadT, PREC, SKIP>(g, F, ray, sure, acc, ns);
+    if constexpr (!RECT && (LIST || SPLIT)) {
+      if (split) {
+        const bool active = vertex((unsigned)tile * (32 / kSplit) + lane / kSplit, id, V);
+        light_origin(g, V, L);
+        const LightRay ray = light_ray(g, V, L, dir);
+        acc.init(STITCH && active ? stitch_prefix(refs, nrefs, self, L, V, dir) : 0.f);
+        light_march_split<QuadT, PREC, SKIP, kSplit>(g, F, ray, active, acc, ns);
+        if (active && (lane & (kSplit - 1)) == 0) {
+          acc.store(map, id);
+          ++built;
+        }
+        continue;
+      }
     }
-    acc.store(map, id);
+    if constexpr (!SPLIT) {
+      if (!vertex(((unsigned)tile << 5) + lane, id, V)) continue;
+      ++built;
+      light_origin(g, V, L);
+      const LightRay ray = light_ray(g, V, L, dir);
+      acc.init(STITCH ? stitch_prefix(refs, nrefs, self, L, V, dir) : 0.f);
+      if constexpr (RECT) {
+        light_march_rect(g, quads, s_tab, s_a, ray, acc, ns);
+      } else {
+        // the lanes leave the untested steps together
+        const int sure = SKIP ? ray.sure : __reduce_min_sync(__activemask(), ray.sure);
+        light_march<QuadT, PREC, SKIP>(g, F, ray, sure, acc, ns);
+      }
+      acc.store(map, id);
+    }
   }
   warp_add(&cnt->light_samples, ns);
   if (LIST) warp_add(&cnt->map_vertices, built);
@@ -637,97 +670,59 @@ size_t macro_bytes(const int n[3]) {
   return ((size_t)m[0] * m[1] * m[2] + (size_t)m[0] * m[1] * n[2]) * sizeof(float2);
 }
 
+// One instantiation of K1 over the launch's rays.
+template <typename QuadT, bool STITCH, bool PREC, bool SKIP, bool RECT, bool LIST, bool SPLIT>
+static cudaError_t launch_k1_as(const ExactGeo& g, const void* quads, const float4* tab, const float4* tf,
+                                const float* tau, void* map, unsigned nslots, Counters* cnt, cudaStream_t st,
+                                const BrickRef* refs, int nrefs, int self, const unsigned* gate,
+                                const unsigned char* occ, const unsigned* vlist) {
+  const size_t smem = (size_t)g.max_off[0] * sizeof(float4) + 2 * (size_t)g.tf_n * sizeof(float);
+  // warps take tiles from a launch-wide counter, so the tiles in flight stay a
+  // compact window of the vertex order however unevenly the rays run
+  const int ntiles = (int)(((unsigned long long)nslots * (SPLIT || LIST ? kSplit : 1) + kThreads - 1) / kThreads);
+  int grid = 0;
+  const auto kernel = k_light_march<QuadT, STITCH, PREC, SKIP, RECT, LIST, SPLIT>;
+  cudaError_t e = persistent_grid(kernel, smem, ntiles, grid);
+  if (e != cudaSuccess) return e;
+  kernel<<<grid, kThreads, smem, st>>>(g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate,
+                                       occ, vlist);
+  return cudaGetLastError();
+}
+
 template <typename QuadT, bool STITCH, bool PREC>
 static cudaError_t launch_k1(const ExactGeo& g, const void* quads, const float4* tab, const float4* tf,
                              const float* tau, void* map, Counters* cnt, cudaStream_t st, const BrickRef* refs,
                              int nrefs, int self, const unsigned* gate = nullptr,
                              const unsigned char* occ = nullptr, const unsigned* vlist = nullptr) {
-  const int nvert = g.pd[0] * g.pd[1] * g.pd[2];
   // vertex slots in the launch's order (the vertices themselves in rows)
-  const unsigned nslots = g.light_brick_log2 ? light_slots(g, g.light_brick_log2) : (unsigned)nvert;
-  const size_t smem = (size_t)g.max_off[0] * sizeof(float4) + 2 * (size_t)g.tf_n * sizeof(float);
-  const int ntiles = (nvert + kThreads - 1) / kThreads;
-  int grid = 0;
-  // warps take tiles from a launch-wide counter, so the tiles in flight stay a
-  // compact window of the brick order however unevenly the rays run
+  const unsigned nslots = g.light_brick_log2 ? light_slots(g, g.light_brick_log2)
+                                             : (unsigned)g.pd[0] * (unsigned)g.pd[1] * (unsigned)g.pd[2];
   cudaError_t e = cudaMemsetAsync(&cnt->tiles_light, 0, sizeof(unsigned), st);
   if (e != cudaSuccess) return e;
+#define BEAMS_K1(SKIP, RECT, LIST, SPLIT)                                                                             \
+  launch_k1_as<QuadT, STITCH, PREC, SKIP, RECT, LIST, SPLIT>(g, quads, tab, tf, tau, map, nslots, cnt, st, refs, nrefs, \
+                                                             self, gate, occ, vlist)
   if (g.rect && !PREC) {
     // explicit rectilinear coordinates, exact form: binary-search cell location, no
     // empty-space skipping (the precision form keeps the seeded walk, correct for
     // any increasing coordinates)
     if constexpr (!STITCH && !PREC && std::is_same<QuadT, float4>::value) {
-      if (vlist) {
-        e = persistent_grid(k_light_march<float4, false, false, false, true, true>, smem, ntiles, grid);
-        if (e != cudaSuccess) return e;
-        k_light_march<float4, false, false, false, true, true><<<grid, kThreads, smem, st>>>(
-            g, (const float4*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, nullptr, vlist);
-        return cudaGetLastError();
-      }
-      e = persistent_grid(k_light_march<float4, false, false, false, true>, smem, ntiles, grid);
-      if (e != cudaSuccess) return e;
-      k_light_march<float4, false, false, false, true><<<grid, kThreads, smem, st>>>(
-          g, (const float4*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, nullptr, nullptr);
-      return cudaGetLastError();
+      occ = nullptr;
+      return vlist ? BEAMS_K1(false, true, true, false) : BEAMS_K1(false, true, false, false);
     } else {
       return cudaErrorInvalidValue;
     }
   }
-  if constexpr (!STITCH && !PREC) {
-    if (vlist) {
-      if (occ) {
-        e = persistent_grid(k_light_march<QuadT, false, false, true, false, true>, smem, ntiles, grid);
-        if (e != cudaSuccess) return e;
-        k_light_march<QuadT, false, false, true, false, true><<<grid, kThreads, smem, st>>>(
-            g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, occ, vlist);
-      } else {
-        e = persistent_grid(k_light_march<QuadT, false, false, false, false, true>, smem, ntiles, grid);
-        if (e != cudaSuccess) return e;
-        k_light_march<QuadT, false, false, false, false, true><<<grid, kThreads, smem, st>>>(
-            g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, nullptr, vlist);
-      }
-      return cudaGetLastError();
+  if (vlist) {  // a masked build: lazy maps, the learned form's fallback, the multi-brick Phase 1
+    if constexpr (STITCH) {
+      return occ ? cudaErrorInvalidValue : BEAMS_K1(false, false, true, false);
+    } else {
+      return occ ? BEAMS_K1(true, false, true, false) : BEAMS_K1(false, false, true, false);
     }
-  } else if constexpr (!STITCH && PREC) {
-    if (vlist) {  // the precision form's lazy map
-      if (occ) {
-        e = persistent_grid(k_light_march<QuadT, false, true, true, false, true>, smem, ntiles, grid);
-        if (e != cudaSuccess) return e;
-        k_light_march<QuadT, false, true, true, false, true><<<grid, kThreads, smem, st>>>(
-            g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, occ, vlist);
-      } else {
-        e = persistent_grid(k_light_march<QuadT, false, true, false, false, true>, smem, ntiles, grid);
-        if (e != cudaSuccess) return e;
-        k_light_march<QuadT, false, true, false, false, true><<<grid, kThreads, smem, st>>>(
-            g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, nullptr, vlist);
-      }
-      return cudaGetLastError();
-    }
-  } else if constexpr (STITCH && !PREC) {
-    if (vlist) {  // the lazy map of a multi-block scene: the stitched march over a brick's list
-      if (occ) return cudaErrorInvalidValue;
-      e = persistent_grid(k_light_march<QuadT, true, false, false, false, true>, smem, ntiles, grid);
-      if (e != cudaSuccess) return e;
-      k_light_march<QuadT, true, false, false, false, true><<<grid, kThreads, smem, st>>>(
-          g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, nullptr, vlist);
-      return cudaGetLastError();
-    }
-  } else {
-    if (vlist) return cudaErrorInvalidValue;
   }
-  if (occ) {
-    e = persistent_grid(k_light_march<QuadT, STITCH, PREC, true>, smem, ntiles, grid);
-    if (e != cudaSuccess) return e;
-    k_light_march<QuadT, STITCH, PREC, true><<<grid, kThreads, smem, st>>>(g, (const QuadT*)quads, tab, tf, tau, map, nslots, cnt, refs, nrefs, self, gate, occ,
-                                                                           nullptr);
-  } else {
-    e = persistent_grid(k_light_march<QuadT, STITCH, PREC, false>, smem, ntiles, grid);
-    if (e != cudaSuccess) return e;
-    k_light_march<QuadT, STITCH, PREC, false><<<grid, kThreads, smem, st>>>(g, (const QuadT*)quads, tab, tf, tau,
-                                                                            map, nslots, cnt, refs, nrefs, self, gate,
-                                                                            nullptr, nullptr);
-  }
-  return cudaGetLastError();
+  if (nslots <= split_rays<PREC>()) return occ ? BEAMS_K1(true, false, false, true) : BEAMS_K1(false, false, false, true);
+  return occ ? BEAMS_K1(true, false, false, false) : BEAMS_K1(false, false, false, false);
+#undef BEAMS_K1
 }
 
 template <bool RECT, bool LIST, bool SKIP = false, typename QuadT = float4>
