@@ -86,14 +86,25 @@ __global__ void __launch_bounds__(256) k_gen_data(const ExactGeo g, const float4
 }
 
 // ---- encoding --------------------------------------------------------------------
-__global__ void k_features(const float4* __restrict__ samples, const float4* __restrict__ lfeat, Encoding enc,
-                           __nv_bfloat16* __restrict__ X, int n) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float4 s = samples[i];
-    const float4 lf = lfeat[(int)s.w];
+// One thread per feature pair, so that a row's 224 bytes are written by neighbouring
+// threads (2^18 rows: 256 us with a thread per row, each storing its own row).
+constexpr int kPairs = kIn / 2;       // 56
+constexpr int kFeatThreads = 4 * kPairs;  // four rows a block
+__global__ void __launch_bounds__(kFeatThreads) k_features(const float4* __restrict__ samples,
+                                                           const float4* __restrict__ lfeat, Encoding enc,
+                                                           __nv_bfloat162* __restrict__ X, int n) {
+  __shared__ float s_freq[kFreq];
+  if (threadIdx.x < kFreq) s_freq[threadIdx.x] = freq(threadIdx.x);
+  __syncthreads();
+  const int c = threadIdx.x % kPairs;
+  for (int row = blockIdx.x * 4 + threadIdx.x / kPairs; row < n; row += gridDim.x * 4) {
+    const float4 s = __ldg(samples + row);
+    const float4 lf = __ldg(lfeat + (int)s.w);
     const float p[3] = {s.x, s.y, s.z}, l[3] = {lf.x, lf.y, lf.z};
-    __nv_bfloat16* row = X + (size_t)i * kIn;
-    encode(enc, p, l, [&](int j, float v) { row[j] = __float2bfloat16_rn(v); });
+    float u[3], a, b;
+    normalised(enc, p, u);
+    feature_pair(u, l, 2 * c, a, b, s_freq);
+    X[(size_t)row * kPairs + c] = __floats2bfloat162_rn(a, b);
   }
 }
 
@@ -293,7 +304,7 @@ cudaError_t mlp_gen_data(const ExactGeo& g, const float4* quads, const float4* t
 
 cudaError_t mlp_features(const float4* samples, const float4* lfeat, const Encoding& enc, __nv_bfloat16* X, int n,
                          cudaStream_t st) {
-  k_features<<<grid_cap(n, 256), 256, 0, st>>>(samples, lfeat, enc, X, n);
+  k_features<<<148 * 9, kFeatThreads, 0, st>>>(samples, lfeat, enc, (__nv_bfloat162*)X, n);
   return cudaGetLastError();
 }
 

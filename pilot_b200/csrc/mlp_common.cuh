@@ -81,23 +81,10 @@ __device__ __forceinline__ void feature_pair(const float u[3], const float l[3],
   }
 }
 
-// Writes the kIn features of position p (world space) under light feature l.
+// Position p (world space) relative to the volume.
 __device__ __forceinline__ void normalised(const Encoding& e, const float p[3], float u[3]) {
 #pragma unroll
   for (int a = 0; a < 3; ++a) u[a] = (p[a] - e.bmin[a]) * e.inv_ext[a];
-}
-
-template <typename Out>
-__device__ __forceinline__ void encode(const Encoding& e, const float p[3], const float l[3], Out&& out) {
-  float u[3];
-  normalised(e, p, u);
-#pragma unroll 1
-  for (int c = 0; c < kIn; c += 2) {
-    float a, b;
-    feature_pair(u, l, c, a, b);
-    out(c, a);
-    out(c + 1, b);
-  }
 }
 
 }  // namespace mlp
