@@ -23,6 +23,11 @@ beams_status ensure_buffer(beams_renderer* r, void** buf, size_t* cap, size_t by
 beams_status prepare_layouts(beams_renderer* r, const ExactGeo& g, int& launches);
 beams_status check_ready(beams_renderer* r);
 
+// A training set up to this size (2^20 samples) stays allocated for the next
+// training on the renderer: allocating and freeing it took 1 to 3 ms of a training
+// whose kernels run 2 ms. A larger one is freed, as its training takes far longer.
+constexpr size_t kKeepTrainBytes = (size_t)256 << 20;
+
 // Device state of the learned form (owned by the renderer).
 struct MlpState {
   float* P = nullptr;  // float32 masters
@@ -37,6 +42,8 @@ struct MlpState {
   float4* lights = nullptr;  // training light positions (xyz)
   float4* lfeat = nullptr;   // their direction features
   int nlights = 0;
+  void* train_mem = nullptr;  // training samples, targets and features (kept up to kKeepTrainBytes)
+  size_t train_bytes = 0;
   void* packed = nullptr;    // inference weights: B fragments + biases
   void* probe_mem = nullptr; // probe records, counts, tile flags, fallback list
   size_t probe_bytes = 0;
@@ -55,7 +62,7 @@ struct MlpState {
   volatile unsigned* h_fallback = nullptr;
   int fb_tiles = 0;
   ~MlpState() {
-    for (void* p : {(void*)P, (void*)G, (void*)m, (void*)v, ws_mem, (void*)lights, (void*)lfeat, packed, probe_mem,
+    for (void* p : {(void*)P, (void*)G, (void*)m, (void*)v, ws_mem, train_mem, (void*)lights, (void*)lfeat, packed, probe_mem,
                     (void*)probe_err, (void*)vmask})
       if (p) cudaFree(p);
     if (h_fallback) cudaFreeHost((void*)h_fallback);
@@ -493,22 +500,41 @@ beams_status beams_mlp_train(beams_renderer* r, const beams_mlp_options* opt, be
   st->nlights = o.n_lights;
 
   const int n = 1 << o.samples_log2;
-  float4* d_samples = nullptr;
-  float* d_target = nullptr;
-  __nv_bfloat16* d_X = nullptr;
+  // samples, targets and features in one block, kept for the next training while it is small
+  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t b_samples = al((size_t)n * sizeof(float4)), b_target = al((size_t)n * sizeof(float));
+  const size_t b_all = b_samples + b_target + (size_t)n * kIn * sizeof(__nv_bfloat16);
   cudaEvent_t t0, t1, t2;
   cudaEventCreate(&t0);
   cudaEventCreate(&t1);
   cudaEventCreate(&t2);
-  e = cudaMalloc((void**)&d_samples, (size_t)n * sizeof(float4));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_target, (size_t)n * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_X, (size_t)n * kIn * sizeof(__nv_bfloat16));
-  if (e != cudaSuccess) {
-    cudaFree(d_samples);
-    cudaFree(d_target);
-    cudaFree(d_X);
-    return cuda_fail(r, e, "mlp_train: allocating the training set");
+  if (st->train_bytes < b_all) {
+    if (st->train_mem) cudaFree(st->train_mem);
+    st->train_mem = nullptr;
+    st->train_bytes = 0;
+    e = cudaMalloc(&st->train_mem, b_all);
+    if (e != cudaSuccess) {
+      st->train_mem = nullptr;
+      cudaEventDestroy(t0);
+      cudaEventDestroy(t1);
+      cudaEventDestroy(t2);
+      return cuda_fail(r, e, "mlp_train: allocating the training set");
+    }
+    st->train_bytes = b_all;
   }
+  auto release = [&]() {
+    if (st->train_bytes > kKeepTrainBytes) {
+      cudaFree(st->train_mem);
+      st->train_mem = nullptr;
+      st->train_bytes = 0;
+    }
+    cudaEventDestroy(t0);
+    cudaEventDestroy(t1);
+    cudaEventDestroy(t2);
+  };
+  float4* d_samples = (float4*)st->train_mem;
+  float* d_target = (float*)((char*)st->train_mem + b_samples);
+  __nv_bfloat16* d_X = (__nv_bfloat16*)((char*)st->train_mem + b_samples + b_target);
   cudaEventRecord(t0, r->stream);
   e = mlp_gen_data(g, (const float4*)r->d_quads, r->d_tab, r->d_tf, st->lights, o.n_lights, o.seed, o.focus, d_samples,
                    d_target, n, r->stream);
@@ -524,9 +550,8 @@ beams_status beams_mlp_train(beams_renderer* r, const beams_mlp_options* opt, be
   st->step = 0;
   beams_status bs = ensure_ws(r, st, std::max(o.batch, std::min(n / 16, 65536)));
   if (bs != BEAMS_OK) {
-    cudaFree(d_samples);
-    cudaFree(d_target);
-    cudaFree(d_X);
+    cudaStreamSynchronize(r->stream);
+    release();
     return bs;
   }
   const int holdout = std::min(n / 16, 65536);
@@ -581,12 +606,7 @@ beams_status beams_mlp_train(beams_renderer* r, const beams_mlp_options* opt, be
     e = cudaMemcpyAsync(&tc_err, st->ws.err, sizeof(unsigned), cudaMemcpyDeviceToHost, r->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(r->stream);
   if (e == cudaSuccess && tc_err) {
-    cudaFree(d_samples);
-    cudaFree(d_target);
-    cudaFree(d_X);
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
-    cudaEventDestroy(t2);
+    release();
     return fail(r, BEAMS_ERR_TIMEOUT, "mlp_train: a tensor-core wait timed out");
   }
   if (rep && e == cudaSuccess) {
@@ -600,12 +620,7 @@ beams_status beams_mlp_train(beams_renderer* r, const beams_mlp_options* opt, be
     rep->steps = st->step;
     rep->samples = n;
   }
-  cudaEventDestroy(t0);
-  cudaEventDestroy(t1);
-  cudaEventDestroy(t2);
-  cudaFree(d_samples);
-  cudaFree(d_target);
-  cudaFree(d_X);
+  release();
   if (e != cudaSuccess) return cuda_fail(r, e, "mlp_train");
   st->ready = true;
   return BEAMS_OK;
