@@ -286,9 +286,12 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<RECT, LIST>()) k_li
 // ---------------------------------------------------------------------------
 // K2 (point field)
 // ---------------------------------------------------------------------------
+// Four blocks a SM (64 registers): left to itself the compiler takes 78 and three
+// blocks run (1024^2 view of 384^3 bfloat16 3.25 -> 2.86 ms, 512^2 of 128^3 blobs 0.33
+// -> 0.31 ms; five blocks spill: 3.05 and 0.34 ms).
 template <typename QuadT, bool USE_MAP, typename MapT, bool LIST = false, bool SKIP = false, bool MULTI = false,
           bool RECT = false>
-__global__ void __launch_bounds__(kThreads) k_view_march(const ExactGeo g, const QuadT* __restrict__ quads,
+__global__ void __launch_bounds__(kThreads, 4) k_view_march(const ExactGeo g, const QuadT* __restrict__ quads,
                                                          const float4* __restrict__ tab,
                                                          const float4* __restrict__ tf,
                                                          const MapT* __restrict__ map,
@@ -340,7 +343,7 @@ __global__ void __launch_bounds__(kThreads) k_view_march(const ExactGeo g, const
 // kFallbackTile^2 tiles while *fcount > 0; tile counter cnt->tiles_mark. The
 // march reads no map, so only the field axes' cell tables are staged.
 template <typename QuadT, bool RECT, bool LIST, bool SKIP = false>
-__global__ void __launch_bounds__(kThreads) k_mark_view_cells(const ExactGeo g, const QuadT* __restrict__ quads,
+__global__ void __launch_bounds__(kThreads, 4) k_mark_view_cells(const ExactGeo g, const QuadT* __restrict__ quads,
                                                               const float4* __restrict__ tab,
                                                               const float4* __restrict__ tf,
                                                               unsigned char* __restrict__ mask,
