@@ -410,7 +410,7 @@ __device__ __forceinline__ bool light_slot_vertex(unsigned slot, int bl, const i
   return true;
 }
 
-// Quad layout of a point field: Q[z][y][x] = {f(x,y,z), f(x+1,y,z), f(x,y+1,z),
+// Quad layout of a point field: Q[z][y][x] = {f(x,y,z), f(x,y+1,z), f(x+1,y,z),
 // f(x+1,y+1,z)} for x < nx-1, y < ny-1, so one cell is two 16-byte loads
 // (z and z+1). VTK corner order 0..7 = lo.x lo.y lo.w lo.z hi.x hi.y hi.w hi.z.
 // Cell (x, y, z) is entry qi = z qz + y qx + x; strides() gives qx and qz.
@@ -452,8 +452,8 @@ template <> struct QuadLoad<QuadBF16> {
   static __device__ __forceinline__ void cell(const QuadBF16* __restrict__ q, unsigned qi, unsigned, unsigned qz, float v[8]) {
     const uint2 a = __ldg((const uint2*)(q + qi));
     const uint2 b = __ldg((const uint2*)(q + qi + qz));
-    v[0] = bf16_lo(a.x); v[1] = bf16_hi(a.x); v[2] = bf16_hi(a.y); v[3] = bf16_lo(a.y);
-    v[4] = bf16_lo(b.x); v[5] = bf16_hi(b.x); v[6] = bf16_hi(b.y); v[7] = bf16_lo(b.y);
+    v[0] = bf16_lo(a.x); v[3] = bf16_hi(a.x); v[1] = bf16_lo(a.y); v[2] = bf16_hi(a.y);
+    v[4] = bf16_lo(b.x); v[7] = bf16_hi(b.x); v[5] = bf16_lo(b.y); v[6] = bf16_hi(b.y);
   }
 };
 template <> struct QuadLoad<QuadF16> {
@@ -461,8 +461,8 @@ template <> struct QuadLoad<QuadF16> {
   static __device__ __forceinline__ void cell(const QuadF16* __restrict__ q, unsigned qi, unsigned, unsigned qz, float v[8]) {
     const uint2 a = __ldg((const uint2*)(q + qi));
     const uint2 b = __ldg((const uint2*)(q + qi + qz));
-    v[0] = f16_lo(a.x); v[1] = f16_hi(a.x); v[2] = f16_hi(a.y); v[3] = f16_lo(a.y);
-    v[4] = f16_lo(b.x); v[5] = f16_hi(b.x); v[6] = f16_hi(b.y); v[7] = f16_lo(b.y);
+    v[0] = f16_lo(a.x); v[3] = f16_hi(a.x); v[1] = f16_lo(a.y); v[2] = f16_hi(a.y);
+    v[4] = f16_lo(b.x); v[7] = f16_hi(b.x); v[5] = f16_lo(b.y); v[6] = f16_hi(b.y);
   }
 };
 template <> struct QuadLoad<float4> {
@@ -470,8 +470,8 @@ template <> struct QuadLoad<float4> {
   static __device__ __forceinline__ void cell(const float4* __restrict__ q, unsigned qi, unsigned, unsigned qz, float v[8]) {
     const float4 a = __ldg(q + qi);
     const float4 b = __ldg(q + qi + qz);
-    v[0] = a.x; v[1] = a.y; v[2] = a.w; v[3] = a.z;
-    v[4] = b.x; v[5] = b.y; v[6] = b.w; v[7] = b.z;
+    v[0] = a.x; v[3] = a.y; v[1] = a.z; v[2] = a.w;
+    v[4] = b.x; v[7] = b.y; v[5] = b.z; v[6] = b.w;
   }
 };
 

@@ -495,12 +495,13 @@ __global__ void k_build_tables(const ExactGeo g, float4* __restrict__ tab) {
 }
 
 // Quad makers: V is the value kept of an input element (as stored in the quad),
-// value() what the marches read back, make() the quad of rows y and y + 1.
+// value() what the marches read back, make(f(x, y), f(x + 1, y), f(x, y + 1),
+// f(x + 1, y + 1)) the quad.
 struct MakeF32 {
   using V = float;
   static __device__ __forceinline__ V get(const float* p) { return __ldg(p); }
   static __device__ __forceinline__ float value(V v) { return v; }
-  static __device__ __forceinline__ float4 make(V a, V b, V c, V d) { return make_float4(a, b, c, d); }
+  static __device__ __forceinline__ float4 make(V a, V b, V c, V d) { return make_float4(a, c, b, d); }
 };
 template <bool BF16>
 struct Make16 {
@@ -510,7 +511,7 @@ struct Make16 {
   }
   static __device__ __forceinline__ V get(const unsigned short* p) { return __ldg(p); }
   static __device__ __forceinline__ float value(V v) { return BF16 ? bf16_lo(v) : f16_lo(v); }
-  static __device__ __forceinline__ uint2 make(V a, V b, V c, V d) { return make_uint2(a | (b << 16), c | (d << 16)); }
+  static __device__ __forceinline__ uint2 make(V a, V b, V c, V d) { return make_uint2(a | (c << 16), b | (d << 16)); }
 };
 
 // The quads of one volume, and the value ranges its macro-cells' emptiness is

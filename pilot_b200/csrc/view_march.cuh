@@ -114,6 +114,90 @@ __device__ __forceinline__ float map_value(const ExactGeo& g, const MapT* __rest
   return hex_interp(v, pc[0], pc[1], pc[2]);
 }
 
+// Shades and composites one sample at p whose interpolated field value is fs
+// (Sampler::operator(), LightedVolumeRenderer.cxx:440-489).
+template <bool USE_MAP, typename MapT, typename Rec, bool MULTI>
+__device__ __forceinline__ void shade_sample(const ExactGeo& g, const ViewTables& T, const float4* s_tab,
+                                             const MapT* __restrict__ map, const float p[3], float fs, float4& color,
+                                             unsigned& lit, Rec* rec) {
+  const float fi = ((fs - g.min_scalar) * g.inv_delta) * g.n1f;
+  if (!(fi > -1.f && fi < g.n1f + 1.f)) return;
+  const float4 tfc = ld_shared4(T.tf + (__float_as_uint(__fadd_rz(fmaxf(fi, 0.f), 8388608.f)) << 4));
+  const float sa = tfc.w * (1.f - color.w);
+  if (rec) (*rec)(p, tfc, sa);
+  // a sample of alpha 0 adds 0 times its shading, which is 0 unless the shading is not finite
+  if (sa != 0.f || !g.tame) {
+    float sc0 = tfc.x, sc1 = tfc.y, sc2 = tfc.z;
+    if (USE_MAP) {
+      float pc[3];
+      const unsigned idx = map_cell(g, T, s_tab, p, pc);
+      if (MULTI) {
+        // the multi-light extension: sum over the maps of (1 - opacity_l) *
+        // light_colors[l], in light order, over one map grid
+        const size_t nv = (size_t)g.pd[0] * (unsigned)g.pd[1] * (unsigned)g.pd[2];
+        float e0 = 0.f, e1 = 0.f, e2 = 0.f;
+        for (int l = 0; l < g.n_lights; ++l) {
+          const float tr = 1.f - map_value(g, (const float*)map + l * nv, idx, pc);
+          const float t0 = tr * g.light_colors[l][0], t1 = tr * g.light_colors[l][1], t2 = tr * g.light_colors[l][2];
+          e0 = (l == 0) ? t0 : e0 + t0;
+          e1 = (l == 0) ? t1 : e1 + t1;
+          e2 = (l == 0) ? t2 : e2 + t2;
+        }
+        sc0 = sc0 * e0;
+        sc1 = sc1 * e1;
+        sc2 = sc2 * e2;
+      } else {
+        // exact form: 1 - opacity (TransmittanceMap.h:195); precision form: stored transmittance
+        const float mv = map_value(g, map, idx, pc);
+        const float tr = (sizeof(MapT) == 2) ? mv : 1.f - mv;
+        sc0 = sc0 * (tr * g.light_color[0]);
+        sc1 = sc1 * (tr * g.light_color[1]);
+        sc2 = sc2 * (tr * g.light_color[2]);
+      }
+    }
+    if (g.tame) {  // no NaN: clamp01 is a saturation
+      sc0 = __saturatef(sc0);
+      sc1 = __saturatef(sc1);
+      sc2 = __saturatef(sc2);
+    } else {
+      sc0 = clamp01(sc0);
+      sc1 = clamp01(sc1);
+      sc2 = clamp01(sc2);
+    }
+    color.x = color.x + sc0 * sa;
+    color.y = color.y + sc1 * sa;
+    color.z = color.z + sc2 * sa;
+  }
+  color.w = sa + color.w;
+  ++lit;
+}
+
+// The reference's trilinear value (LightedVolumeRenderer.cxx:425-438) of the corner
+// values v (VTK order) at t. The differences and products of the four x
+// interpolations run as packed pairs (two float32 operations an instruction, each
+// rounded as the single one is): the quads hold (v0, v3), (v1, v2) and (v4, v7),
+// (v5, v6) in register pairs. The sums stay single: the compiler contracts a packed
+// product and a packed sum into one rounding, -fmad=false or not.
+__device__ __forceinline__ float2 lerp_pair(float a0, float a1, float b0, float b1, float t) {
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, t;\n\t"
+      "mov.b64 a, {%2, %3};\n\t"
+      "mov.b64 b, {%4, %5};\n\t"
+      "mov.b64 t, {%6, %6};\n\t"
+      "sub.rn.f32x2 b, b, a;\n\t"
+      "mul.rn.f32x2 b, t, b;\n\t"
+      "mov.b64 {%0, %1}, b;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(t));
+  return make_float2(__fadd_rn(a0, r.x), __fadd_rn(a1, r.y));
+}
+__device__ __forceinline__ float view_interp(const float v[8], float tx, float ty, float tz) {
+  const float2 b = lerp_pair(v[0], v[3], v[1], v[2], tx), a = lerp_pair(v[4], v[7], v[5], v[6], tx);
+  const float top = a.x + ty * (a.y - a.x);
+  const float bot = b.x + ty * (b.y - b.x);
+  return bot + tz * (top - bot);
+}
+
 // How many steps of the march from p (inside the volume, distance dist) are
 // certain to stay inside the volume and below maxD, so that they need no tests.
 // Positions and dist move by repeated addition of a constant, which is monotonic
@@ -133,12 +217,80 @@ __device__ __forceinline__ int sure_steps(const ExactGeo& g, const float p[3], c
   return k > 3.f ? min((int)fminf(k, 1e9f) - 2, budget) : 0;
 }
 
-// SKIP: a sample that enters a cell of an empty macro-cell (every value there
-// maps to an in-range TF entry of alpha 0, occ != 0 = the distance in macro-cells
-// to the nearest one that is not empty) only advances and counts as lit: its
-// premultiplied alpha is 0, so it changes neither colour nor alpha. Macro-cells
-// nearer than that distance are empty too, so the march advances without further
-// tests for as many steps as cannot leave them.
+// The cell a view sample is interpolated in. The reference keeps the previous
+// sample's cell while the parametric coordinates t = (p - lower) inv in it stay in
+// [0, 1] and else walks to the cell that holds p (RectilinearLocator::LocateCell,
+// LightedVolumeRenderer.cxx:119-165); on a max face that is the last cell, and inv
+// is left as it was (its invSpacing keeps the previous value). A sample inside its
+// own cell by more than rounding is outside every other cell by t, so the two rules
+// part only within kFace of a face: elsewhere the cell is p's own, found afresh
+// without a look at the previous one. ViewCell holds what the faces need.
+constexpr float kFace = 1e-6f;  // in cells; far above the few 2^-24 that t errs by
+
+struct ViewCell {
+  unsigned off;   // the previous sample's cell (its quad index); none: 0xffffffff
+  bool kept;      // it holds an inv other than its own (after a sample on a max face)
+  float inv[3];   // that inv
+};
+
+struct ViewFace {
+  float t[3];
+  ViewCell cell;
+};
+
+// The reference's rule in full, for a sample near a face.
+struct ViewGrid {  // the part of ExactGeo it reads, by value (a reference would put all of it on the stack)
+  unsigned fs[3];
+  int n[3], ax[3];
+  float org[3], seed[3], maxp[3];
+};
+static __device__ __noinline__ ViewFace view_cell_at_face(const ViewGrid g, const float4* s_tab, const ViewCell prev,
+                                                          const float p0, const float p1, const float p2) {
+  const float p[3] = {p0, p1, p2};
+  ViewFace r;
+  float inv[3] = {0.f, 0.f, 0.f};
+  if (prev.off != 0xffffffffu) {
+    unsigned rest = prev.off;
+    bool in = true;
+#pragma unroll
+    for (int k = 2; k >= 0; --k) {
+      const unsigned c = rest / g.fs[k];
+      rest -= c * g.fs[k];
+      const float4* e = s_tab + g.ax[k] + c;
+      inv[k] = prev.kept ? prev.inv[k] : e->z;
+      r.t[k] = (p[k] - e->x) * inv[k];
+      in = in && r.t[k] >= 0.f && r.t[k] <= 1.f;
+    }
+    if (in) {
+      r.cell = prev;
+      return r;
+    }
+  }
+  r.cell.off = 0;
+  r.cell.kept = false;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float4* T = s_tab + g.ax[k];
+    const int seed = (int)(__float_as_uint(__fmaf_rz(p[k] - g.org[k], g.seed[k], 8388608.f)) - kGuessBias);
+    const int c = walk_cell_view(T, g.n[k] - 2, p[k], seed);
+    if (p[k] == g.maxp[k]) {
+      r.cell.kept = r.cell.kept || inv[k] != T[c].z;
+    } else {
+      inv[k] = T[c].z;
+    }
+    r.cell.inv[k] = inv[k];
+    r.t[k] = (p[k] - T[c].x) * inv[k];
+    r.cell.off += __float_as_uint(T[c].y);
+  }
+  return r;
+}
+
+// SKIP: a sample in an empty macro-cell (every value there maps to an in-range TF
+// entry of alpha 0; occ != 0 = the distance in macro-cells to the nearest one that
+// is not empty) only advances and counts as lit: its premultiplied alpha is 0, so
+// it changes neither colour nor alpha. Macro-cells nearer than that distance are
+// empty too, so the march advances without further tests for as many steps as
+// cannot leave them.
 template <typename QuadT, bool USE_MAP, typename MapT, typename Rec = NoRecord, bool SKIP = false, bool MULTI = false,
           bool RECT = false>
 __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT* __restrict__ quads,
@@ -165,150 +317,110 @@ __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT*
   // steps after this one certain to pass the loop's tests
   int left = sure_steps(g, p, sd, dist, maxD, budget - 1);
   budget -= left + 1;
-  float per_macro = 0.f;  // steps that cannot move further than one macro-cell
-  if (SKIP) {
-    float cells = 0.f;  // cells a step moves at most, over the axes
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-      cells = fmaxf(cells, (fabsf(sd[k]) * 1.00001f + 1.2e-7f * fmaxf(fabsf(g.minp[k]), fabsf(g.maxp[k]))) * g.invh[k]);
-    per_macro = __fdividef(0.999f * (float)(1 << kMacroLog2), cells);
-  }
   const ViewTables T(g, s_tab, s_tf);
-  // no cell yet: t is NaN until a cell is located (inv starts at 0 for the max-face rule)
-  const float none = __int_as_float(0x7fffffff);
-  float bl[3] = {none, none, none}, inv[3] = {0.f, 0.f, 0.f};
-  float tx = none, ty = none, tz = none;
-  float s0 = 0.f, s1m0 = 0.f, s2m3 = 0.f, s3 = 0.f, s4 = 0.f, s5m4 = 0.f, s6m7 = 0.f, s7 = 0.f;
-  for (;;) {
-    bool skipped = false;
-    if (!(min3(tx, ty, tz) >= 0.f && max3(tx, ty, tz) <= 1.f)) {
+  if constexpr (RECT) {
+    // explicit coordinates: a binary search when a sample leaves its cell, so the
+    // cell and its values are kept. No cell yet: t is NaN (inv starts at 0 for the
+    // max-face rule).
+    const float none = __int_as_float(0x7fffffff);
+    float bl[3] = {none, none, none}, inv[3] = {0.f, 0.f, 0.f}, t[3] = {none, none, none}, v[8];
+    for (;;) {
+      if (!(min3(t[0], t[1], t[2]) >= 0.f && max3(t[0], t[1], t[2]) <= 1.f)) {
+        unsigned off = 0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const float4* A = s_tab + g.ax_off[k];
+          float4 e;
+          if (p[k] == g.maxp[k]) {
+            e = A[g.n[k] - 2];  // the reference leaves invSpacing[k] unchanged here
+          } else {
+            find_cell_walk_rect(A, g.n[k] - 2, p[k], e);
+            inv[k] = e.z;  // 1.f / (coord(c+1) - coord(c)), IEEE
+          }
+          bl[k] = e.x;
+          off += __float_as_uint(e.y);
+          t[k] = (p[k] - bl[k]) * inv[k];
+        }
+        QuadLoad<QuadT>::cell(quads, off, g.fs[1], g.fs[2], v);
+      }
+      shade_sample<USE_MAP, MapT, Rec, MULTI>(g, T, s_tab, map, p, view_interp(v, t[0], t[1], t[2]), color, lit, rec);
+      dist += g.sd;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        p[k] = p[k] + sd[k];
+        t[k] = (p[k] - bl[k]) * inv[k];
+      }
+      if (color.w >= g.cutoff) return;
+      if (left > 0) {
+        --left;
+      } else if (!(inside_vol(g, p) && dist < maxD && budget-- > 0)) {
+        return;
+      }
+    }
+  } else {
+    float per_macro = 0.f;  // steps that cannot move further than one macro-cell
+    if (SKIP) {
+      float cells = 0.f;  // cells a step moves at most, over the axes
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        cells =
+            fmaxf(cells, (fabsf(sd[k]) * 1.00001f + 1.2e-7f * fmaxf(fabsf(g.minp[k]), fabsf(g.maxp[k]))) * g.invh[k]);
+      per_macro = __fdividef(0.999f * (float)(1 << kMacroLog2), cells);
+    }
+    ViewCell cell;
+    cell.off = 0xffffffffu;
+    cell.kept = false;
+    cell.inv[0] = cell.inv[1] = cell.inv[2] = 0.f;
+    for (;;) {
       const unsigned b0 = guess(p[0], g.org[0], g.seed[0]), b1 = guess(p[1], g.org[1], g.seed[1]),
                      b2 = guess(p[2], g.org[2], g.seed[2]);
-      if (SKIP) {
-        const int far = macro_distance(g, occ, b0, b1, b2);
-        if (far) {
-          skipped = true;
-          const int more = min((int)((float)(far - 1) * per_macro), left);
-          left -= more;
-          lit += (unsigned)more + 1u;
-          for (int i = 0; i < more; ++i) {
-            dist += g.sd;
-            p[0] = p[0] + sd[0];
-            p[1] = p[1] + sd[1];
-            p[2] = p[2] + sd[2];
-          }
+      const int far = SKIP ? macro_distance(g, occ, b0, b1, b2) : 0;
+      if (SKIP && far) {
+        const int more = min((int)((float)(far - 1) * per_macro), left);
+        left -= more;
+        lit += (unsigned)more + 1u;
+        for (int i = 0; i < more; ++i) {
+          dist += g.sd;
+          p[0] = p[0] + sd[0];
+          p[1] = p[1] + sd[1];
+          p[2] = p[2] + sd[2];
         }
-      }
-      if (!skipped) {
-        unsigned off;
-        if constexpr (RECT) {
-          off = 0;
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const float4* A = s_tab + g.ax_off[k];
-            float4 e;
-            if (p[k] == g.maxp[k]) {
-              e = A[g.n[k] - 2];  // the reference leaves invSpacing[k] unchanged here
-            } else {
-              find_cell_walk_rect(A, g.n[k] - 2, p[k], e);
-              inv[k] = e.z;  // 1.f / (coord(c+1) - coord(c)), IEEE
-            }
-            bl[k] = e.x;
-            off += __float_as_uint(e.y);
-          }
-          tx = (p[0] - bl[0]) * inv[0];
-          ty = (p[1] - bl[1]) * inv[1];
-          tz = (p[2] - bl[2]) * inv[2];
-        } else {
-          off = locate_view_cell(g, T.cells, p, b0, b1, b2, inv, bl, tx, ty, tz);
-        }
+      } else {
+        const float4 e0 = ld_shared4(T.cells.tab[0] + (b0 << 4)), e1 = ld_shared4(T.cells.tab[1] + (b1 << 4)),
+                     e2 = ld_shared4(T.cells.tab[2] + (b2 << 4));
+        unsigned off = __float_as_uint(e0.y) + __float_as_uint(e1.y) + __float_as_uint(e2.y);
         float v[8];
         QuadLoad<QuadT>::cell(quads, off, g.fs[1], g.fs[2], v);
-        s0 = v[0];
-        s3 = v[3];
-        s4 = v[4];
-        s7 = v[7];
-        s6m7 = v[6] - v[7];
-        s5m4 = v[5] - v[4];
-        s1m0 = v[1] - v[0];
-        s2m3 = v[2] - v[3];
-      }
-    }
-    if (!skipped) {
-      const float l76 = s7 + tx * s6m7;
-      const float l45 = s4 + tx * s5m4;
-      const float top = l45 + ty * (l76 - l45);
-      const float l01 = s0 + tx * s1m0;
-      const float l32 = s3 + tx * s2m3;
-      const float bot = l01 + ty * (l32 - l01);
-      float fs = bot + tz * (top - bot);
-      fs = (fs - g.min_scalar) * g.inv_delta;
-      const float fi = fs * g.n1f;
-      if (fi > -1.f && fi < g.n1f + 1.f) {
-        const float4 tfc = ld_shared4(T.tf + (__float_as_uint(__fadd_rz(fmaxf(fi, 0.f), 8388608.f)) << 4));
-        const float sa = tfc.w * (1.f - color.w);
-        if (rec) (*rec)(p, tfc, sa);
-        // a sample of alpha 0 adds 0 times its shading, which is 0 unless the shading is not finite
-        if (sa != 0.f || !g.tame) {
-          float sc0 = tfc.x, sc1 = tfc.y, sc2 = tfc.z;
-          if (USE_MAP) {
-            float pc[3];
-            const unsigned idx = map_cell(g, T, s_tab, p, pc);
-            if (MULTI) {
-              // the multi-light extension: sum over the maps of (1 - opacity_l) *
-              // light_colors[l], in light order, over one map grid
-              const size_t nv = (size_t)g.pd[0] * (unsigned)g.pd[1] * (unsigned)g.pd[2];
-              float e0 = 0.f, e1 = 0.f, e2 = 0.f;
-              for (int l = 0; l < g.n_lights; ++l) {
-                const float tr = 1.f - map_value(g, (const float*)map + l * nv, idx, pc);
-                const float t0 = tr * g.light_colors[l][0], t1 = tr * g.light_colors[l][1],
-                            t2 = tr * g.light_colors[l][2];
-                e0 = (l == 0) ? t0 : e0 + t0;
-                e1 = (l == 0) ? t1 : e1 + t1;
-                e2 = (l == 0) ? t2 : e2 + t2;
-              }
-              sc0 = sc0 * e0;
-              sc1 = sc1 * e1;
-              sc2 = sc2 * e2;
-            } else {
-              // exact form: 1 - opacity (TransmittanceMap.h:195); precision form: stored transmittance
-              const float mv = map_value(g, map, idx, pc);
-              const float tr = (sizeof(MapT) == 2) ? mv : 1.f - mv;
-              sc0 = sc0 * (tr * g.light_color[0]);
-              sc1 = sc1 * (tr * g.light_color[1]);
-              sc2 = sc2 * (tr * g.light_color[2]);
-            }
-          }
-          if (g.tame) {  // no NaN: clamp01 is a saturation
-            sc0 = __saturatef(sc0);
-            sc1 = __saturatef(sc1);
-            sc2 = __saturatef(sc2);
-          } else {
-            sc0 = clamp01(sc0);
-            sc1 = clamp01(sc1);
-            sc2 = clamp01(sc2);
-          }
-          color.x = color.x + sc0 * sa;
-          color.y = color.y + sc1 * sa;
-          color.z = color.z + sc2 * sa;
+        float tx = (p[0] - e0.x) * e0.z, ty = (p[1] - e1.x) * e1.z, tz = (p[2] - e2.x) * e2.z;
+        if (!(min3(tx, ty, tz) >= kFace && max3(tx, ty, tz) <= 1.f - kFace) || cell.kept) {
+          const ViewGrid grid{{g.fs[0], g.fs[1], g.fs[2]},
+                              {g.n[0], g.n[1], g.n[2]},
+                              {g.ax_off[0], g.ax_off[1], g.ax_off[2]},
+                              {g.org[0], g.org[1], g.org[2]},
+                              {g.seed[0], g.seed[1], g.seed[2]},
+                              {g.maxp[0], g.maxp[1], g.maxp[2]}};
+          const ViewFace f = view_cell_at_face(grid, s_tab, cell, p[0], p[1], p[2]);
+          cell = f.cell;
+          off = cell.off;
+          tx = f.t[0];
+          ty = f.t[1];
+          tz = f.t[2];
+          QuadLoad<QuadT>::cell(quads, off, g.fs[1], g.fs[2], v);
         }
-        color.w = sa + color.w;
-        ++lit;
+        cell.off = off;
+        shade_sample<USE_MAP, MapT, Rec, MULTI>(g, T, s_tab, map, p, view_interp(v, tx, ty, tz), color, lit, rec);
+        if (color.w >= g.cutoff) return;
+      }
+      dist += g.sd;
+      p[0] = p[0] + sd[0];
+      p[1] = p[1] + sd[1];
+      p[2] = p[2] + sd[2];
+      if (left > 0) {
+        --left;
+      } else if (!(inside_vol(g, p) && dist < maxD && budget-- > 0)) {
+        return;
       }
     }
-    dist += g.sd;
-    p[0] = p[0] + sd[0];
-    p[1] = p[1] + sd[1];
-    p[2] = p[2] + sd[2];
-    if (!skipped && color.w >= g.cutoff) return;
-    if (left > 0) {
-      --left;
-    } else if (!(inside_vol(g, p) && dist < maxD && budget-- > 0)) {
-      return;
-    }
-    tx = (p[0] - bl[0]) * inv[0];
-    ty = (p[1] - bl[1]) * inv[1];
-    tz = (p[2] - bl[2]) * inv[2];
   }
 }
 
