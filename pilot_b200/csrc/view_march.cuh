@@ -25,8 +25,8 @@ __device__ __forceinline__ int next_warp_tile(unsigned* counter) {
   return (int)__shfl_sync(0xffffffffu, t, 0);
 }
 
-// A view-march observer: called once per lit sample with its position, TF
-// entry and premultiplied alpha (the default observes nothing).
+// A view-march observer: called with the position, TF entry and premultiplied
+// alpha of every lit sample whose alpha is not 0 (the default observes nothing).
 struct NoRecord {
   __device__ __forceinline__ void operator()(const float*, const float4&, float) {}
 };
@@ -115,19 +115,21 @@ __device__ __forceinline__ float map_value(const ExactGeo& g, const MapT* __rest
 }
 
 // Shades and composites one sample at p whose interpolated field value is fs
-// (Sampler::operator(), LightedVolumeRenderer.cxx:440-489).
+// (Sampler::operator(), LightedVolumeRenderer.cxx:440-489). wild: shading may be
+// NaN (ExactGeo::tame is 0).
 template <bool USE_MAP, typename MapT, typename Rec, bool MULTI>
 __device__ __forceinline__ void shade_sample(const ExactGeo& g, const ViewTables& T, const float4* s_tab,
-                                             const MapT* __restrict__ map, const float p[3], float fs, float4& color,
+                                             const MapT* __restrict__ map, const float p[3], float fs, int wild, float4& color,
                                              unsigned& lit, Rec* rec) {
   const float fi = ((fs - g.min_scalar) * g.inv_delta) * g.n1f;
-  if (!(fi > -1.f && fi < g.n1f + 1.f)) return;
-  const float4 tfc = ld_shared4(T.tf + (__float_as_uint(__fadd_rz(fmaxf(fi, 0.f), 8388608.f)) << 4));
-  const float sa = tfc.w * (1.f - color.w);
-  if (rec) (*rec)(p, tfc, sa);
+  // a value outside the colour map's range is not lit and adds nothing (NaN too)
+  const bool in = fi > -1.f && fi < g.n1f + 1.f;
+  const float4 tfc = ld_shared4(T.tf + (__float_as_uint(__fadd_rz(fminf(fmaxf(fi, 0.f), g.n1f), 8388608.f)) << 4));
+  const float sa = in ? tfc.w * (1.f - color.w) : 0.f;
   // a sample of alpha 0 adds 0 times its shading, which is 0 unless the shading is not finite
-  if (sa != 0.f || !g.tame) {
-    float sc0 = tfc.x, sc1 = tfc.y, sc2 = tfc.z;
+  if (sa != 0.f || (wild && in)) {
+    if (rec) (*rec)(p, tfc, sa);  // observers look at samples of alpha above 0
+    float m0 = 1.f, m1 = 1.f, m2 = 1.f;
     if (USE_MAP) {
       float pc[3];
       const unsigned idx = map_cell(g, T, s_tab, p, pc);
@@ -135,41 +137,35 @@ __device__ __forceinline__ void shade_sample(const ExactGeo& g, const ViewTables
         // the multi-light extension: sum over the maps of (1 - opacity_l) *
         // light_colors[l], in light order, over one map grid
         const size_t nv = (size_t)g.pd[0] * (unsigned)g.pd[1] * (unsigned)g.pd[2];
-        float e0 = 0.f, e1 = 0.f, e2 = 0.f;
         for (int l = 0; l < g.n_lights; ++l) {
           const float tr = 1.f - map_value(g, (const float*)map + l * nv, idx, pc);
           const float t0 = tr * g.light_colors[l][0], t1 = tr * g.light_colors[l][1], t2 = tr * g.light_colors[l][2];
-          e0 = (l == 0) ? t0 : e0 + t0;
-          e1 = (l == 0) ? t1 : e1 + t1;
-          e2 = (l == 0) ? t2 : e2 + t2;
+          m0 = (l == 0) ? t0 : m0 + t0;
+          m1 = (l == 0) ? t1 : m1 + t1;
+          m2 = (l == 0) ? t2 : m2 + t2;
         }
-        sc0 = sc0 * e0;
-        sc1 = sc1 * e1;
-        sc2 = sc2 * e2;
       } else {
         // exact form: 1 - opacity (TransmittanceMap.h:195); precision form: stored transmittance
         const float mv = map_value(g, map, idx, pc);
         const float tr = (sizeof(MapT) == 2) ? mv : 1.f - mv;
-        sc0 = sc0 * (tr * g.light_color[0]);
-        sc1 = sc1 * (tr * g.light_color[1]);
-        sc2 = sc2 * (tr * g.light_color[2]);
+        m0 = tr * g.light_color[0];
+        m1 = tr * g.light_color[1];
+        m2 = tr * g.light_color[2];
       }
     }
-    if (g.tame) {  // no NaN: clamp01 is a saturation
-      sc0 = __saturatef(sc0);
-      sc1 = __saturatef(sc1);
-      sc2 = __saturatef(sc2);
-    } else {
-      sc0 = clamp01(sc0);
-      sc1 = clamp01(sc1);
-      sc2 = clamp01(sc2);
+    // without a NaN, clamp01 is the saturation that the product does for free
+    float sc0 = __saturatef(tfc.x * m0), sc1 = __saturatef(tfc.y * m1), sc2 = __saturatef(tfc.z * m2);
+    if (wild) {
+      sc0 = clamp01(tfc.x * m0);
+      sc1 = clamp01(tfc.y * m1);
+      sc2 = clamp01(tfc.z * m2);
     }
     color.x = color.x + sc0 * sa;
     color.y = color.y + sc1 * sa;
     color.z = color.z + sc2 * sa;
   }
   color.w = sa + color.w;
-  ++lit;
+  lit += in ? 1u : 0u;
 }
 
 // The reference's trilinear value (LightedVolumeRenderer.cxx:425-438) of the corner
@@ -318,6 +314,8 @@ __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT*
   int left = sure_steps(g, p, sd, dist, maxD, budget - 1);
   budget -= left + 1;
   const ViewTables T(g, s_tab, s_tf);
+  int wild = !g.tame;
+  asm volatile("" : "+r"(wild));  // in a register, not read again for every sample
   if constexpr (RECT) {
     // explicit coordinates: a binary search when a sample leaves its cell, so the
     // cell and its values are kept. No cell yet: t is NaN (inv starts at 0 for the
@@ -343,7 +341,8 @@ __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT*
         }
         QuadLoad<QuadT>::cell(quads, off, g.fs[1], g.fs[2], v);
       }
-      shade_sample<USE_MAP, MapT, Rec, MULTI>(g, T, s_tab, map, p, view_interp(v, t[0], t[1], t[2]), color, lit, rec);
+      shade_sample<USE_MAP, MapT, Rec, MULTI>(g, T, s_tab, map, p, view_interp(v, t[0], t[1], t[2]), wild, color,
+                                              lit, rec);
       dist += g.sd;
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
@@ -408,7 +407,7 @@ __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT*
           QuadLoad<QuadT>::cell(quads, off, g.fs[1], g.fs[2], v);
         }
         cell.off = off;
-        shade_sample<USE_MAP, MapT, Rec, MULTI>(g, T, s_tab, map, p, view_interp(v, tx, ty, tz), color, lit, rec);
+        shade_sample<USE_MAP, MapT, Rec, MULTI>(g, T, s_tab, map, p, view_interp(v, tx, ty, tz), wild, color, lit, rec);
         if (color.w >= g.cutoff) return;
       }
       dist += g.sd;
