@@ -121,7 +121,7 @@ beams_status make_geo_vol(beams_renderer* r, const beams_volume& v, const beams_
   g.bo_axis[2] = 1;
   // the renderer's own volume may carry explicit rectilinear coordinates
   const bool rect = r->rect && &v == &r->vol;
-  g.rect = rect ? 1 : 0;
+  g.rect = !rect ? 0 : (r->rect_near ? 1 : 2);
   for (int d = 0; d < 3; ++d) {
     g.n[d] = v.dims[d];
     if (rect) {
@@ -1044,8 +1044,15 @@ beams_status beams_set_volume_coordinates(beams_renderer* r, const float* x, con
       if (!std::isfinite(a[d][i]) || (i > 0 && !(a[d][i] > a[d][i - 1])))
         return fail(r, BEAMS_ERR_INVALID_ARG, "volume coordinates must be finite and strictly increasing");
   }
-  for (int d = 0; d < 3; ++d) r->coords[d].assign(a[d], a[d] + r->vol.dims[d]);
+  bool near = true;
+  for (int d = 0; d < 3; ++d) {
+    const int n = r->vol.dims[d];
+    r->coords[d].assign(a[d], a[d] + n);
+    const double mean = ((double)a[d][n - 1] - a[d][0]) / (n - 1);
+    for (int i = 0; i < n && near; ++i) near = std::fabs(((double)a[d][i] - a[d][0]) / mean - i) <= kRectNear;
+  }
   r->rect = true;
+  r->rect_near = near;
   ++r->volume_version;  // new cell tables, occupancy and map
   return BEAMS_OK;
 }

@@ -69,7 +69,8 @@ struct ExactGeo {
   // Explicit rectilinear coordinates (beams_set_volume_coordinates): the field
   // axes' cell tables hold the given coordinates and cells are found by
   // search instead of from the uniform spacing; org/h/invh then only describe
-  // the average spacing. 0: coord(d, i) = org[d] + h[d] * float(i).
+  // the average spacing. 0: coord(d, i) = org[d] + h[d] * float(i); 1: no cell is
+  // more than kRectNear from where the average spacing puts it; 2: any.
   int rect;
   // The light march's cell guess scale per field axis: 1 / h, lowered where
   // floor((maxp - org) * seed) would exceed n - 1, so that a guess always indexes
@@ -97,6 +98,7 @@ struct ExactGeo {
 constexpr int kMaxMultiLights = 8;
 
 constexpr int kMacroLog2 = 3;  // macro-cell edge = 8 field cells
+constexpr int kRectNear = 6;
 
 // What the stitch kernel needs of every other brick (multi-block scenes): its
 // bounds (for SegmentAABB) and its Phase-1 map with that map's geometry.

@@ -45,11 +45,11 @@ __device__ __forceinline__ void load_tables(float4* s_tab, const float4* __restr
 // Blocks per SM: 6 (40 registers), where the loads' latency is covered best (the
 // 257^3-vertex map of a 512^3 noise field, mean of eight light directions: 2.39 ms
 // against 2.63 ms at 4; skipping, 256^3 noise 0.40 against 0.44 ms, 384^3
-// bfloat16 0.99 against 1.04 ms); the rectilinear march, and the listed ones with
-// both ways to march a ray, spill there and keep 4.
-template <bool RECT, bool LIST>
+// bfloat16 0.99 against 1.04 ms; rectilinear, 160^3 0.34 against 0.37 ms); the listed
+// ones, with both ways to march a ray, spill there and keep 4.
+template <bool LIST>
 constexpr int k1_blocks_per_sm() {
-  return RECT || LIST ? 4 : 6;
+  return LIST ? 4 : 6;
 }
 
 // A masked map build (the exact form's lazy map, the learned form's fallback,
@@ -183,7 +183,7 @@ constexpr unsigned split_rays() {
 // the whole map's vertex order. SPLIT: kSplit lanes a ray (a list decides by its
 // own length).
 template <typename QuadT, bool STITCH, bool PREC, bool SKIP, bool RECT = false, bool LIST = false, bool SPLIT = false>
-__global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<RECT, LIST>()) k_light_march(const ExactGeo g, const QuadT* __restrict__ quads,
+__global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<LIST>()) k_light_march(const ExactGeo g, const QuadT* __restrict__ quads,
                                                           const float4* __restrict__ tab,
                                                           const float4* __restrict__ tf,
                                                           const float* __restrict__ tau,
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<RECT, LIST>()) k_li
       const LightRay ray = light_ray(g, V, L, dir);
       acc.init(STITCH ? stitch_prefix(refs, nrefs, self, L, V, dir) : 0.f);
       if constexpr (RECT) {
-        light_march_rect(g, quads, s_tab, s_a, ray, acc, ns);
+        light_march_rect<QuadT, PREC>(g, quads, s_tab, PREC ? s_tau : s_a, ray, acc, ns);
       } else {
         // the lanes leave the untested steps together
         const int sure = SKIP ? ray.sure : __reduce_min_sync(__activemask(), ray.sure);
@@ -706,11 +706,8 @@ static cudaError_t launch_k1(const ExactGeo& g, const void* quads, const float4*
 #define BEAMS_K1(SKIP, RECT, LIST, SPLIT)                                                                             \
   launch_k1_as<QuadT, STITCH, PREC, SKIP, RECT, LIST, SPLIT>(g, quads, tab, tf, tau, map, nslots, cnt, st, refs, nrefs, \
                                                              self, gate, occ, vlist)
-  if (g.rect && !PREC) {
-    // explicit rectilinear coordinates, exact form: binary-search cell location, no
-    // empty-space skipping (the precision form keeps the seeded walk, correct for
-    // any increasing coordinates)
-    if constexpr (!STITCH && !PREC && std::is_same<QuadT, float4>::value) {
+  if (g.rect) {  // explicit rectilinear coordinates: no empty-space skipping
+    if constexpr (!STITCH) {
       occ = nullptr;
       return vlist ? BEAMS_K1(false, true, true, false) : BEAMS_K1(false, true, false, false);
     } else {
@@ -743,23 +740,23 @@ static cudaError_t launch_mark(const ExactGeo& g, const QuadT* quads, const floa
   return cudaGetLastError();
 }
 
-// The precision form's view march reads the 16-bit quads and never takes the
-// rectilinear instantiation (its seeded walk serves both), so its marking
-// pass does the same.
+template <typename QuadT>
+static cudaError_t launch_mark_prec(const ExactGeo& g, const QuadT* quads, const float4* tab, const float4* tf,
+                                    unsigned char* cell_mask, Counters* cnt, cudaStream_t st,
+                                    const unsigned char* occ) {
+  if (g.rect) return launch_mark<true, false, false>(g, quads, tab, tf, cell_mask, cnt, nullptr, nullptr, st);
+  return occ ? launch_mark<false, false, true>(g, quads, tab, tf, cell_mask, cnt, nullptr, nullptr, st, occ)
+             : launch_mark<false, false, false>(g, quads, tab, tf, cell_mask, cnt, nullptr, nullptr, st);
+}
+
+// The precision form's marking pass reads the 16-bit quads its view march reads.
 cudaError_t launch_mark_view_cells_prec(const ExactGeo& g, int quad_dtype, const void* quads, const float4* tab,
                                         const float4* tf, unsigned char* cell_mask, Counters* cnt, cudaStream_t st,
                                         const unsigned char* occ) {
   cudaError_t e = cudaMemsetAsync(&cnt->tiles_mark, 0, sizeof(unsigned), st);
   if (e != cudaSuccess) return e;
-  if (quad_dtype == 1)
-    return occ ? launch_mark<false, false, true>(g, (const QuadBF16*)quads, tab, tf, cell_mask, cnt, nullptr, nullptr,
-                                                 st, occ)
-               : launch_mark<false, false, false>(g, (const QuadBF16*)quads, tab, tf, cell_mask, cnt, nullptr,
-                                                  nullptr, st);
-  return occ ? launch_mark<false, false, true>(g, (const QuadF16*)quads, tab, tf, cell_mask, cnt, nullptr, nullptr, st,
-                                               occ)
-             : launch_mark<false, false, false>(g, (const QuadF16*)quads, tab, tf, cell_mask, cnt, nullptr, nullptr,
-                                                st);
+  if (quad_dtype == 1) return launch_mark_prec(g, (const QuadBF16*)quads, tab, tf, cell_mask, cnt, st, occ);
+  return launch_mark_prec(g, (const QuadF16*)quads, tab, tf, cell_mask, cnt, st, occ);
 }
 
 cudaError_t launch_mark_view_cells(const ExactGeo& g, const float4* quads, const float4* tab, const float4* tf,
@@ -935,19 +932,19 @@ static cudaError_t launch_k2(const ExactGeo& g, const QuadT* quads, const float4
                              const MapT* map, float4* out, Counters* cnt, const unsigned char* occ, cudaStream_t st) {
   const size_t smem = ((size_t)g.ntab + (size_t)g.tf_n) * sizeof(float4);
   const int ntiles = (((g.win[2] + 7) >> 3) * ((g.win[3] + 3) >> 2) + 7) / 8;  // 8 warp tiles per block
-  int grid = 0;
-  cudaError_t e;
-  if (occ) {
-    e = persistent_grid(k_view_march<QuadT, USE_MAP, MapT, false, true, MULTI>, smem, ntiles, grid);
+  const auto run = [&](auto kernel, const unsigned char* skip) {
+    int grid = 0;
+    cudaError_t e = persistent_grid(kernel, smem, ntiles, grid);
     if (e != cudaSuccess) return e;
-    k_view_march<QuadT, USE_MAP, MapT, false, true, MULTI><<<grid, kThreads, smem, st>>>(g, quads, tab, tf, map, out, cnt,
-                                                                                  nullptr, nullptr, occ);
-  } else {
-    e = persistent_grid(k_view_march<QuadT, USE_MAP, MapT, false, false, MULTI>, smem, ntiles, grid);
-    if (e != cudaSuccess) return e;
-    k_view_march<QuadT, USE_MAP, MapT, false, false, MULTI><<<grid, kThreads, smem, st>>>(g, quads, tab, tf, map, out, cnt);
+    kernel<<<grid, kThreads, smem, st>>>(g, quads, tab, tf, map, out, cnt, nullptr, nullptr, skip);
+    return cudaGetLastError();
+  };
+  if constexpr (!MULTI) {
+    // explicit rectilinear coordinates (single light, no empty-space skipping)
+    if (g.rect) return run(k_view_march<QuadT, USE_MAP, MapT, false, false, false, true>, nullptr);
   }
-  return cudaGetLastError();
+  return occ ? run(k_view_march<QuadT, USE_MAP, MapT, false, true, MULTI>, occ)
+             : run(k_view_march<QuadT, USE_MAP, MapT, false, false, MULTI>, nullptr);
 }
 
 cudaError_t launch_view_march_f32(const ExactGeo& g, const float* field, const float4* quads, const float4* tab,
@@ -961,20 +958,8 @@ cudaError_t launch_view_march_f32(const ExactGeo& g, const float* field, const f
     e = persistent_grid(k_view_march_cells<float>, smem, ntiles, grid);
     if (e != cudaSuccess) return e;
     k_view_march_cells<float><<<grid, kThreads, smem, st>>>(g, field, tab, tf, out, cnt);
-  } else if (g.rect) {
-    // explicit rectilinear coordinates (single light, no empty-space skipping)
-    if (g.n_lights > 1) return cudaErrorInvalidValue;
-    if (g.use_map) {
-      e = persistent_grid(k_view_march<float4, true, float, false, false, false, true>, smem, ntiles, grid);
-      if (e != cudaSuccess) return e;
-      k_view_march<float4, true, float, false, false, false, true><<<grid, kThreads, smem, st>>>(g, quads, tab, tf,
-                                                                                                map, out, cnt);
-    } else {
-      e = persistent_grid(k_view_march<float4, false, float, false, false, false, true>, smem, ntiles, grid);
-      if (e != cudaSuccess) return e;
-      k_view_march<float4, false, float, false, false, false, true><<<grid, kThreads, smem, st>>>(
-          g, quads, tab, tf, (const float*)nullptr, out, cnt);
-    }
+  } else if (g.rect && g.n_lights > 1) {
+    return cudaErrorInvalidValue;
   } else if (g.use_map && g.n_lights > 1) {
     return launch_k2<float4, true, float, true>(g, quads, tab, tf, map, out, cnt, occ, st);  // the multi-light extension
   } else if (g.use_map) {

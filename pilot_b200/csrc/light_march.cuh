@@ -322,37 +322,60 @@ __device__ __forceinline__ void light_march_split(const ExactGeo& g, const Light
   if (j == 0) ns += n;
 }
 
-// The same for explicit rectilinear coordinates, where no guess from a uniform
-// spacing is close: binary-search cell location over the cell tables.
-__device__ __forceinline__ void light_march_rect(const ExactGeo& g, const float4* __restrict__ quads,
-                                                 const float4* s_tab, const float* s_a, const LightRay& ray,
-                                                 Accum<false>& acc, unsigned& ns) {
+// The same for explicit rectilinear coordinates, where a guess from a uniform
+// spacing only starts the search. vals: s_a (exact) or s_tau (precision).
+template <typename QuadT, bool PREC>
+__device__ __forceinline__ void light_march_rect(const ExactGeo& g, const QuadT* __restrict__ quads,
+                                                 const float4* s_tab, const float* vals, const LightRay& ray,
+                                                 Accum<PREC>& acc, unsigned& ns) {
   float s[3] = {ray.st[0], ray.st[1], ray.st[2]};
   const int n1 = g.tf_n - 1;
-  for (int b = g.light_budget; b > 0; --b) {
-    const float q0 = s[0] - ray.st[0], q1 = s[1] - ray.st[1], q2 = s[2] - ray.st[2];
-    if (!(q0 * q0 + q1 * q1 + q2 * q2 <= ray.len2)) break;
+  unsigned k = 0;
+  for (; k < (unsigned)g.light_budget; ++k) {
+    const bool sure = k < (unsigned)ray.sure;
+    if (!sure) {
+      const float q0 = s[0] - ray.st[0], q1 = s[1] - ray.st[1], q2 = s[2] - ray.st[2];
+      if (!(q0 * q0 + q1 * q1 + q2 * q2 <= ray.len2)) break;
+    }
 #pragma unroll
     for (int d = 0; d < 3; ++d) s[d] = s[d] + ray.sd[d];
-    if (!inside_vol(g, s)) break;
+    if (!sure && !inside_vol(g, s)) break;
     float pc[3];
-    unsigned qi = 0;
+    int cell[3];
+    float4 e[3];
+    if (g.rect == 1) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const float4* T = s_tab + g.ax_off[d];
-      float4 e;
-      const int c = find_cell_bsearch_rect(T, g.n[d] - 2, s[d], e);
-      qi += float_bits(e.y);
-      pc[d] = div_field(s[d] - e.x, e);
-      if (pc[d] != pc[d]) pc[d] = (s[d] - e.x) / (T[c + 1].x - e.x);
+      for (int d = 0; d < 3; ++d) {
+        cell[d] = trunc_small(fminf((s[d] - g.org[d]) * g.invh[d], (float)(g.n[d] - 2)));
+        e[d] = s_tab[g.ax_off[d] + cell[d]];
+      }
+#pragma unroll
+      for (int d = 0; d < 3; ++d) walk_cell_rect(s_tab + g.ax_off[d], g.n[d] - 2, s[d], cell[d], e[d]);
+    } else {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) cell[d] = find_cell_bsearch_rect(s_tab + g.ax_off[d], g.n[d] - 2, s[d], e[d]);
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) pc[d] = div_field(s[d] - e[d].x, e[d]);
+    const unsigned qi = float_bits(e[0].y) + float_bits(e[1].y) + float_bits(e[2].y);
+    const float sum = pc[0] + pc[1] + pc[2];
+    if (sum != sum) {  // an entry whose two-term division is not exact (see field_entry)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const float4* T = s_tab + g.ax_off[d] + cell[d];
+        pc[d] = (s[d] - T[0].x) / (T[1].x - T[0].x);
+      }
     }
     float v[8];
-    QuadLoad<float4>::cell(quads, qi, g.fs[1], g.fs[2], v);
+    QuadLoad<QuadT>::cell(quads, qi, g.fs[1], g.fs[2], v);
     float scalar = hex_interp(v, pc[0], pc[1], pc[2]);
     scalar = (scalar - g.min_scalar) * g.inv_delta;
-    ++ns;
-    if (acc.add(s_a[tf_index_clamped(scalar * (float)n1, n1)])) break;
+    if (acc.add(vals[tf_index_clamped(scalar * (float)n1, n1)])) {
+      ++k;
+      break;
+    }
   }
+  ns += k;
 }
 
 }  // namespace beams

@@ -144,6 +144,7 @@ struct beams_renderer {
   float bg_rgba[4] = {1.f, 1.f, 1.f, 1.f};
   // explicit rectilinear coordinates of the volume's point axes (beams_set_volume_coordinates)
   bool rect = false;
+  bool rect_near = false;  // no coordinate is more than kRectNear cells from its place at the mean spacing
   std::vector<float> coords[3];
   // canvas depth buffer (beams_set_depth_buffer) and the per-pixel ray limits derived from it
   bool depth_set = false;

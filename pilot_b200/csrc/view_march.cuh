@@ -317,7 +317,7 @@ __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT*
   int wild = !g.tame;
   asm volatile("" : "+r"(wild));  // in a register, not read again for every sample
   if constexpr (RECT) {
-    // explicit coordinates: a binary search when a sample leaves its cell, so the
+    // explicit coordinates: a search when a sample leaves its cell, so the
     // cell and its values are kept. No cell yet: t is NaN (inv starts at 0 for the
     // max-face rule).
     const float none = __int_as_float(0x7fffffff);
@@ -332,7 +332,7 @@ __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT*
           if (p[k] == g.maxp[k]) {
             e = A[g.n[k] - 2];  // the reference leaves invSpacing[k] unchanged here
           } else {
-            find_cell_walk_rect(A, g.n[k] - 2, p[k], e);
+            find_cell_walk_rect(A, g.n[k] - 2, g.org[k], g.invh[k], g.rect == 1, p[k], e);
             inv[k] = e.z;  // 1.f / (coord(c+1) - coord(c)), IEEE
           }
           bl[k] = e.x;
