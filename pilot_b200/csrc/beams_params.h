@@ -220,6 +220,27 @@ __host__ __device__ inline unsigned light_slots(const ExactGeo& g, int bl) {
          (((unsigned)g.pd[g.bo_axis[2]] + pad) & ~pad);
 }
 
+// Sets bo_axis and bo_shear, the light-aligned order, from the light's travel
+// direction at the volume centre in map-vertex units (v: the position of a point
+// light, kind 0, else the direction).
+inline void geo_light_order(ExactGeo& g, int kind, const double v[3]) {
+  double e[3];
+  for (int d = 0; d < 3; ++d) {
+    const double c = 0.5 * (g.bmin[d] + g.bmax[d]);
+    const double t = (kind == 0) ? c - v[d] : v[d];
+    e[d] = (g.msp[d] > 0.f) ? t / (double)g.msp[d] : 0.0;
+  }
+  int w = 2;
+  for (int d = 0; d < 3; ++d)
+    if (std::fabs(e[d]) > std::fabs(e[w])) w = d;
+  g.bo_axis[0] = w;
+  g.bo_axis[1] = (w == 0) ? 1 : 0;
+  g.bo_axis[2] = (w == 2) ? 1 : 2;
+  const bool ok = std::fabs(e[w]) > 0.0 && std::isfinite(e[w]);
+  for (int k = 0; k < 2; ++k)
+    g.bo_shear[k] = ok ? (int)std::lround(65536.0 * e[g.bo_axis[1 + k]] / e[w]) : 0;
+}
+
 // Derives seed, n1f and fs. Coordinates that are not finite in float32 (an origin
 // past its range) have no inside: their bounds become NaN, which no position
 // passes, so no guess is ever formed from them.

@@ -260,17 +260,6 @@ __device__ __forceinline__ int find_cell_walk_rect(const float4* T, int cmax, fl
   return lo;
 }
 
-// View-march cell search: RectilinearLocator::LocateCell (LightedVolumeRenderer.cxx:119-165)
-// walks to the unique cell with coord(c) <= p < coord(c+1).
-__device__ __forceinline__ int find_cell_walk_t(const float4* T, int cmax, float org, float invh, float p,
-                                                float4& e) {
-  int c = trunc_small(fminf(fmaxf((p - org) * invh, 0.f), (float)cmax));
-  while (c > 0 && p < T[c].x) --c;
-  while (c < cmax && p >= T[c + 1].x) ++c;
-  e = T[c];
-  return c;
-}
-
 // The view march's walk (the unique c with coord(c) <= p < coord(c+1)) that
 // settles seeded guesses off by a face, out of line like walk_cells_bsearch.
 static __device__ __noinline__ int walk_cell_view(const float4* T, int cmax, float p, int c) {

@@ -400,6 +400,7 @@ __global__ void __launch_bounds__(kThreads) k_view_march_cells(const ExactGeo g,
   load_tables(s_tab, tab, g.ntab);
   for (int i = threadIdx.x; i < g.tf_n; i += blockDim.x) s_tf[i] = tf[i];
   __syncthreads();
+  const CellTables cells(g, s_tab);
   const int tiles_x = (g.width + 7) >> 3;
   const int ntiles = tiles_x * ((g.height + 3) >> 2);
   unsigned lit = 0, hit = 0;
@@ -422,40 +423,38 @@ __global__ void __launch_bounds__(kThreads) k_view_march_cells(const ExactGeo g,
         p[2] = o[2] + dist * d[2];
       }
       const float sdx = g.sd * d[0], sdy = g.sd * d[1], sdz = g.sd * d[2];
-      bool newCell = true;
-      float tx = 2.f, ty = 2.f, tz = 2.f;
+      float tx = 2.f, ty = 2.f, tz = 2.f;  // outside any cell: the first sample locates its cell
       float4 sc = make_float4(0.f, 0.f, 0.f, 0.f);
       float bl[3] = {0.f, 0.f, 0.f};
       float inv[3] = {0.f, 0.f, 0.f};
-      int c[3] = {0, 0, 0};
       const int n1 = g.tf_n - 1;
-      const unsigned cx = (unsigned)(g.n[0] - 1), cxy = (unsigned)(g.n[0] - 1) * (unsigned)(g.n[1] - 1);
       while (inside_vol(g, p) && dist < maxD && budget-- > 0) {
-        const float mint = mn(tx, mn(ty, tz));
-        const float maxt = mx(tx, mx(ty, tz));
-        if (maxt > 1.f || mint < 0.f) newCell = true;
-        if (newCell) {
+        if (!(min3(tx, ty, tz) >= 0.f && max3(tx, ty, tz) <= 1.f)) {
+          unsigned cid = 0;  // the quads' strides are the cells'
+          if (g.rect) {
 #pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const float4* T = s_tab + g.ax_off[k];
-            float4 e;
-            if (p[k] == g.maxp[k]) {
-              c[k] = g.n[k] - 2;
-              e = T[c[k]];
-            } else {
-              c[k] = find_cell_walk_t(T, g.n[k] - 2, g.org[k], g.invh[k], p[k], e);
-              inv[k] = e.z;
+            for (int k = 0; k < 3; ++k) {
+              const float4* T = s_tab + g.ax_off[k];
+              float4 e;
+              if (p[k] == g.maxp[k]) {
+                e = T[g.n[k] - 2];
+              } else {
+                find_cell_walk_rect(T, g.n[k] - 2, g.org[k], g.invh[k], g.rect == 1, p[k], e);
+                inv[k] = e.z;
+              }
+              bl[k] = e.x;
+              cid += __float_as_uint(e.y);
             }
-            bl[k] = e.x;
+            tx = (p[0] - bl[0]) * inv[0];
+            ty = (p[1] - bl[1]) * inv[1];
+            tz = (p[2] - bl[2]) * inv[2];
+          } else {
+            cid = locate_view_cell(g, cells, p, guess(p[0], g.org[0], g.seed[0]), guess(p[1], g.org[1], g.seed[1]),
+                                   guess(p[2], g.org[2], g.seed[2]), inv, bl, tx, ty, tz);
           }
-          const unsigned cid = (unsigned)c[2] * cxy + (unsigned)c[1] * cx + (unsigned)c[0];
           const float v = FieldLoad<FieldT>::ld(field, cid);
           const float nsv = (v - g.min_scalar) * g.inv_delta;
           sc = s_tf[tf_index_clamped(nsv * (float)n1, n1)];
-          tx = (p[0] - bl[0]) * inv[0];
-          ty = (p[1] - bl[1]) * inv[1];
-          tz = (p[2] - bl[2]) * inv[2];
-          newCell = false;
         }
         const float alpha = sc.w * (1.f - color.w);
         color.x = color.x + sc.x * alpha;
