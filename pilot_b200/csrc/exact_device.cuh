@@ -99,6 +99,14 @@ __device__ __forceinline__ float brick_map_opacity(const BrickRef& R, const floa
   return hex_interp(v, pc[0], pc[1], pc[2]);
 }
 
+// Whether the float nearest t is the float nearest q, for a double t within 3 units
+// of its last place of q: t's float is normal and t lies more than 4 units from the
+// midpoint of two floats.
+__device__ __forceinline__ bool same_float(double t) {
+  const unsigned ex = ((unsigned)__double2hiint(t) >> 20) & 0x7ffu;
+  return ex - 897u <= 252u && (((unsigned)__double2loint(t) - 0x0ffffffcu) & 0x1fffffffu) > 8u;
+}
+
 // Cross-brick shadow prefix of one vertex ray (the reference's Phases 2-3,
 // LightedVolumeRenderer.cxx:968-1235, TransmittanceMap.h:387-453): every other
 // brick the segment light->vertex crosses (SegmentAABB hit, glancing hits
@@ -106,16 +114,36 @@ __device__ __forceinline__ float brick_map_opacity(const BrickRef& R, const floa
 // contributions are over-composited in increasing exit distance (HitSort;
 // ties by brick id). The over operator on opacity is a product of
 // transmittances, so no cross-brick exchange or sort of hit lists is needed.
+// The slab ratios (segment_aabb_b's) of all bricks divide by the same three
+// directions: they are products with their reciprocals, whose rounding to float is
+// the quotients' (same_float), else the divisions are made. With six double
+// divisions a brick the tests were most of a stitched march. MEASURED
 __device__ __forceinline__ float stitch_prefix(const BrickRef* __restrict__ refs, int nrefs, int self,
                                                const float L[3], const float V[3], const float dir[3]) {
   float ht[kMaxBricks], ho[kMaxBricks];
   int hb[kMaxBricks];
   int nh = 0;
+  float sdir[3] = {V[0] - L[0], V[1] - L[1], V[2] - L[2]};
+  const float len = sqrtf(sdir[0] * sdir[0] + sdir[1] * sdir[1] + sdir[2] * sdir[2]);
+  double r[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) r[d] = 1.0 / (double)(sdir[d] / len);
   for (int c = 0; c < nrefs; ++c) {
     if (c == self) continue;
     const BrickRef& R = refs[c];
-    float tmin, tmax;
-    segment_aabb_b(R.bmin, R.bmax, L, V, tmin, tmax);
+    float tmin = 0.f, tmax = __int_as_float(0x7f800000);
+    bool sure = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double q0 = (R.bmin[d] - (double)L[d]) * r[d], q1 = (R.bmax[d] - (double)L[d]) * r[d];
+      sure = sure && same_float(q0) && same_float(q1);
+      const float t0 = (float)q0, t1 = (float)q1;
+      tmin = mx(tmin, mn(t0, t1));
+      tmax = mn(tmax, mx(t0, t1));
+    }
+    if (tmin < 0.f) tmin = 1e-4f;
+    if (tmax > len) tmax = len;
+    if (!sure) segment_aabb_b(R.bmin, R.bmax, L, V, tmin, tmax);
     if (!(tmin <= tmax)) continue;
     const float P[3] = {L[0] + dir[0] * tmax, L[1] + dir[1] * tmax, L[2] + dir[2] * tmax};
     const float op = brick_map_opacity(R, P);

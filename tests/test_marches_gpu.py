@@ -16,7 +16,7 @@ import numpy as np
 import pytest
 
 from oracle import mlp_oracle as M
-from oracle.oracle import Oracle, quantize
+from oracle.oracle import Oracle, quantize, render_bricks
 from pilot_b200 import beams as B
 from pilot_b200 import scenes
 from test_rectilinear_gpu import check, stretched
@@ -165,6 +165,25 @@ def test_leaps_in_the_batched_form_change_nothing(cuda_device):
                     ref = ref or cur
                     assert cur[1] == ref[1], (skip, split, brick)
                     assert all(np.array_equal(a, b) for a, b in zip(out, ref[0])), (skip, split, brick)
+
+
+@pytest.mark.parametrize("light", LIGHTS + [(0, (0.5, 2.0, 0.5)), (0, (-1.0, 0.5, 0.25)), (1, (0.0, -3.0, 0.0))],
+                         ids=str)
+def test_stitched_maps_for_lights_on_and_along_brick_faces(cuda_device, light):
+    """Slab ratios of zero, without bound and undefined, where a product with the
+    direction's reciprocal may not stand for the quotient."""
+    s = dataclasses.replace(scenes.small(44, n=33, image=48, m=9, kind="noise"), dims=(33, 25, 29),
+                            light_kind=light[0], light=light[1], array=None)
+    bricks = scenes.split_bricks(s, (2, 3, 2))
+    img, _, _, maps, lit = render_bricks(bricks)
+    with B.Renderer(0) as r:
+        bricks[0].configure(r)
+        r.set_bricks([(b.field_numpy(), b.origin, b.spacing, b.value_range) for b in bricks])
+        got, t = r.render(s.camera())
+        assert t["lit_samples"] == lit
+        for b in range(len(bricks)):
+            assert np.array_equal(r.get_brick_map(b, 1, 1000), np.ravel(maps[b])), b
+    check(got, img)
 
 
 @pytest.mark.parametrize("nextra", [1, 3])
