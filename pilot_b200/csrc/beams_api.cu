@@ -674,6 +674,7 @@ beams_status render_bricks(beams_renderer* r, const beams_camera* cam, float4* o
   e = cudaMemsetAsync(r->d_brick_cnt, 0, nb * sizeof(Counters), r->stream);
   if (e != cudaSuccess) return cuda_fail(r, e, "clearing brick counters");
   auto lane = [&](int b) { return r->brick_lane[b % beams_renderer::kBrickLanes]; };
+  for (ExactGeo& g : G) g.light_marches = std::min(nb, beams_renderer::kBrickLanes);
   const bool lazy = r->lazy_map && r->use_map;
   auto lane_fail = [&](cudaError_t err, const char* what) {
     brick_lanes_join(r);

@@ -174,9 +174,11 @@ __global__ void __launch_bounds__(256) k_list_marked_vertices(const ExactGeo g, 
 // 108 and 118 us). The precision form's sums cost more in the split march (41^3
 // vertices 62 and 53 us, 49^3 65 and 70 us).
 constexpr int kSplit = 4;
+// The limits are for the rays of all launches in flight (the bricks of a scene run
+// side by side): 27 bricks of 33^3 vertices, split, took SPLIT27.
 template <bool PREC>
-constexpr unsigned split_rays() {
-  return PREC ? 100000u : 160000u;
+__host__ __device__ inline unsigned split_rays(const ExactGeo& g) {
+  return (PREC ? 100000u : 160000u) / (unsigned)(g.light_marches > 1 ? g.light_marches : 1);
 }
 
 // LIST: the vertices come from a work list (k_list_marked_vertices) instead of
@@ -220,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<LIST>()) k_light_ma
   if (threadIdx.x == 0) light_order_setup(g, s_lo);
   __syncthreads();
   const unsigned nrays = LIST ? vlist[0] : nslots;
-  const bool split = !RECT && (SPLIT || (LIST && nrays <= split_rays<PREC>()));
+  const bool split = !RECT && (SPLIT || (LIST && nrays <= (STITCH ? split_rays<PREC>(g) : (PREC ? 100000u : 160000u))));
   const int ntiles = split ? (int)((nrays + 32 / kSplit - 1) / (32 / kSplit)) : (int)((nrays + 31u) >> 5);
   const int bl = g.light_brick_log2;
   unsigned ns = 0, built = 0;
@@ -720,7 +722,7 @@ static cudaError_t launch_k1(const ExactGeo& g, const void* quads, const float4*
       return occ ? BEAMS_K1(true, false, true, false) : BEAMS_K1(false, false, true, false);
     }
   }
-  if (nslots <= split_rays<PREC>()) return occ ? BEAMS_K1(true, false, false, true) : BEAMS_K1(false, false, false, true);
+  if (nslots <= split_rays<PREC>(g)) return occ ? BEAMS_K1(true, false, false, true) : BEAMS_K1(false, false, false, true);
   return occ ? BEAMS_K1(true, false, false, false) : BEAMS_K1(false, false, false, false);
 #undef BEAMS_K1
 }

@@ -202,14 +202,14 @@ struct beams_renderer {
   // Per-brick launches run on kBrickLanes side streams (fork/join by events),
   // so one brick's launch fills the SMs that the previous one's tail leaves
   // idle; each brick has its own work counters (d_brick_cnt[b]).
-  static constexpr int kBrickLanes = 4;
-  cudaStream_t brick_lane[kBrickLanes] = {nullptr, nullptr, nullptr, nullptr};
+  static constexpr int kBrickLanes = 8;
+  cudaStream_t brick_lane[kBrickLanes] = {};
   unsigned char* d_shell_mask = nullptr;  // Phase 1's outer-cell-layer mask
   bool shell_listed = false;              // this frame's Phase 1 ran over the shell's list (d_vlist)
   size_t shell_cap = 0;
   int shell_pd[3] = {0, 0, 0};
   cudaEvent_t brick_fork = nullptr;
-  cudaEvent_t brick_join[kBrickLanes] = {nullptr, nullptr, nullptr, nullptr};
+  cudaEvent_t brick_join[kBrickLanes] = {};
   beams::Counters* d_brick_cnt = nullptr;  // kMaxBricks entries
 
   // learned form: parameters, optimiser state, inference weights
