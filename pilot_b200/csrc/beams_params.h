@@ -53,7 +53,7 @@ struct ExactGeo {
   // rays in flight stay in a narrow corridor towards the light, so the field
   // they read stays in L2, and a warp's rays run side by side.
   int light_brick_log2;
-  // Light marches of like size in flight at a time (0 or 1: this one alone).
+  // Stitched light marches in flight at a time (at least 1 in those).
   int light_marches;
   // That order's axes: columns run along bo_axis[0] (the axis the light travels
   // most along, in map-vertex units), the two other coordinates (bo_axis[1],

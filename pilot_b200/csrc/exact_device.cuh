@@ -117,7 +117,8 @@ __device__ __forceinline__ bool same_float(double t) {
 // The slab ratios (segment_aabb_b's) of all bricks divide by the same three
 // directions: they are products with their reciprocals, whose rounding to float is
 // the quotients' (same_float), else the divisions are made. With six double
-// divisions a brick the tests were most of a stitched march. MEASURED
+// divisions a brick the maps of 27 bricks (65^3 vertices each, 257^3 points in all)
+// took 2.68 ms, with the products 2.49 (8 bricks: 0.70 and 0.69).
 __device__ __forceinline__ float stitch_prefix(const BrickRef* __restrict__ refs, int nrefs, int self,
                                                const float L[3], const float V[3], const float dir[3]) {
   float ht[kMaxBricks], ho[kMaxBricks];

@@ -174,11 +174,14 @@ __global__ void __launch_bounds__(256) k_list_marked_vertices(const ExactGeo g, 
 // 108 and 118 us). The precision form's sums cost more in the split march (41^3
 // vertices 62 and 53 us, 49^3 65 and 70 us).
 constexpr int kSplit = 4;
-// The limits are for the rays of all launches in flight (the bricks of a scene run
-// side by side): 27 bricks of 33^3 vertices, split, took SPLIT27.
-template <bool PREC>
+// In a stitched march every lane of a ray computes its prefix, and the bricks' launches
+// fill the GPU together, so there the limit is for all launches in flight: the maps of
+// 27 bricks of 33^3 vertices took 1.03 ms split, 0.57 not; of 8 bricks of 25^3 vertices
+// 0.16 and 0.15. The bricks' lists of shell vertices gain from the split all the same
+// (8 of 47,600 vertices: the maps 0.69 ms with it, 0.71 without).
+template <bool STITCH, bool PREC>
 __host__ __device__ inline unsigned split_rays(const ExactGeo& g) {
-  return (PREC ? 100000u : 160000u) / (unsigned)(g.light_marches > 1 ? g.light_marches : 1);
+  return (PREC ? 100000u : 160000u) / (STITCH ? (unsigned)g.light_marches : 1u);
 }
 
 // LIST: the vertices come from a work list (k_list_marked_vertices) instead of
@@ -222,7 +225,7 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<LIST>()) k_light_ma
   if (threadIdx.x == 0) light_order_setup(g, s_lo);
   __syncthreads();
   const unsigned nrays = LIST ? vlist[0] : nslots;
-  const bool split = !RECT && (SPLIT || (LIST && nrays <= (STITCH ? split_rays<PREC>(g) : (PREC ? 100000u : 160000u))));
+  const bool split = !RECT && (SPLIT || (LIST && nrays <= split_rays<STITCH, PREC>(g)));
   const int ntiles = split ? (int)((nrays + 32 / kSplit - 1) / (32 / kSplit)) : (int)((nrays + 31u) >> 5);
   const int bl = g.light_brick_log2;
   unsigned ns = 0, built = 0;
@@ -722,7 +725,7 @@ static cudaError_t launch_k1(const ExactGeo& g, const void* quads, const float4*
       return occ ? BEAMS_K1(true, false, true, false) : BEAMS_K1(false, false, true, false);
     }
   }
-  if (nslots <= split_rays<PREC>(g)) return occ ? BEAMS_K1(true, false, false, true) : BEAMS_K1(false, false, false, true);
+  if (nslots <= split_rays<STITCH, PREC>(g)) return occ ? BEAMS_K1(true, false, false, true) : BEAMS_K1(false, false, false, true);
   return occ ? BEAMS_K1(true, false, false, false) : BEAMS_K1(false, false, false, false);
 #undef BEAMS_K1
 }
