@@ -594,11 +594,16 @@ beams_status check_ready(beams_renderer* r) {
   return BEAMS_OK;
 }
 
+// The lanes a scene uses: brick b runs on lane b mod kBrickLanes.
+static int brick_lanes(const beams_renderer* r) {
+  return std::min((int)r->bricks.size(), beams_renderer::kBrickLanes);
+}
+
 // Side streams, events and per-brick counters of the per-brick launches (created on first use).
 static beams_status brick_lanes_ready(beams_renderer* r) {
   cudaError_t e = cudaSuccess;
   if (!r->brick_fork) e = cudaEventCreateWithFlags(&r->brick_fork, cudaEventDisableTiming);
-  for (int l = 0; l < beams_renderer::kBrickLanes && e == cudaSuccess; ++l) {
+  for (int l = 0; l < brick_lanes(r) && e == cudaSuccess; ++l) {
     if (!r->brick_lane[l]) e = cudaStreamCreateWithFlags(&r->brick_lane[l], cudaStreamNonBlocking);
     if (e == cudaSuccess && !r->brick_join[l]) e = cudaEventCreateWithFlags(&r->brick_join[l], cudaEventDisableTiming);
   }
@@ -610,7 +615,7 @@ static beams_status brick_lanes_ready(beams_renderer* r) {
 // The fork of work onto the lanes: every lane waits for what r->stream has queued so far.
 static beams_status brick_lanes_fork(beams_renderer* r) {
   cudaError_t e = cudaEventRecord(r->brick_fork, r->stream);
-  for (int l = 0; l < beams_renderer::kBrickLanes && e == cudaSuccess; ++l)
+  for (int l = 0; l < brick_lanes(r) && e == cudaSuccess; ++l)
     e = cudaStreamWaitEvent(r->brick_lane[l], r->brick_fork, 0);
   if (e != cudaSuccess) return cuda_fail(r, e, "forking brick streams");
   return BEAMS_OK;
@@ -619,7 +624,7 @@ static beams_status brick_lanes_fork(beams_renderer* r) {
 // r->stream waits for everything queued on the lanes (called on error paths too).
 static cudaError_t brick_lanes_join(beams_renderer* r) {
   cudaError_t first = cudaSuccess;
-  for (int l = 0; l < beams_renderer::kBrickLanes; ++l) {
+  for (int l = 0; l < brick_lanes(r); ++l) {
     cudaError_t e = cudaEventRecord(r->brick_join[l], r->brick_lane[l]);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(r->stream, r->brick_join[l], 0);
     if (e != cudaSuccess && first == cudaSuccess) first = e;
@@ -674,7 +679,7 @@ beams_status render_bricks(beams_renderer* r, const beams_camera* cam, float4* o
   e = cudaMemsetAsync(r->d_brick_cnt, 0, nb * sizeof(Counters), r->stream);
   if (e != cudaSuccess) return cuda_fail(r, e, "clearing brick counters");
   auto lane = [&](int b) { return r->brick_lane[b % beams_renderer::kBrickLanes]; };
-  for (ExactGeo& g : G) g.light_marches = std::min(nb, beams_renderer::kBrickLanes);
+  for (ExactGeo& g : G) g.light_marches = brick_lanes(r);
   const bool lazy = r->lazy_map && r->use_map;
   auto lane_fail = [&](cudaError_t err, const char* what) {
     brick_lanes_join(r);
