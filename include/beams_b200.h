@@ -497,8 +497,8 @@ beams_status beams_render_noalloc(const beams_volume* vol, const float* tf_rgba_
 /* Fault injection for tests (no reference counterpart): the nth following device
  * buffer allocation of any renderer fails with BEAMS_ERR_OOM (0 disarms). */
 beams_status beams_test_fail_allocation(int nth);
-/* Checks, on the device, the kernels' correctly rounded division (Markstein's
- * correction on a tabulated reciprocal) against IEEE division for every cell
+/* Checks, on the device, the kernels' correctly rounded division (a product and an
+ * fma with a tabulated two-term reciprocal) against IEEE division for every cell
  * width of the counting coordinates origin + i*spacing (ncells cells) and
  * `samples` numerators per width. No reference counterpart (test support). */
 beams_status beams_selftest_division(float origin, float spacing, int ncells, int samples,

@@ -452,20 +452,12 @@ __device__ __forceinline__ bool light_slot_vertex(unsigned slot, int bl, const i
 // Quad layout of a point field: Q[z][y][x] = {f(x,y,z), f(x,y+1,z), f(x+1,y,z),
 // f(x+1,y+1,z)} for x < nx-1, y < ny-1, so one cell is two 16-byte loads
 // (z and z+1). VTK corner order 0..7 = lo.x lo.y lo.w lo.z hi.x hi.y hi.w hi.z.
-// Cell (x, y, z) is entry qi = z qz + y qx + x; strides() gives qx and qz.
+// Cell (x, y, z) is entry qi = z qz + y qx + x, qx and qz = ExactGeo::fs[1] and fs[2].
 // FieldF32 reads the float32 field itself (x fastest, eight scalar loads per
 // cell; qx = nx, qz = nx ny): the allocation-free entry point's layout.
 template <typename Q> struct QuadLoad;
 struct FieldF32 { float v; };
-__device__ __forceinline__ void quad_strides(const ExactGeo& g, unsigned& qx, unsigned& qz) {
-  qx = (unsigned)(g.n[0] - 1);
-  qz = qx * (unsigned)(g.n[1] - 1);
-}
 template <> struct QuadLoad<FieldF32> {
-  static __device__ __forceinline__ void strides(const ExactGeo& g, unsigned& qx, unsigned& qz) {
-    qx = (unsigned)g.n[0];
-    qz = qx * (unsigned)g.n[1];
-  }
   static __device__ __forceinline__ void cell(const FieldF32* __restrict__ q, unsigned qi, unsigned qx, unsigned qz,
                                               float v[8]) {
     const float* f = reinterpret_cast<const float*>(q) + qi;
@@ -487,7 +479,6 @@ __device__ __forceinline__ float bf16_hi(unsigned u) { return __uint_as_float(u 
 __device__ __forceinline__ float f16_lo(unsigned u) { return __half2float(__ushort_as_half((unsigned short)(u & 0xffffu))); }
 __device__ __forceinline__ float f16_hi(unsigned u) { return __half2float(__ushort_as_half((unsigned short)(u >> 16))); }
 template <> struct QuadLoad<QuadBF16> {
-  static __device__ __forceinline__ void strides(const ExactGeo& g, unsigned& qx, unsigned& qz) { quad_strides(g, qx, qz); }
   static __device__ __forceinline__ void cell(const QuadBF16* __restrict__ q, unsigned qi, unsigned, unsigned qz, float v[8]) {
     const uint2 a = __ldg((const uint2*)(q + qi));
     const uint2 b = __ldg((const uint2*)(q + qi + qz));
@@ -496,7 +487,6 @@ template <> struct QuadLoad<QuadBF16> {
   }
 };
 template <> struct QuadLoad<QuadF16> {
-  static __device__ __forceinline__ void strides(const ExactGeo& g, unsigned& qx, unsigned& qz) { quad_strides(g, qx, qz); }
   static __device__ __forceinline__ void cell(const QuadF16* __restrict__ q, unsigned qi, unsigned, unsigned qz, float v[8]) {
     const uint2 a = __ldg((const uint2*)(q + qi));
     const uint2 b = __ldg((const uint2*)(q + qi + qz));
@@ -505,7 +495,6 @@ template <> struct QuadLoad<QuadF16> {
   }
 };
 template <> struct QuadLoad<float4> {
-  static __device__ __forceinline__ void strides(const ExactGeo& g, unsigned& qx, unsigned& qz) { quad_strides(g, qx, qz); }
   static __device__ __forceinline__ void cell(const float4* __restrict__ q, unsigned qi, unsigned, unsigned qz, float v[8]) {
     const float4 a = __ldg(q + qi);
     const float4 b = __ldg(q + qi + qz);

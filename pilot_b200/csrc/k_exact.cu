@@ -12,10 +12,10 @@
 // Both marches are instruction-bound (the field and map are served from L1/L2),
 // so the layout is chosen to cut instructions per sample:
 //  * the field is read as 4-corner quads (two 16-byte loads per cell);
-//  * per-axis cell tables {lo, hi, RN(1/(hi-lo))} live in shared memory, so a
-//    cell search is one guess plus rare fix-ups, and the parametric division is
-//    Markstein's correction on the tabulated reciprocal;
-//  * blocks are persistent and take 256-ray tiles from an atomic counter.
+//  * per-axis cell tables {lo, offset, rh, rl} live in shared memory (field_entry),
+//    so a cell search is one guess plus rare fix-ups and the parametric division a
+//    product and an fma with the two-term reciprocal rh + rl;
+//  * warps of persistent blocks take 32-ray tiles from an atomic counter.
 // Compiled with -fmad=false (see exact_device.cuh).
 #include <cuda_runtime.h>
 
