@@ -250,7 +250,8 @@ beams_status beams_get_ray_limits(beams_renderer* r, const beams_camera* cam, fl
 beams_status beams_set_multi_light(beams_renderer* r, int enable);
 /* Launch tuning (no reference counterpart; results do not depend on it).
  * light_brick: the order in which the map build takes its vertices: 0 = rows
- * (x fastest), or cubic bricks of 8 (default), 16, 32 or 64 vertices per edge.
+ * (x fastest), or columns along the light in groups of 8 x 8 (default), 16 x 16,
+ * 32 x 32 or 64 x 64.
  * no_empty_skip: 1 turns off the map build's skipping of 8^3-cell macro-cells
  * whose values all map to colour-map alpha 0 (such samples change nothing).
  * no_view_skip: the same for the view march (skipped samples still count as lit). */
@@ -318,7 +319,7 @@ typedef struct beams_request {
 typedef struct beams_batch_options {
   int tile_w, tile_h;       /* view work item in pixels (default 32 x 32): tile_w a multiple of 8, tile_h of 4,
                                at most 16384 pixels; warps take its 8 x 4 sub-tiles */
-  int light_brick;          /* map-build vertex order: 0 rows, 8/16/32/64 bricks */
+  int light_brick;          /* map-build vertex order: 0 rows, 8/16/32/64 columns along the light */
   int use_graph;            /* 1: capture once, replay (default) */
   int no_skip;              /* 1: no empty-space skipping (default 0: both marches skip empty macro-cells) */
   int split;                /* 1: two launches, every request's map build and then every view march, each

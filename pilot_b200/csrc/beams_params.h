@@ -49,7 +49,7 @@ struct ExactGeo {
   int max_off[3];  // offset of map axis d in the table
   int ntab;        // total table entries
   // K1 vertex order: 0 = x-fastest rows of the vertex grid; b > 0 = columns
-  // along the light in bricks of 2^b vertices per edge (light_slot_vertex): the
+  // along the light in groups of 2^b x 2^b (light_slot_vertex): the
   // rays in flight stay in a narrow corridor towards the light, so the field
   // they read stays in L2, and a warp's rays run side by side.
   int light_brick_log2;

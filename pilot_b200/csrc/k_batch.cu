@@ -5,7 +5,7 @@
 // by a view march. Here a batch of requests (each its own volume, camera,
 // light and map size) is one grid of persistent blocks pulling work items from
 // a global queue (batch.h): map-build items (kBatchChunk vertex slots of the
-// light-aligned brick order each) and view items (a tile of pixels), with the
+// light-aligned vertex order each) and view items (a tile of pixels), with the
 // map items of one request beside the view items of the one before it. A view
 // item of request r waits, with a bounded wait, until all of r's map items have
 // completed, so the grid never drains between the two stages. Queue order

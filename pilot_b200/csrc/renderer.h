@@ -126,7 +126,7 @@ struct beams_renderer {
   float density_scale = 1.f;  // SetDensityScale: stored, never read (as in the reference)
   float light_steps = 128.f;
   int slab_fp64 = 1;
-  int light_brick_log2 = 3;  // beams_set_tuning (8^3-vertex bricks)
+  int light_brick_log2 = 3;  // beams_set_tuning (columns in groups of 8 x 8)
   bool reuse_map = false;
   // beams_set_lazy_shadow_map: the exact form builds only the map vertices
   // that the frame's view rays read (d_cell_mask marks their cells)
