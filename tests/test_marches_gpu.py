@@ -309,6 +309,22 @@ def test_network_features_by_pairs(cuda_device, n):
     assert np.all(np.abs(got - ref) <= np.abs(ref) * 2.0 ** -7 + 1e-3)
 
 
+@pytest.mark.parametrize("n", [127, 129, 148 * 128, 148 * 128 + 1, 6 * 148 * 128 + 5])
+def test_dense_forward_around_its_tile_rounds(cuda_device, n):
+    """Tiles are dealt to the CTAs' first pipelines, then their second, ...: one tile, a full
+    round of first pipelines, one more, all six and a partial one. Bar: the rows' T equal the
+    training kernel's, which deals its tiles otherwise, bit for bit (the same operations)."""
+    s = scenes.small(83, n=24, image=16, m=8)
+    rng = np.random.default_rng(n)
+    with renderer(s) as r:
+        r.mlp_set_params(rng.normal(0, 0.15, M.N_PARAMS).astype(np.float32))
+        X = np.tile(rng.normal(0, 0.5, (1009, 112)).astype(np.float32), (n // 1009 + 1, 1))[:n]  # prime: no tile repeats
+        T = r.mlp_forward_tc(X)
+        _, _, T_train = r.mlp_loss_grad(X, np.zeros(n, np.float32))
+    assert np.all(np.isfinite(T)) and np.array_equal(T, T_train)
+    assert np.array_equal(T[1009:], T[:-1009] if n > 1009 else T[1009:])
+
+
 def test_training_buffers_kept_between_sizes(cuda_device):
     """The training set's buffers are kept up to 256 MB: a smaller set, a larger one
     that is given back, and the first again. Bar: the same seed's loss; the sums'
