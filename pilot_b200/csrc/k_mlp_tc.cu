@@ -471,13 +471,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train_tc(const __grid_const
   const int ntiles = (n + kTile - 1) / kTile;
   const bool bwd = G != nullptr;
 
-  stage_weights(P, sm, aux);
+  // What needs none of the preceding launch's results comes before the wait for it
   if (tid == 0) {
     mbar_init(bar_load, 1);
     mbar_init(bar_mma, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) tmem_alloc(&s_tmem, kTrCols);
+  launch_dependents();
+  wait_for_preceding();
+  stage_weights(P, sm, aux);
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
@@ -741,8 +744,7 @@ cudaError_t mlp_train_step_tc(const float* P, float* G, const __nv_bfloat16* X, 
   const int tiles = (n + kTile - 1) / kTile;
   int grid = sm_count();
   if (grid > tiles) grid = tiles;
-  k_mlp_train_tc<<<grid, kThreads, kTrSmem + 1024, st>>>(map, 0, n, P, target, scale, G, T, loss, err);
-  return cudaGetLastError();
+  return launch_early(k_mlp_train_tc, grid, kThreads, kTrSmem + 1024, st, map, 0, n, P, target, scale, G, T, loss, err);
 }
 
 }  // namespace beams

@@ -269,6 +269,8 @@ __global__ void k_head_wgrad(const __nv_bfloat16* __restrict__ H4, const float* 
 
 __global__ void k_adam(float* __restrict__ P, float* __restrict__ G, float* __restrict__ m, float* __restrict__ v,
                        int n, float lr, float b1, float b2, float eps, float c1, float c2) {
+  wait_for_preceding();  // the gradient of the whole step
+  launch_dependents();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float g = G[i];
     const float mi = b1 * m[i] + (1.f - b1) * g;
@@ -349,8 +351,7 @@ cudaError_t mlp_fwd_bwd(const float* P, float* G, const __nv_bfloat16* X, const 
 cudaError_t mlp_adam(float* P, float* G, float* m, float* v, float lr, int t, cudaStream_t st) {
   const float b1 = 0.9f, b2 = 0.99f;
   const float c1 = 1.f - powf(b1, (float)t), c2 = 1.f - powf(b2, (float)t);
-  k_adam<<<grid_cap(kParams, 256), 256, 0, st>>>(P, G, m, v, kParams, lr, b1, b2, 1e-8f, c1, c2);
-  return cudaGetLastError();
+  return launch_early(k_adam, (int)grid_cap(kParams, 256), 256, 0, st, P, G, m, v, kParams, lr, b1, b2, 1e-8f, c1, c2);
 }
 
 }  // namespace beams

@@ -325,6 +325,22 @@ def test_dense_forward_around_its_tile_rounds(cuda_device, n):
     assert np.array_equal(T[1009:], T[:-1009] if n > 1009 else T[1009:])
 
 
+@pytest.mark.parametrize("batch", [256, 512])
+def test_overlapped_training_steps_follow_the_separate_ones(cuda_device, batch):
+    """The step's two launches overlap their starts; the CUDA-core path runs whole launches
+    one after the other. Bar: the held-out error after one epoch within 2% of the first
+    error, the bound on the two backward passes' relative difference per step."""
+    s = scenes.small(84, n=24, image=16, m=8)
+    out = []
+    for tensor in (True, False):
+        with renderer(s) as r:
+            r.mlp_set_tensor_cores(tensor)
+            rep = r.mlp_train(B.mlp_options(samples_log2=14, epochs=1, batch=batch, lr=1e-3))
+            out.append((rep["initial_rmse"], rep["holdout_rmse"]))
+    assert out[0][1] < out[0][0]
+    assert abs(out[0][1] - out[1][1]) <= 0.02 * out[1][0]
+
+
 def test_training_buffers_kept_between_sizes(cuda_device):
     """The training set's buffers are kept up to 256 MB: a smaller set, a larger one
     that is given back, and the first again. Bar: the same seed's loss; the sums'
