@@ -816,7 +816,9 @@ cudaError_t launch_light_march_prec(const ExactGeo& g, int quad_dtype, const voi
 // Emptiness of the 8^3-cell macro-cells under the colour map: 1 when every value
 // the trilinear interpolation can produce inside cells [8m - 1, 8m + 8] (per axis)
 // maps to a TF entry of alpha 0 that lies inside the TF's index range (so a
-// skipped view sample still counts as lit). The range is widened by a relative
+// skipped view sample still counts as lit). A negative alpha is not 0: the light
+// march of a map without a positive one adds nothing, but the view march adds it.
+// The range is widened by a relative
 // margin (the interpolation can overshoot its corners by a few ulps) and the TF
 // index range by 0.01 on each side; a NaN corner makes the range infinite and so
 // the macro-cell not empty, and a macro-cell touching a volume max face is not
@@ -826,7 +828,7 @@ __global__ void __launch_bounds__(256) k_macro_empty(const ExactGeo g, const flo
                                                      const float4* __restrict__ tf, unsigned char* __restrict__ empty) {
   // s_next[i]: the first TF entry from i on whose alpha is not 0 (tf_n when there is none)
   __shared__ short s_next[1024];
-  for (int i = threadIdx.x; i < g.tf_n; i += blockDim.x) s_next[i] = (g.max_alpha > 0.f && tf[i].w != 0.f) ? 1 : 0;
+  for (int i = threadIdx.x; i < g.tf_n; i += blockDim.x) s_next[i] = tf[i].w != 0.f ? 1 : 0;
   __syncthreads();
   if (threadIdx.x == 0) {
     short next = (short)g.tf_n;
