@@ -162,7 +162,7 @@ beams_status make_geo_vol(beams_renderer* r, const beams_volume& v, const beams_
     for (int l = 0; l < g.n_lights; ++l)
       for (int d = 0; d < 3; ++d) g.light_colors[l][d] = r->lights[l].color[d] * r->lights[l].intensity;
   }
-  bool tame = true;  // the colour map's entries are finite (beams_set_color_map)
+  bool tame = map_cells_have_width(g);  // the colour map's entries are finite (beams_set_color_map)
   for (int i = 0; i < r->tf_n; ++i) tame = tame && r->tf[4 * i + 3] >= 0.f;
   for (int l = 0; l < g.n_lights; ++l)
     for (int d = 0; d < 3; ++d) tame = tame && std::fabs(g.light_colors[l][d]) <= 1e30f;

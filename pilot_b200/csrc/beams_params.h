@@ -83,8 +83,9 @@ struct ExactGeo {
   // quads' {1, n0 - 1, (n0 - 1)(n1 - 1)}, or the plain field's (set by
   // geo_loop_constants); cell (x, y, z) is entry fs . (x, y, z).
   unsigned fs[3];
-  // 1: no shading can be NaN (colour map and light colours finite, alphas >= 0),
-  // so a sample of alpha 0 adds nothing and clamping is saturation.
+  // 1: no shading can be NaN (colour map and light colours finite, alphas >= 0, no
+  // map cell of width 0), so a sample of alpha 0 adds nothing and clamping is
+  // saturation.
   int tame;
   // Pixel window {x0, y0, w, h} the (non-listed) view march covers; the whole
   // image unless a brick's projection is known to lie inside a smaller one
@@ -211,6 +212,16 @@ __host__ __device__ inline float4 field_entry(float lo, float hi, unsigned offse
 // offset (a load in bounds) and NaN, so that no position looks inside it.
 __host__ __device__ inline float4 closing_entry(float lo, unsigned offset) {
   return make_float4(lo, bits_float(offset), NAN, NAN);
+}
+
+// Whether every map cell has a width above 0: the spacing has to exceed what rounding
+// moves two neighbouring vertices, less than 2^-23 of the largest bound and of the
+// extent (at most twice that bound). Far from the coordinate origin a fine map's cells
+// can vanish, and a position in one has no parametric coordinate (0 / 0).
+inline bool map_cells_have_width(const ExactGeo& g) {
+  for (int d = 0; d < 3; ++d)
+    if (!(g.msp[d] > 1e-6f * std::fmax(std::fabs(g.minp[d]), std::fabs(g.maxp[d])))) return false;
+  return true;
 }
 
 // Slots of the light-aligned vertex order with groups of 2^bl x 2^bl columns

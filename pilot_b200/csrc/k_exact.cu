@@ -967,7 +967,8 @@ cudaError_t launch_view_march_f32(const ExactGeo& g, const float* field, const f
   } else if (g.rect && g.n_lights > 1) {
     return cudaErrorInvalidValue;
   } else if (g.use_map && g.n_lights > 1) {
-    return launch_k2<float4, true, float, true>(g, quads, tab, tf, map, out, cnt, occ, st);  // the multi-light extension
+    // the multi-light extension (where a shading may be NaN, alpha 0 does not hide it: no skipping)
+    return launch_k2<float4, true, float, true>(g, quads, tab, tf, map, out, cnt, g.tame ? occ : nullptr, st);
   } else if (g.use_map) {
     return launch_k2<float4, true, float>(g, quads, tab, tf, map, out, cnt, occ, st);
   } else {

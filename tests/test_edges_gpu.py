@@ -40,3 +40,43 @@ def test_opacities_that_are_never_positive(cuda_device, nextra):
         oimg, lit = Oracle(s).view_march(Oracle(s).light_march()[0])
         assert out[1][2][1] == lit
         check(out[1][0], oimg)
+
+
+def far(s, org, sp):
+    """s with its field placed at org with the spacing sp."""
+    at = lambda p: tuple(o + c * (n - 1) * sp for o, c, n in zip(org, p, s.dims))
+    return dataclasses.replace(s, origin=org, brick_spacing=(sp,) * 3, cam_pos=at(s.cam_pos), cam_look=at(s.cam_look),
+                               light=at(s.light) if s.light_kind == 0 else s.light,
+                               sample_distance=s.sample_distance * (s.dims[0] - 1) * sp)
+
+
+@pytest.mark.parametrize("lights", [1, 3])
+@pytest.mark.parametrize("org", [(0.0, 0.0, 0.0), (4.0e3, 0.0, 9.0e3), (5.0e4, 0.0, 0.0)], ids=str)
+def test_maps_finer_than_their_coordinates(cuda_device, org, lights):
+    """Cells of 0.02 in a map 16 times as fine: near the coordinate origin every map cell has
+    a width, 50,000 away most have none, and a sample in such a cell has no shading (not a
+    number, whatever its opacity)."""
+    s = far(dataclasses.replace(scenes.small(45, n=9, image=48, m=4, kind="blobs"), map_m=(128, 128, 128)), org, 0.02)
+    with renderer(s) as r:
+        for i in range(1, lights):
+            r.add_directional_light(LIGHTS[i][1], (0.3, 0.9, 0.5), 0.7)
+        r.set_multi_light(lights > 1)
+        r.set_tuning(empty_skip=False, view_skip=False)
+        img, t = r.render(s.camera())
+        maps = r.get_shadow_map(lights * 129 ** 3)
+        r.set_tuning(empty_skip=True, view_skip=True)
+        again, t2 = r.render(s.camera())
+        assert t2["lit_samples"] == t["lit_samples"]
+        if lights > 1:
+            assert np.array_equal(again, img, equal_nan=True)
+    o = Oracle(s)
+    if lights == 1:
+        oimg, lit = o.view_march(maps.reshape(129, 129, 129))
+    else:
+        lc = np.stack([np.float32(s.light_color) * np.float32(s.light_intensity)]
+                      + [np.float32((0.3, 0.9, 0.5)) * np.float32(0.7)] * (lights - 1))
+        oimg, lit = o.view_march_multi(maps.reshape(lights, -1), lc)
+    assert t["lit_samples"] == lit and np.isnan(oimg).any() == (org[0] > 1e4)
+    nan = np.isnan(oimg)
+    assert np.mean(np.isnan(img) == nan) > 0.999
+    check(np.where(nan, 0, img), np.where(nan, 0, oimg))
