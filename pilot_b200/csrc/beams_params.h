@@ -25,7 +25,7 @@ struct ExactGeo {
   float max_alpha;              // TransmittanceMap.h:515-525
   // Map grid: (M+1)^3 vertices over the field bounds (TransmittanceMap.h:550-563).
   int pd[3];
-  float morig[3], msp[3], minv[3];
+  float morig[3], msp[3], minv[3];  // minv: 1 / msp, or 0 (geo_loop_constants)
   float light_color[3];         // Color * Intensity (LightedVolumeRenderer.cxx:840)
   float extent_mag;             // BoundsMagnitude (beams/Math.h:13-21)
   float sd;                     // view sample distance
@@ -254,7 +254,9 @@ inline void geo_light_order(ExactGeo& g, int kind, const double v[3]) {
     g.bo_shear[k] = ok ? (int)std::lround(65536.0 * e[g.bo_axis[1 + k]] / e[w]) : 0;
 }
 
-// Derives seed, n1f and fs. Coordinates that are not finite in float32 (an origin
+// Derives seed, n1f and fs, and makes minv one that takes every position inside to an
+// entry of the map's cell tables (a spacing below 2^-128 or of 0 has no reciprocal: all
+// positions go to the first cell). Coordinates that are not finite in float32 (an origin
 // past its range) have no inside: their bounds become NaN, which no position
 // passes, so no guess is ever formed from them.
 inline void geo_loop_constants(ExactGeo& g, bool quads) {
@@ -267,6 +269,7 @@ inline void geo_loop_constants(ExactGeo& g, bool quads) {
     g.seed[d] = (std::isfinite(g.invh[d]) && std::isfinite(room)) ? g.invh[d] : 0.f;
     if ((double)room * g.seed[d] >= (double)g.n[d])  // the product of two floats is exact
       g.seed[d] = (float)((g.n[d] - 1) / (double)room);
+    if (!((double)room * g.minv[d] < (double)g.pd[d])) g.minv[d] = 0.f;
   }
   g.n1f = (float)(g.tf_n - 1);
 }

@@ -211,7 +211,6 @@ extern "C" beams_status beams_render_noalloc(const beams_volume* vol, const floa
     }
     g.ntab = off;
   }
-  geo_loop_constants(g, false);
   float ext[3];
   for (int d = 0; d < 3; ++d) ext[d] = (float)(g.bmax[d] - g.bmin[d]);
   g.extent_mag = std::sqrt(ext[0] * ext[0] + ext[1] * ext[1] + ext[2] * ext[2]);
@@ -223,6 +222,7 @@ extern "C" beams_status beams_render_noalloc(const beams_volume* vol, const floa
     g.light_color[d] = light_color[d] * light_intensity;
     g.light[d] = (float)light_pos[d];
   }
+  geo_loop_constants(g, false);
   g.sd = (sample_distance > 0.f) ? sample_distance : g.extent_mag / 200.f;
   if (!(g.extent_mag / g.sd <= 1.0e6f))
     return nf(BEAMS_ERR_INVALID_ARG, "render_noalloc: sample distance below 1e-6 of the volume diagonal");
