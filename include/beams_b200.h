@@ -372,7 +372,7 @@ typedef struct beams_mlp_options {
   int samples_log2;      /* training samples 2^k (default 24) */
   int n_lights;          /* light directions on a Fibonacci sphere (default 32) */
   int epochs;            /* default 4 */
-  int batch;             /* rows per step (default 16384) */
+  int batch;             /* rows per step (default 16384), at most the training set (15/16 of the samples) */
   float lr;              /* Adam learning rate, cosine-decayed (default 2e-3) */
   unsigned seed;
   float fallback_tol;    /* render: |MLP - exact| on the probe set that sends a tile to the exact map (0.01) */

@@ -500,6 +500,9 @@ beams_status beams_mlp_train(beams_renderer* r, const beams_mlp_options* opt, be
   st->nlights = o.n_lights;
 
   const int n = 1 << o.samples_log2;
+  const int holdout = std::min(n / 16, 65536);
+  const int ntrain = n - holdout;
+  const int batch = std::min(o.batch, ntrain);  // a step takes at most the whole training set
   // samples, targets and features in one block, kept for the next training while it is small
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t b_samples = al((size_t)n * sizeof(float4)), b_target = al((size_t)n * sizeof(float));
@@ -548,14 +551,12 @@ beams_status beams_mlp_train(beams_renderer* r, const beams_mlp_options* opt, be
   for (float* p : {st->G, st->m, st->v})
     if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, kParams * sizeof(float), r->stream);
   st->step = 0;
-  beams_status bs = ensure_ws(r, st, std::max(o.batch, std::min(n / 16, 65536)));
+  beams_status bs = ensure_ws(r, st, std::max(batch, holdout));
   if (bs != BEAMS_OK) {
     cudaStreamSynchronize(r->stream);
     release();
     return bs;
   }
-  const int holdout = std::min(n / 16, 65536);
-  const int ntrain = n - holdout;
   // Baselines on the held-out samples: the initial network, no shadow model
   // (T = 1) and the best constant.
   float init_loss = 0.f;
@@ -574,16 +575,16 @@ beams_status beams_mlp_train(beams_renderer* r, const beams_mlp_options* opt, be
     su += (1.0 - t) * (1.0 - t);
   }
   const double mean_t = s1 / holdout;
-  const int steps_per_epoch = std::max(1, ntrain / o.batch);
+  const int steps_per_epoch = std::max(1, ntrain / batch);
   const int total = steps_per_epoch * o.epochs;
   bool timed_out = false;
   for (int ep = 0; ep < o.epochs && e == cudaSuccess && !timed_out; ++ep) {
-    const int rot = (int)(((unsigned)ep * 2654435761u) % (unsigned)std::max(1, ntrain - o.batch));
+    const int rot = (int)(((unsigned)ep * 2654435761u) % (unsigned)std::max(1, ntrain - batch));
     for (int k = 0; k < steps_per_epoch && e == cudaSuccess && !timed_out; ++k) {
-      int off = (rot + k * o.batch) % std::max(1, ntrain - o.batch + 1);
+      int off = (rot + k * batch) % std::max(1, ntrain - batch + 1);
       const float prog = (float)st->step / (float)total;
       const float lr = o.lr * (0.05f + 0.95f * 0.5f * (1.f + std::cos((float)M_PI * prog)));
-      e = mlp_fwd_bwd(st->P, st->G, d_X + (size_t)off * kIn, d_target + off, o.batch, st->ws, r->stream);
+      e = mlp_fwd_bwd(st->P, st->G, d_X + (size_t)off * kIn, d_target + off, batch, st->ws, r->stream);
       if (e == cudaSuccess) e = mlp_adam(st->P, st->G, st->m, st->v, lr, ++st->step, r->stream);
       // a tensor-core wait that gave up ends the training early (checked every 256 steps)
       if (e == cudaSuccess && st->ws.err && (st->step & 255) == 0) {

@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 
 from oracle.oracle import Oracle
+from pilot_b200 import beams as B
 from pilot_b200 import scenes
 from test_marches_gpu import LIGHTS, frame, renderer, same, sparse
 from test_rectilinear_gpu import check
@@ -80,3 +81,18 @@ def test_maps_finer_than_their_coordinates(cuda_device, org, lights):
     nan = np.isnan(oimg)
     assert np.mean(np.isnan(img) == nan) > 0.999
     check(np.where(nan, 0, img), np.where(nan, 0, oimg))
+
+
+@pytest.mark.parametrize("log2", [10, 13])
+def test_batches_larger_than_the_training_set(cuda_device, log2):
+    """A step takes at most the whole set: 15/16 of the samples, the rest is held out. Bar: as
+    a batch of just that size, whatever an earlier, larger training left behind (the sums'
+    order varies, which four steps of 1e-3 keep below 1% of the error)."""
+    s = scenes.small(46, n=24, image=16, m=8)
+    size = (1 << log2) - (1 << (log2 - 4))
+    with renderer(s) as r:
+        r.mlp_train(B.mlp_options(samples_log2=16, epochs=1, batch=16384, lr=1e-3))
+        reps = [r.mlp_train(B.mlp_options(samples_log2=log2, epochs=4, batch=b, lr=1e-3)) for b in (size, size + 1, 1 << 20)]
+    for rep in reps:
+        assert rep["steps"] == 4 and rep["initial_rmse"] == pytest.approx(reps[0]["initial_rmse"], rel=1e-5)
+        assert abs(rep["holdout_rmse"] - reps[0]["holdout_rmse"]) <= 0.01 * reps[0]["holdout_rmse"]
