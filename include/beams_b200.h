@@ -395,7 +395,10 @@ typedef struct beams_mlp_report {
   int samples;
 } beams_mlp_report;
 
-/* Trains the network on the current volume and colour map. */
+/* Trains the network on the current volume and colour map. The training set's device
+ * memory (up to 256 MB: 2^20 samples) stays with the renderer for its next training; it
+ * is given back when an allocation of the renderer's own buffers fails, and by
+ * beams_destroy. A larger set is given back before the call returns. */
 beams_status beams_mlp_train(beams_renderer* r, const beams_mlp_options* opts, beams_mlp_report* report);
 int beams_mlp_param_count(void);
 beams_status beams_mlp_get_params(beams_renderer* r, float* dst, int n);

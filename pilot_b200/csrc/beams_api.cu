@@ -48,6 +48,8 @@ beams_status cuda_fail(beams_renderer* r, cudaError_t e, const char* what) {
 // n-th following buffer allocation reports out-of-memory instead of allocating.
 static std::atomic<int> g_fail_alloc_in{0};
 
+bool mlp_release_training_set(beams_renderer* r);
+
 beams_status ensure_buffer(beams_renderer* r, void** buf, size_t* cap, size_t bytes, const char* what) {
   if (*cap >= bytes && *buf) return BEAMS_OK;
   if (*buf) {
@@ -58,10 +60,16 @@ beams_status ensure_buffer(beams_renderer* r, void** buf, size_t* cap, size_t by
   int pending = g_fail_alloc_in.load();
   while (pending > 0 && !g_fail_alloc_in.compare_exchange_weak(pending, pending - 1)) {
   }
-  if (pending == 1) return fail(r, BEAMS_ERR_OOM, std::string(what) + ": out of device memory (injected)");
-  cudaError_t e = cudaMalloc(buf, bytes);
+  bool injected = pending == 1;
+  cudaError_t e = injected ? cudaErrorMemoryAllocation : cudaMalloc(buf, bytes);
+  if (e == cudaErrorMemoryAllocation && r && mlp_release_training_set(r)) {
+    cudaGetLastError();
+    injected = false;
+    e = cudaMalloc(buf, bytes);
+  }
   if (e != cudaSuccess) {
     *buf = nullptr;
+    if (injected) return fail(r, BEAMS_ERR_OOM, std::string(what) + ": out of device memory (injected)");
     return cuda_fail(r, e, what);
   }
   *cap = bytes;

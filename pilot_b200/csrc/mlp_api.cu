@@ -26,6 +26,8 @@ beams_status check_ready(beams_renderer* r);
 // A training set up to this size (2^20 samples) stays allocated for the next
 // training on the renderer: allocating and freeing it took 1 to 3 ms of a training
 // whose kernels run 2 ms. A larger one is freed, as its training takes far longer.
+// The kept one goes when the renderer's own buffers need the memory
+// (mlp_release_training_set) or with the renderer.
 constexpr size_t kKeepTrainBytes = (size_t)256 << 20;
 
 // Device state of the learned form (owned by the renderer).
@@ -72,6 +74,17 @@ struct MlpState {
 MlpState* mlp_state(beams_renderer* r) {
   if (!r->mlp) r->mlp = new MlpState();
   return r->mlp;
+}
+
+// Gives back the training set kept for the next training (kKeepTrainBytes), for a
+// renderer that is out of device memory; false when there is none.
+bool mlp_release_training_set(beams_renderer* r) {
+  MlpState* st = r->mlp;
+  if (!st || !st->train_mem) return false;
+  cudaFree(st->train_mem);  // waits for what reads it
+  st->train_mem = nullptr;
+  st->train_bytes = 0;
+  return true;
 }
 void mlp_release(beams_renderer* r) {
   delete r->mlp;

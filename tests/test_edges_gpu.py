@@ -96,3 +96,28 @@ def test_batches_larger_than_the_training_set(cuda_device, log2):
     for rep in reps:
         assert rep["steps"] == 4 and rep["initial_rmse"] == pytest.approx(reps[0]["initial_rmse"], rel=1e-5)
         assert abs(rep["holdout_rmse"] - reps[0]["holdout_rmse"]) <= 0.01 * reps[0]["holdout_rmse"]
+
+
+def test_training_set_given_back_when_memory_runs_out(cuda_device):
+    """The set kept for the next training goes when a buffer of the renderer cannot be had; with
+    nothing kept the call fails as before, and the next training allocates its set again."""
+    s = scenes.small(47, n=24, image=16, m=8)
+    opts = B.mlp_options(samples_log2=12, epochs=1, batch=1024, lr=1e-3)
+    with renderer(s) as r:
+        r.render(s.camera())
+        r.mlp_train(opts)
+        for m in (20, 30):
+            r.set_shadow_map_size(m)  # a larger map buffer
+            B.lib().beams_test_fail_allocation(1)
+            try:
+                if m == 20:
+                    r.render(s.camera())
+                else:
+                    with pytest.raises(B.BeamsError, match="OOM"):
+                        r.render(s.camera())
+            finally:
+                B.lib().beams_test_fail_allocation(0)
+        img, _ = r.render(s.camera())
+        assert r.mlp_train(opts)["steps"] == 3
+        again, _ = r.render(s.camera())
+    assert np.array_equal(img, again)
