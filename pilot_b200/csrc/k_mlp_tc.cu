@@ -182,11 +182,21 @@ __device__ __forceinline__ void red_add4(float* g, const float* v) {
                : "memory");
 }
 
+// A load that stays behind the volatile instructions before it (wait_for_preceding).
+__device__ __forceinline__ float ld_ordinary(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+
 // Stages the four weight matrices as bfloat16 B operands (W_l^T: N = 64
 // outputs as rows, chunked over the inputs) and the biases, bf16(w5), b5. A
 // thread takes eight inputs of one output at a time: eight loads in flight
 // (coalesced over the outputs) and one 16-byte store without bank conflicts.
-__device__ void stage_weights(const float* __restrict__ P, unsigned char* W, float* aux) {
+// The loads are ordinary ones, not the read-only path's, which wants memory that
+// nobody writes while the kernel runs: the training kernel starts while the
+// optimiser still writes P, and reads it after wait_for_preceding.
+__device__ void stage_weights(const float* P, unsigned char* W, float* aux) {
   constexpr int u1 = kIn / 8 * kHid, uh = kHid / 8 * kHid;  // such pieces of the first and of a later matrix
 #pragma unroll 2
   for (int i = threadIdx.x; i < u1 + 3 * uh; i += blockDim.x) {
@@ -195,7 +205,7 @@ __device__ void stage_weights(const float* __restrict__ P, unsigned char* W, flo
     const float* w = P + (l == 0 ? oW1 : (l == 1 ? oW2 : (l == 2 ? oW3 : oW4))) + k * kHid + n;
     float x[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = __ldg(w + j * kHid);
+    for (int j = 0; j < 8; ++j) x[j] = ld_ordinary(w + j * kHid);
     uint32_t b[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -206,9 +216,9 @@ __device__ void stage_weights(const float* __restrict__ P, unsigned char* W, flo
         make_uint4(b[0], b[1], b[2], b[3]);
   }
   const int oB[4] = {oB1, oB2, oB3, oB4};
-  for (int i = threadIdx.x; i < 4 * kHid; i += blockDim.x) aux[i] = P[oB[i / kHid] + (i % kHid)];
-  for (int i = threadIdx.x; i < kHid; i += blockDim.x) aux[4 * kHid + i] = bf16r(P[oW5 + i]);
-  if (threadIdx.x == 0) aux[5 * kHid] = P[oB5];
+  for (int i = threadIdx.x; i < 4 * kHid; i += blockDim.x) aux[i] = ld_ordinary(P + oB[i / kHid] + (i % kHid));
+  for (int i = threadIdx.x; i < kHid; i += blockDim.x) aux[4 * kHid + i] = bf16r(ld_ordinary(P + oW5 + i));
+  if (threadIdx.x == 0) aux[5 * kHid] = ld_ordinary(P + oB5);
 }
 
 __device__ __forceinline__ uint32_t w_addr(uint32_t wbase, int l) {
@@ -451,7 +461,7 @@ static_assert(kTrOffX + 16 * kTile * 16 <= kTrOffDY, "wgrad A read of X stays in
 static_assert(kTrOffH + 2 * kHBytes + 16 * kTile * 16 <= kTrOffDY, "wgrad A read of H2 stays inside H3");
 
 __global__ void __launch_bounds__(kThreads, 1) k_mlp_train_tc(const __grid_constant__ CUtensorMap xmap, int row0,
-                                                              int n, const float* __restrict__ P,
+                                                              int n, const float* P,
                                                               const float* __restrict__ target, float scale,
                                                               float* __restrict__ G, float* __restrict__ T,
                                                               float* __restrict__ loss, unsigned* __restrict__ err) {
