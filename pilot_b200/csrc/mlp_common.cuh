@@ -102,7 +102,9 @@ cudaError_t launch_early(void (*kernel)(Params...), int grid, int threads, size_
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // returned here, not by the next call that asks
+  return e;
 }
 
 // Position p (world space) relative to the volume.

@@ -8,12 +8,16 @@ sums to the gradient and the order in which they arrive changes nothing. Bar: th
 bit for bit; a gradient of weights one step old gives others.
 """
 import ctypes as C
+import subprocess
+from pathlib import Path
 
 import pytest
 
 from pilot_b200 import beams as B
+from pilot_b200.build import NVCC
 
 pytestmark = pytest.mark.gpu
+CSRC = Path(B.__file__).parent / "csrc"
 KIN, PARAMS, STEPS = 112, 19777, 24
 
 
@@ -61,3 +65,25 @@ def test_overlapping_steps_read_the_finished_ones(cuda_device, rows):
     assert not torch.equal(train(wait=True, stale=True), apart)
     for _ in range(8):
         assert torch.equal(train(wait=False), apart)
+
+
+SRC = r"""
+#include <cstdio>
+#include "mlp_common.cuh"
+__global__ void k_nothing(int) {}
+int main() {
+  const cudaError_t e = beams::mlp::launch_early(k_nothing, 1, 2048, 0, nullptr, 1);  // 1024 threads at most
+  const cudaError_t left = cudaGetLastError();
+  std::printf("%d %d", (int)(e == cudaErrorInvalidConfiguration || e == cudaErrorInvalidValue), (int)left);
+  return 0;
+}
+"""
+
+
+def test_a_refused_launch_leaves_no_error_behind(cuda_device, tmp_path):
+    """The launch's own status reports it; the next call that asks for the last error has none."""
+    (tmp_path / "t.cu").write_text(SRC)
+    subprocess.run([NVCC, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", str(CSRC),
+                    str(tmp_path / "t.cu"), "-o", str(tmp_path / "t")], check=True)
+    p = subprocess.run([str(tmp_path / "t")], capture_output=True, text=True)
+    assert p.stdout == "1 0"
