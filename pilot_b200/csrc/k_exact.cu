@@ -269,7 +269,9 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<LIST>()) k_light_ma
       }
     }
     if constexpr (!SPLIT) {
-      if (!vertex(((unsigned)tile << 5) + lane, id, V)) continue;
+      const bool active = vertex(((unsigned)tile << 5) + lane, id, V);
+      const unsigned lanes = __ballot_sync(0xffffffffu, active);
+      if (!active) continue;
       ++built;
       light_origin(g, V, L);
       const LightRay ray = light_ray(g, V, L, dir);
@@ -278,7 +280,7 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<LIST>()) k_light_ma
         light_march_rect<QuadT, PREC>(g, quads, s_tab, PREC ? s_tau : s_a, ray, acc, ns);
       } else {
         // the lanes leave the untested steps together
-        const int sure = SKIP ? ray.sure : __reduce_min_sync(__activemask(), ray.sure);
+        const int sure = SKIP ? ray.sure : __reduce_min_sync(lanes, ray.sure);
         light_march<QuadT, PREC, SKIP>(g, F, ray, sure, acc, ns);
       }
       acc.store(map, id);
