@@ -10,6 +10,7 @@ import dataclasses
 import numpy as np
 import pytest
 
+from oracle import mlp_oracle as M
 from oracle.oracle import Oracle
 from pilot_b200 import beams as B
 from pilot_b200 import scenes
@@ -121,3 +122,25 @@ def test_training_set_given_back_when_memory_runs_out(cuda_device):
         assert r.mlp_train(opts)["steps"] == 3
         again, _ = r.render(s.camera())
     assert np.array_equal(img, again)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_hidden_units_that_are_not_numbers_are_off(cuda_device, value):
+    """The march's network clamps a sum that is not a number to 0. Bar: the image of the network
+    whose units are switched off by their biases, bit for bit."""
+    s = scenes.small(49, n=24, image=24, m=8)
+    P = np.random.default_rng(49).normal(0, 0.08, M.N_PARAMS).astype(np.float32)
+
+    off, odd = P.copy(), P.copy()
+    for layer, unit in (("1", 3), ("2", 9), ("3", 17), ("4", 40)):
+        w, b = M.OFF["W" + layer][0], M.OFF["B" + layer][0]
+        off[b + unit] = -1e30
+        # weights of the value and of its opposite (two infinities that meet sum to NaN), and the bias
+        odd[w + unit], odd[w + 64 + unit], odd[b + unit] = value, -value, np.nan
+    out = []
+    with renderer(s) as r:
+        for p in (off, odd):
+            r.mlp_set_params(p)
+            r.set_form(B.FORM_MLP, B.mlp_options(knot=1, probe_fraction=0.0))
+            out.append(r.render(s.camera())[0])
+    assert np.isfinite(out[0]).all() and np.array_equal(out[1], out[0])
