@@ -218,29 +218,6 @@ __device__ __forceinline__ int trunc_small(float x) {
 // width w in two operations (see field_entry); NaN when two terms do not suffice.
 __device__ __forceinline__ float div_field(float x, const float4& e) { return fmaf(x, e.z, x * e.w); }
 
-// Light-march cell search: RectilinearMeshOracle's binary search
-// (RectilinearMeshOracle.h:154-176) returns the smallest cell c with
-// val <= coord(c+1). The seed (val - org) / h is that cell for counting
-// coordinates except within an ulp of a cell face, where the bounded walk
-// below settles it. At c == 0 a point on the lower face stays in cell 0 and
-// inside the volume val <= coord(cmax+1), so one test per side suffices.
-// The bounded walk that settles a seeded light-march cell guess (the smallest
-// c with val <= coord(c+1), RectilinearMeshOracle.h:154-176), for the rare
-// sample within an ulp of a cell face; kept out of line (noinline) so that the
-// march's common path carries none of its code.
-static __device__ __noinline__ int walk_cell_bsearch(const float4* T, int cmax, float val, int c) {
-  c = min(c, cmax);
-  while (c > 0 && val <= T[c].x) --c;
-  while (c < cmax && val > T[c + 1].x) ++c;
-  return c;
-}
-static __device__ __noinline__ int3 walk_cells_bsearch(const float4* T0, const float4* T1, const float4* T2, int m0,
-                                                       int m1, int m2, float v0, float v1, float v2, int c0, int c1,
-                                                       int c2) {
-  return make_int3(walk_cell_bsearch(T0, m0, v0, c0), walk_cell_bsearch(T1, m1, v1, c1),
-                   walk_cell_bsearch(T2, m2, v2, c2));
-}
-
 // Searches for explicit (non-uniform) rectilinear coordinates over the cell table.
 // near (ExactGeo::rect 1): the cell that a uniform spacing would give is never more
 // than kRectNear cells off, and the search walks from it; else it halves the

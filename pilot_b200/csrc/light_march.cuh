@@ -120,13 +120,35 @@ struct LightField {
       : q(quads), cells(g, s_tab), val((unsigned)__cvta_generic_to_shared(vals) - (kGuessBias << 2)), occ(occupancy) {}
 };
 
+// Settles a guess on one axis: the smallest cell c with s <= coord(c + 1)
+// (RectilinearMeshOracle.h:154-176) by steps from the guessed entry's address a. p: the
+// parametric coordinate in the guessed cell, which tells whether there is anything to do,
+// then in the found one. Returns the found cell's offset.
+__device__ __forceinline__ unsigned settle_light_cell(unsigned tab, int last_cell, float s, unsigned a, float& p) {
+  float4 e = ld_shared4(a);
+  if (!(p > 0.f && p < 1.f)) {
+    const unsigned first = tab + (kGuessBias << 4), last = first + ((unsigned)last_cell << 4);
+    if (a > last) e = ld_shared4(a = last);
+    if (s <= e.x) {
+      while (a > first && s <= e.x) e = ld_shared4(a -= 16u);
+    } else {
+      for (float4 up; a < last && s > (up = ld_shared4(a + 16u)).x; a += 16u) e = up;
+    }
+    p = div_field(s - e.x, e);
+    if (p != p) p = (s - e.x) / (ld_shared1(a + 16u) - e.x);
+  }
+  return float_bits(e.y);
+}
 // Corner values and parametric coordinates of the cell of s, whose guess is b. A
 // guess is the found cell unless s lies within an ulp of a cell face. The
 // parametric coordinates tell: s > lo exactly when its coordinate is > 0, and a
 // coordinate < 1 implies s < hi, so one minimum and one maximum test the three
-// axes (a NaN quotient fails); the rest takes the walk, out of line, and IEEE
-// divisions. The loads go out before the test; a wrong guess loads some cell in
-// vain.
+// axes (a NaN quotient fails); the rest settles its axes. The loads go out before
+// the test; a wrong guess loads some cell in vain. Settling is inline and does no more
+// than the face asks for: along an axis on a map whose vertices lie on faces, and far
+// from the coordinate origin, where rounding puts positions on faces, most samples do it
+// (the 129^3-vertex map of a 129^3 field along z without skipping: 0.58 ms, with the
+// walks called and IEEE divisions 0.90).
 template <typename QuadT>
 __device__ __forceinline__ void sample_fetch(const ExactGeo& g, const LightField<QuadT>& F, const float s[3],
                                              unsigned b0, unsigned b1, unsigned b2, float v[8], float p[3]) {
@@ -140,13 +162,11 @@ __device__ __forceinline__ void sample_fetch(const ExactGeo& g, const LightField
     p[2] = div_field(s[2] - e2.x, e2);
   }
   if (!(min3(p[0], p[1], p[2]) > 0.f && max3(p[0], p[1], p[2]) < 1.f)) {
-    const int3 c = walk_cells_bsearch(F.cells.T[0], F.cells.T[1], F.cells.T[2], g.n[0] - 2, g.n[1] - 2, g.n[2] - 2, s[0], s[1], s[2],
-                                      (int)(b0 - kGuessBias), (int)(b1 - kGuessBias), (int)(b2 - kGuessBias));
-    const float4 *e0 = F.cells.T[0] + c.x, *e1 = F.cells.T[1] + c.y, *e2 = F.cells.T[2] + c.z;
-    QuadLoad<QuadT>::cell(F.q, float_bits(e0->y) + float_bits(e1->y) + float_bits(e2->y), g.fs[1], g.fs[2], v);
-    p[0] = (s[0] - e0->x) / (e0[1].x - e0->x);
-    p[1] = (s[1] - e1->x) / (e1[1].x - e1->x);
-    p[2] = (s[2] - e2->x) / (e2[1].x - e2->x);
+    const unsigned b[3] = {b0, b1, b2};
+    unsigned off = 0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) off += settle_light_cell(F.cells.tab[d], g.n[d] - 2, s[d], F.cells.tab[d] + (b[d] << 4), p[d]);
+    QuadLoad<QuadT>::cell(F.q, off, g.fs[1], g.fs[2], v);
   }
 }
 template <typename QuadT>

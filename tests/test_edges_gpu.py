@@ -14,7 +14,7 @@ from oracle import mlp_oracle as M
 from oracle.oracle import Oracle
 from pilot_b200 import beams as B
 from pilot_b200 import scenes
-from test_marches_gpu import LIGHTS, frame, renderer, same, sparse
+from test_marches_gpu import DTYPES, LIGHTS, frame, oracle, renderer, same, sparse
 from test_rectilinear_gpu import check
 
 pytestmark = pytest.mark.gpu
@@ -144,3 +144,22 @@ def test_hidden_units_that_are_not_numbers_are_off(cuda_device, value):
             r.set_form(B.FORM_MLP, B.mlp_options(knot=1, probe_fraction=0.0))
             out.append(r.render(s.camera())[0])
     assert np.isfinite(out[0]).all() and np.array_equal(out[1], out[0])
+
+
+@pytest.mark.parametrize("name,dt", DTYPES[:2], ids=lambda d: str(d))
+@pytest.mark.parametrize("org", [(3.0e5, 0.0, 1.0e3), (4.0e6, 2.5e6, 0.0), (0.0, 3.0e7, 5.0e6)], ids=str)
+def test_positions_rounded_onto_faces(cuda_device, org, name, dt):
+    """Cells of width 1 far from the coordinate origin: positions are multiples of 1/32, of 1/4
+    and 1/2, and of 2 (where cells have width 0 or 2), so samples lie on faces and edges."""
+    s = far(dataclasses.replace(scenes.small(50, n=21, image=40, m=8, kind="noise"), map_m=(9, 11, 8)), org, 1.0)
+    o = oracle(s, name)
+    om, _ = o.light_march()
+    oimg, lit = o.view_march(om)
+    with renderer(s, dt) as r:
+        for skip in (False, True):
+            r.set_tuning(empty_skip=skip, view_skip=skip)
+            img, m, n = frame(r, s)
+            assert np.array_equal(m, om.ravel()) and n[1] == lit, skip
+            nan = np.isnan(oimg)
+            assert np.array_equal(np.isnan(img), nan)
+            check(np.where(nan, 0, img), np.where(nan, 0, oimg))
