@@ -83,6 +83,7 @@ struct ExactGeo {
   // quads' {1, n0 - 1, (n0 - 1)(n1 - 1)}, or the plain field's (set by
   // geo_loop_constants); cell (x, y, z) is entry fs . (x, y, z).
   unsigned fs[3];
+  double ifs[2];  // 1 / fs[1], 1 / fs[2]
   // 1: no shading can be NaN (colour map and light colours finite, alphas >= 0, no
   // map cell of width 0), so a sample of alpha 0 adds nothing and clamping is
   // saturation.
@@ -263,6 +264,7 @@ inline void geo_loop_constants(ExactGeo& g, bool quads) {
   g.fs[0] = 1u;
   g.fs[1] = (unsigned)(quads ? g.n[0] - 1 : g.n[0]);
   g.fs[2] = g.fs[1] * (unsigned)(quads ? g.n[1] - 1 : g.n[1]);
+  for (int k = 0; k < 2; ++k) g.ifs[k] = 1.0 / (double)g.fs[k + 1];
   for (int d = 0; d < 3; ++d) {
     const float room = g.maxp[d] - g.org[d];
     if (!(std::isfinite(g.org[d]) && std::isfinite(room))) g.minp[d] = g.maxp[d] = NAN;
