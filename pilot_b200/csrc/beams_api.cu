@@ -687,7 +687,14 @@ beams_status render_bricks(beams_renderer* r, const beams_camera* cam, float4* o
   e = cudaMemsetAsync(r->d_brick_cnt, 0, nb * sizeof(Counters), r->stream);
   if (e != cudaSuccess) return cuda_fail(r, e, "clearing brick counters");
   auto lane = [&](int b) { return r->brick_lane[b % beams_renderer::kBrickLanes]; };
-  for (ExactGeo& g : G) g.light_marches = brick_lanes(r);
+  // a stitched map is NaN where its prefix is: along a ray without a direction, or from a
+  // map with cells of no width
+  bool widths = true;
+  for (const ExactGeo& g : G) widths = widths && map_cells_have_width(g);
+  for (ExactGeo& g : G) {
+    g.light_marches = brick_lanes(r);
+    g.tame = (g.tame && widths && light_rays_have_direction(g)) ? 1 : 0;
+  }
   const bool lazy = r->lazy_map && r->use_map;
   auto lane_fail = [&](cudaError_t err, const char* what) {
     brick_lanes_join(r);

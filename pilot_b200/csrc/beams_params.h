@@ -225,6 +225,22 @@ inline bool map_cells_have_width(const ExactGeo& g) {
   return true;
 }
 
+// Whether the rays from the light to the map's vertices all have a direction: of one to a
+// vertex at the light it is 0 / 0, and squares of very short or long ones under- or
+// overflow. (A whole volume's map does not notice, its march takes no sample then; a
+// brick's cross-brick prefix is read along the direction.)
+inline bool light_rays_have_direction(const ExactGeo& g) {
+  float apart = g.light_kind == 0 ? 0.f : g.dir_dist, far = apart, B = 0.f;
+  for (int d = 0; d < 3; ++d) {
+    B = std::fmax(B, std::fmax(std::fabs(g.minp[d]), std::fabs(g.maxp[d])));
+    if (g.light_kind != 0) continue;
+    const float below = g.minp[d] - g.light[d], above = g.light[d] - g.maxp[d];
+    apart = std::fmax(apart, std::fmax(below, above));
+    far = std::fmax(far, std::fmax(std::fabs(below), std::fabs(above)));
+  }
+  return apart > 1e-6f * B && apart > 1e-15f && far < 1e15f;
+}
+
 // Slots of the light-aligned vertex order with groups of 2^bl x 2^bl columns
 // (light_slot_vertex): every vertex once, plus the padding columns of the last
 // groups.

@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 from oracle import mlp_oracle as M
-from oracle.oracle import Oracle
+from oracle.oracle import Oracle, render_bricks
 from pilot_b200 import beams as B
 from pilot_b200 import scenes
 from test_marches_gpu import DTYPES, LIGHTS, frame, oracle, renderer, same, sparse
@@ -163,3 +163,23 @@ def test_positions_rounded_onto_faces(cuda_device, org, name, dt):
             nan = np.isnan(oimg)
             assert np.array_equal(np.isnan(img), nan)
             check(np.where(nan, 0, img), np.where(nan, 0, oimg))
+
+
+@pytest.mark.parametrize("light", [(0, (0.5, 0.5, 0.5)), (0, (0.0, 0.5, 1.0)), (0, (1.0, 0.25, 0.5)), (0, (2.0, 0.5, 0.5)),
+                                   (0, (1e25, 0.0, 0.0)), (1, (0.3, -0.8, 0.1))], ids=str)
+def test_bricks_lit_from_one_of_their_vertices(cuda_device, light):
+    """The ray to a vertex at the light has no direction and its stitched value is not a number, as
+    are the shadings that read it, whatever the samples' opacity."""
+    s = dataclasses.replace(scenes.small(51, n=33, image=40, m=8, kind="blobs"), light_kind=light[0], light=light[1])
+    bricks = scenes.split_bricks(s, (2, 2, 2))
+    oimg, _, _, maps, lit = render_bricks(bricks)
+    with B.Renderer(0) as r:
+        bricks[0].configure(r)
+        r.set_bricks([(b.field_numpy(), b.origin, b.spacing, b.value_range) for b in bricks])
+        img, t = r.render(s.camera())
+        assert t["lit_samples"] == lit
+        for b in range(len(bricks)):
+            assert np.array_equal(r.get_brick_map(b, 1, 729), np.ravel(maps[b]), equal_nan=True), b
+    nan = np.isnan(oimg)
+    assert np.array_equal(np.isnan(img), nan)
+    check(np.where(nan, 0, img), np.where(nan, 0, oimg))
