@@ -354,8 +354,11 @@ beams_status prepare_layouts(beams_renderer* r, const ExactGeo& g, int& launches
       // explicit coordinates: the field axes' entries
       std::vector<float4> fe((size_t)g.max_off[0]);
       for (int d = 0; d < 3; ++d) {
-        for (int c = 0; c + 1 < g.n[d]; ++c)
-          fe[(size_t)g.ax_off[d] + c] = field_entry(r->coords[d][c], r->coords[d][c + 1], (unsigned)c * g.fs[d]);
+        for (int c = 0; c + 1 < g.n[d]; ++c) {
+          float4& f = fe[(size_t)g.ax_off[d] + c];
+          f = field_entry(r->coords[d][c], r->coords[d][c + 1], 0u);
+          f.y = r->coords[d][c + 1];  // their searches test the upper coordinate
+        }
         fe[(size_t)g.ax_off[d] + g.n[d] - 1] =
             closing_entry(r->coords[d].back(), (unsigned)(g.n[d] - 2) * g.fs[d]);
       }

@@ -72,7 +72,8 @@ struct ExactGeo {
   // axes' cell tables hold the given coordinates and cells are found by
   // search instead of from the uniform spacing; org/h/invh then only describe
   // the average spacing. 0: coord(d, i) = org[d] + h[d] * float(i); 1: no cell is
-  // more than kRectNear from where the average spacing puts it; 2: any.
+  // more than kRectNear from where the average spacing puts it; 2: any. The field
+  // axes' table entries then are {lo, hi, rh, rl} (no offset).
   int rect;
   // The light march's cell guess scale per field axis: 1 / h, lowered where
   // floor((maxp - org) * seed) would exceed n - 1, so that a guess always indexes

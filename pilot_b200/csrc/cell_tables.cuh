@@ -65,6 +65,36 @@ __device__ __forceinline__ int macro_distance(const ExactGeo& g, const unsigned 
                                                                          (kGuessBias >> kMacroLog2) * (1u + ox + oz)))));
 }
 
+// The cell of s among explicit (non-uniform) coordinates, whose entries {lo, hi, rh, rl} lie
+// at the shared addresses first to last, by halves: the light march's
+// (RectilinearMeshOracle.h:154-176, the smallest c with s <= coord(c + 1)) or, VIEW, the view
+// march's (RectilinearLocator::LocateCell, LightedVolumeRenderer.cxx:119-165, the c with
+// coord(c) <= s < coord(c + 1)). Both are the last cell that s is past the start of.
+template <bool VIEW>
+__device__ __forceinline__ unsigned halve_cells_rect(unsigned first, unsigned last, float s) {
+  unsigned lo = first, hi = last;
+  while (lo < hi) {
+    const unsigned mid = lo + (((hi - lo + 16u) >> 5) << 4);
+    const float start = ld_shared1(mid);
+    if (VIEW ? s >= start : s > start) lo = mid;
+    else hi = mid - 16u;
+  }
+  return lo;
+}
+
+// The same from the cell at a, whose entry is e: a few cells' walk, then by halves.
+constexpr int kRectSteps = 3;
+template <bool VIEW>
+__device__ __forceinline__ unsigned find_cell_rect(unsigned first, unsigned last, unsigned a, float s,
+                                                   float4& e) {
+  int steps = kRectSteps;
+  const auto past = [&](float lo) { return VIEW ? s >= lo : s > lo; };
+  for (; a > first && steps > 0 && !past(e.x); --steps) e = ld_shared4(a -= 16u);
+  for (; a < last && steps > 0 && past(e.y); --steps) e = ld_shared4(a += 16u);
+  if ((a > first && !past(e.x)) || (a < last && past(e.y))) e = ld_shared4(a = halve_cells_rect<VIEW>(first, last, s));
+  return a;
+}
+
 // The view march's cell location on a uniform grid when a sample leaves its cell
 // (RectilinearLocator::LocateCell, LightedVolumeRenderer.cxx:119-165: the unique
 // c with coord(c) <= p < coord(c+1)), from the guesses b: sets the cell's lower

@@ -218,54 +218,6 @@ __device__ __forceinline__ int trunc_small(float x) {
 // width w in two operations (see field_entry); NaN when two terms do not suffice.
 __device__ __forceinline__ float div_field(float x, const float4& e) { return fmaf(x, e.z, x * e.w); }
 
-// Searches for explicit (non-uniform) rectilinear coordinates over the cell table.
-// near (ExactGeo::rect 1): the cell that a uniform spacing would give is never more
-// than kRectNear cells off, and the search walks from it; else it halves the
-// axis. A 160^3 field whose spacing varies by 40% around its mean builds a 97^3
-// map in 0.34 ms walking and 0.53 ms halving; with coordinates i^1.7 walking takes
-// 0.85 ms, halving 0.53 ms.
-// The light march's (RectilinearMeshOracle.h:154-176: the smallest c with
-// val <= coord(c+1)): the walk from c, whose entry is e, and the halving.
-__device__ __forceinline__ void walk_cell_rect(const float4* T, int cmax, float val, int& c, float4& e) {
-  if (val <= e.x) {
-    while (c > 0 && val <= e.x) e = T[--c];
-  } else if (val > T[c + 1].x) {
-    while (c < cmax && val > T[c + 1].x) ++c;
-    e = T[c];
-  }
-}
-__device__ __forceinline__ int find_cell_bsearch_rect(const float4* T, int cmax, float val, float4& e) {
-  int lo = 0, hi = cmax;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (val <= T[mid + 1].x) hi = mid;
-    else lo = mid + 1;
-  }
-  e = T[lo];
-  return lo;
-}
-// The view march's (the c with coord(c) <= p < coord(c+1) that
-// RectilinearLocator::LocateCell walks to, LightedVolumeRenderer.cxx:119-165).
-__device__ __forceinline__ int find_cell_walk_rect(const float4* T, int cmax, float org, float invh, bool near, float p,
-                                                   float4& e) {
-  int lo;
-  if (near) {
-    lo = trunc_small(fminf(fmaxf((p - org) * invh, 0.f), (float)cmax));
-    while (lo > 0 && p < T[lo].x) --lo;
-    while (lo < cmax && p >= T[lo + 1].x) ++lo;
-  } else {
-    int hi = cmax;  // largest c with coord(c) <= p
-    lo = 0;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (T[mid].x <= p) lo = mid;
-      else hi = mid - 1;
-    }
-  }
-  e = T[lo];
-  return lo;
-}
-
 // The view march's walk (the unique c with coord(c) <= p < coord(c+1)) that
 // settles seeded guesses off by a face, out of line like walk_cells_bsearch.
 static __device__ __noinline__ int walk_cell_view(const float4* T, int cmax, float p, int c) {

@@ -45,11 +45,11 @@ __device__ __forceinline__ void load_tables(float4* s_tab, const float4* __restr
 // Blocks per SM: 6 (40 registers), where the loads' latency is covered best (the
 // 257^3-vertex map of a 512^3 noise field, mean of eight light directions: 2.39 ms
 // against 2.63 ms at 4; skipping, 256^3 noise 0.40 against 0.44 ms, 384^3
-// bfloat16 0.99 against 1.04 ms; rectilinear, 160^3 0.34 against 0.37 ms); the listed
-// ones, with both ways to march a ray, spill there and keep 4.
-template <bool LIST>
+// bfloat16 0.99 against 1.04 ms); the listed
+// ones, with both ways to march a ray, and the rectilinear spill there and keep 4.
+template <bool LIST, int RECT>
 constexpr int k1_blocks_per_sm() {
-  return LIST ? 4 : 6;
+  return LIST || RECT ? 4 : 6;
 }
 
 // A masked map build (the exact form's lazy map, the learned form's fallback,
@@ -187,8 +187,8 @@ __host__ __device__ inline unsigned split_rays(const ExactGeo& g) {
 // LIST: the vertices come from a work list (k_list_marked_vertices) instead of
 // the whole map's vertex order. SPLIT: kSplit lanes a ray (a list decides by its
 // own length).
-template <typename QuadT, bool STITCH, bool PREC, bool SKIP, bool RECT = false, bool LIST = false, bool SPLIT = false>
-__global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<LIST>()) k_light_march(const ExactGeo g, const QuadT* __restrict__ quads,
+template <typename QuadT, bool STITCH, bool PREC, bool SKIP, int RECT = 0, bool LIST = false, bool SPLIT = false>
+__global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<LIST, RECT>()) k_light_march(const ExactGeo g, const QuadT* __restrict__ quads,
                                                           const float4* __restrict__ tab,
                                                           const float4* __restrict__ tf,
                                                           const float* __restrict__ tau,
@@ -276,8 +276,8 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<LIST>()) k_light_ma
       light_origin(g, V, L);
       const LightRay ray = light_ray(g, V, L, dir);
       acc.init(STITCH ? stitch_prefix(refs, nrefs, self, L, V, dir) : 0.f);
-      if constexpr (RECT) {
-        light_march_rect<QuadT, PREC>(g, quads, s_tab, PREC ? s_tau : s_a, ray, acc, ns);
+      if constexpr (RECT != 0) {
+        light_march_rect<QuadT, PREC, RECT == 1>(g, quads, s_tab, PREC ? s_tau : s_a, ray, acc, ns);
       } else {
         // the lanes leave the untested steps together
         const int sure = SKIP ? ray.sure : __reduce_min_sync(lanes, ray.sure);
@@ -434,6 +434,9 @@ __global__ void __launch_bounds__(kThreads) k_view_march_cells(const ExactGeo g,
       float4 sc = make_float4(0.f, 0.f, 0.f, 0.f);
       float bl[3] = {0.f, 0.f, 0.f};
       float inv[3] = {0.f, 0.f, 0.f};
+      unsigned a[3];  // explicit coordinates: the previous cell's entries
+#pragma unroll
+      for (int k = 0; k < 3; ++k) a[k] = cells.tab[k] + (kGuessBias << 4);
       const int n1 = g.tf_n - 1;
       while (inside_vol(g, p) && dist < maxD && budget-- > 0) {
         if (!(min3(tx, ty, tz) >= 0.f && max3(tx, ty, tz) <= 1.f)) {
@@ -441,16 +444,16 @@ __global__ void __launch_bounds__(kThreads) k_view_march_cells(const ExactGeo g,
           if (g.rect) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-              const float4* T = s_tab + g.ax_off[k];
-              float4 e;
+              const unsigned first = cells.tab[k] + (kGuessBias << 4), last = first + ((unsigned)(g.n[k] - 2) << 4);
+              float4 e = ld_shared4(a[k]);
               if (p[k] == g.maxp[k]) {
-                e = T[g.n[k] - 2];
+                e = ld_shared4(a[k] = last);
               } else {
-                find_cell_walk_rect(T, g.n[k] - 2, g.org[k], g.invh[k], g.rect == 1, p[k], e);
+                a[k] = find_cell_rect<true>(first, last, a[k], p[k], e);
                 inv[k] = e.z;
               }
               bl[k] = e.x;
-              cid += __float_as_uint(e.y);
+              cid += ((a[k] - first) >> 4) * g.fs[k];
             }
             tx = (p[0] - bl[0]) * inv[0];
             ty = (p[1] - bl[1]) * inv[1];
@@ -681,7 +684,7 @@ size_t macro_bytes(const int n[3]) {
 }
 
 // One instantiation of K1 over the launch's rays.
-template <typename QuadT, bool STITCH, bool PREC, bool SKIP, bool RECT, bool LIST, bool SPLIT>
+template <typename QuadT, bool STITCH, bool PREC, bool SKIP, int RECT, bool LIST, bool SPLIT>
 static cudaError_t launch_k1_as(const ExactGeo& g, const void* quads, const float4* tab, const float4* tf,
                                 const float* tau, void* map, unsigned nslots, Counters* cnt, cudaStream_t st,
                                 const BrickRef* refs, int nrefs, int self, const unsigned* gate,
@@ -715,20 +718,21 @@ static cudaError_t launch_k1(const ExactGeo& g, const void* quads, const float4*
   if (g.rect) {  // explicit rectilinear coordinates: no empty-space skipping
     if constexpr (!STITCH) {
       occ = nullptr;
-      return vlist ? BEAMS_K1(false, true, true, false) : BEAMS_K1(false, true, false, false);
+      if (g.rect == 1) return vlist ? BEAMS_K1(false, 1, true, false) : BEAMS_K1(false, 1, false, false);
+      return vlist ? BEAMS_K1(false, 2, true, false) : BEAMS_K1(false, 2, false, false);
     } else {
       return cudaErrorInvalidValue;
     }
   }
   if (vlist) {  // a masked build: lazy maps, the learned form's fallback, the multi-brick Phase 1
     if constexpr (STITCH) {
-      return occ ? cudaErrorInvalidValue : BEAMS_K1(false, false, true, false);
+      return occ ? cudaErrorInvalidValue : BEAMS_K1(false, 0, true, false);
     } else {
-      return occ ? BEAMS_K1(true, false, true, false) : BEAMS_K1(false, false, true, false);
+      return occ ? BEAMS_K1(true, 0, true, false) : BEAMS_K1(false, 0, true, false);
     }
   }
-  if (nslots <= split_rays<STITCH, PREC>(g)) return occ ? BEAMS_K1(true, false, false, true) : BEAMS_K1(false, false, false, true);
-  return occ ? BEAMS_K1(true, false, false, false) : BEAMS_K1(false, false, false, false);
+  if (nslots <= split_rays<STITCH, PREC>(g)) return occ ? BEAMS_K1(true, 0, false, true) : BEAMS_K1(false, 0, false, true);
+  return occ ? BEAMS_K1(true, 0, false, false) : BEAMS_K1(false, 0, false, false);
 #undef BEAMS_K1
 }
 

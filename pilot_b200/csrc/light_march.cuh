@@ -342,60 +342,104 @@ __device__ __forceinline__ void light_march_split(const ExactGeo& g, const Light
   if (j == 0) ns += n;
 }
 
-// The same for explicit rectilinear coordinates, where a guess from a uniform
-// spacing only starts the search. vals: s_a (exact) or s_tau (precision).
-template <typename QuadT, bool PREC>
+// The same for explicit rectilinear coordinates, whose entries are {lo, hi, rh, rl}. NEAR
+// (ExactGeo::rect 1): the search walks from the cell that the mean spacing gives. Else it looks
+// at the previous sample's cell and at the next one along the ray, without a branch, and
+// searches on from there. A 160^3 field, 97^3-vertex map: spacings within 35% of their mean
+// 0.30 ms near (0.35 from the previous sample), coordinates i^4 0.26 ms from the previous
+// sample (0.39 walking, 0.56 halving the axis for each sample). Four blocks a SM: at six both
+// spill (0.30 -> 0.39 ms). vals: s_a (exact) or s_tau (precision).
+template <typename QuadT, bool PREC, bool NEAR>
 __device__ __forceinline__ void light_march_rect(const ExactGeo& g, const QuadT* __restrict__ quads,
                                                  const float4* s_tab, const float* vals, const LightRay& ray,
                                                  Accum<PREC>& acc, unsigned& ns) {
   float s[3] = {ray.st[0], ray.st[1], ray.st[2]};
   const int n1 = g.tf_n - 1;
-  unsigned k = 0;
-  for (; k < (unsigned)g.light_budget; ++k) {
-    const bool sure = k < (unsigned)ray.sure;
-    if (!sure) {
-      const float q0 = s[0] - ray.st[0], q1 = s[1] - ray.st[1], q2 = s[2] - ray.st[2];
-      if (!(q0 * q0 + q1 * q1 + q2 * q2 <= ray.len2)) break;
-    }
+  unsigned first[3], a[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) s[d] = s[d] + ray.sd[d];
-    if (!sure && !inside_vol(g, s)) break;
-    float pc[3];
-    int cell[3];
+  for (int d = 0; d < 3; ++d) {
+    first[d] = (unsigned)__cvta_generic_to_shared(s_tab + g.ax_off[d]);
+    if (!NEAR) a[d] = halve_cells_rect<false>(first[d], first[d] + ((unsigned)(g.n[d] - 2) << 4), s[d]);
+  }
+  const auto sample = [&]() -> float {
     float4 e[3];
-    if (g.rect == 1) {
+    if (NEAR) {
+      const float4 *T0 = s_tab + g.ax_off[0], *T1 = s_tab + g.ax_off[1], *T2 = s_tab + g.ax_off[2];
+      const int m0 = g.n[0] - 2, m1 = g.n[1] - 2, m2 = g.n[2] - 2;
+      int c0 = trunc_small(fminf((s[0] - g.org[0]) * g.invh[0], (float)m0));
+      int c1 = trunc_small(fminf((s[1] - g.org[1]) * g.invh[1], (float)m1));
+      int c2 = trunc_small(fminf((s[2] - g.org[2]) * g.invh[2], (float)m2));
+      float4 e0 = T0[c0], e1 = T1[c1], e2 = T2[c2];
+      if ((s[0] <= e0.x) | (s[0] > e0.y) | (s[1] <= e1.x) | (s[1] > e1.y) | (s[2] <= e2.x) | (s[2] > e2.y)) {
+        while (c0 > 0 && s[0] <= e0.x) e0 = T0[--c0];
+        while (c0 < m0 && s[0] > e0.y) e0 = T0[++c0];
+        while (c1 > 0 && s[1] <= e1.x) e1 = T1[--c1];
+        while (c1 < m1 && s[1] > e1.y) e1 = T1[++c1];
+        while (c2 > 0 && s[2] <= e2.x) e2 = T2[--c2];
+        while (c2 < m2 && s[2] > e2.y) e2 = T2[++c2];
+      }
+      e[0] = e0;
+      e[1] = e1;
+      e[2] = e2;
+      a[0] = first[0] + ((unsigned)c0 << 4);
+      a[1] = first[1] + ((unsigned)c1 << 4);
+      a[2] = first[2] + ((unsigned)c2 << 4);
+    } else {
+      bool off = false;
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        cell[d] = trunc_small(fminf((s[d] - g.org[d]) * g.invh[d], (float)(g.n[d] - 2)));
-        e[d] = s_tab[g.ax_off[d] + cell[d]];
+        const bool up = ray.sd[d] > 0.f;
+        const unsigned next = up ? a[d] + 16u : max(a[d] - 16u, first[d]);
+        e[d] = ld_shared4(a[d]);
+        const float4 f = ld_shared4(next);
+        if (up ? s[d] > e[d].y : s[d] <= e[d].x) {
+          a[d] = next;
+          e[d] = f;
+        }
+        off = off | (s[d] <= e[d].x) | (s[d] > e[d].y);
       }
+      if (off) {
 #pragma unroll
-      for (int d = 0; d < 3; ++d) walk_cell_rect(s_tab + g.ax_off[d], g.n[d] - 2, s[d], cell[d], e[d]);
-    } else {
-#pragma unroll
-      for (int d = 0; d < 3; ++d) cell[d] = find_cell_bsearch_rect(s_tab + g.ax_off[d], g.n[d] - 2, s[d], e[d]);
+        for (int d = 0; d < 3; ++d)
+          if ((s[d] <= e[d].x) | (s[d] > e[d].y))
+            a[d] = find_cell_rect<false>(first[d], first[d] + ((unsigned)(g.n[d] - 2) << 4), a[d], s[d], e[d]);
+      }
     }
+    float p[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) pc[d] = div_field(s[d] - e[d].x, e[d]);
-    const unsigned qi = float_bits(e[0].y) + float_bits(e[1].y) + float_bits(e[2].y);
-    const float sum = pc[0] + pc[1] + pc[2];
+    for (int d = 0; d < 3; ++d) p[d] = div_field(s[d] - e[d].x, e[d]);
+    const float sum = p[0] + p[1] + p[2];
     if (sum != sum) {  // an entry whose two-term division is not exact (see field_entry)
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const float4* T = s_tab + g.ax_off[d] + cell[d];
-        pc[d] = (s[d] - T[0].x) / (T[1].x - T[0].x);
-      }
+      for (int d = 0; d < 3; ++d) p[d] = (s[d] - e[d].x) / (e[d].y - e[d].x);
     }
     float v[8];
-    QuadLoad<QuadT>::cell(quads, qi, g.fs[1], g.fs[2], v);
-    float scalar = hex_interp(v, pc[0], pc[1], pc[2]);
-    scalar = (scalar - g.min_scalar) * g.inv_delta;
-    if (acc.add(vals[tf_index_clamped(scalar * (float)n1, n1)])) {
+    QuadLoad<QuadT>::cell(quads, ((a[2] - first[2]) >> 4) * g.fs[2] + ((a[1] - first[1]) >> 4) * g.fs[1] +
+                                     ((a[0] - first[0]) >> 4), g.fs[1], g.fs[2], v);
+    const float scalar = (hex_interp(v, p[0], p[1], p[2]) - g.min_scalar) * g.inv_delta;
+    return vals[tf_index_clamped(scalar * (float)n1, n1)];
+  };
+  int k = 0;
+  for (; k < ray.sure; ++k) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) s[d] = s[d] + ray.sd[d];
+    if (acc.add(sample())) {
+      ns += (unsigned)k + 1u;
+      return;
+    }
+  }
+  for (; k < g.light_budget; ++k) {
+    const float q0 = s[0] - ray.st[0], q1 = s[1] - ray.st[1], q2 = s[2] - ray.st[2];
+    if (!(q0 * q0 + q1 * q1 + q2 * q2 <= ray.len2)) break;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) s[d] = s[d] + ray.sd[d];
+    if (!inside_vol(g, s)) break;
+    if (acc.add(sample())) {
       ++k;
       break;
     }
   }
-  ns += k;
+  ns += (unsigned)k;
 }
 
 }  // namespace beams

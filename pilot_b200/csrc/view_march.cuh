@@ -331,21 +331,24 @@ __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT*
     // max-face rule).
     const float none = __int_as_float(0x7fffffff);
     float bl[3] = {none, none, none}, inv[3] = {0.f, 0.f, 0.f}, t[3] = {none, none, none}, v[8];
+    unsigned a[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) a[k] = T.cells.tab[k] + (kGuessBias << 4);
     for (;;) {
       if (!(min3(t[0], t[1], t[2]) >= 0.f && max3(t[0], t[1], t[2]) <= 1.f)) {
         unsigned off = 0;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          const float4* A = s_tab + g.ax_off[k];
-          float4 e;
+          const unsigned first = T.cells.tab[k] + (kGuessBias << 4), last = first + ((unsigned)(g.n[k] - 2) << 4);
+          float4 e = ld_shared4(a[k]);
           if (p[k] == g.maxp[k]) {
-            e = A[g.n[k] - 2];  // the reference leaves invSpacing[k] unchanged here
+            e = ld_shared4(a[k] = last);  // the reference leaves invSpacing[k] unchanged here
           } else {
-            find_cell_walk_rect(A, g.n[k] - 2, g.org[k], g.invh[k], g.rect == 1, p[k], e);
+            a[k] = find_cell_rect<true>(first, last, a[k], p[k], e);
             inv[k] = e.z;  // 1.f / (coord(c+1) - coord(c)), IEEE
           }
           bl[k] = e.x;
-          off += __float_as_uint(e.y);
+          off += ((a[k] - first) >> 4) * g.fs[k];
           t[k] = (p[k] - bl[k]) * inv[k];
         }
         QuadLoad<QuadT>::cell(quads, off, g.fs[1], g.fs[2], v);

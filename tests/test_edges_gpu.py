@@ -183,3 +183,38 @@ def test_bricks_lit_from_one_of_their_vertices(cuda_device, light):
     nan = np.isnan(oimg)
     assert np.array_equal(np.isnan(img), nan)
     check(np.where(nan, 0, img), np.where(nan, 0, oimg))
+
+
+@pytest.mark.parametrize("kind", ["jitter", "power", "wide"])
+@pytest.mark.parametrize("dims", [(2, 3, 60), (41, 5, 2), (70, 33, 9)], ids=str)
+@pytest.mark.parametrize("steps", [3.0, 40.0, 400.0])
+def test_coordinate_searches_over_short_and_long_steps(cuda_device, kind, dims, steps):
+    """From a fraction of a cell a step to most of the axis, up and down, on axes of a few cells."""
+    rng = np.random.default_rng(sum(dims))
+    t = [np.linspace(0.0, 1.0, n) for n in dims]
+    coords = {"jitter": [np.concatenate([[0.0], (q[1:-1] + rng.uniform(-0.3, 0.3, len(q) - 2) / len(q)), [1.0]]) for q in t],
+              "power": [q ** 4 for q in t],
+              "wide": [np.concatenate([q[:-1] * 1e-2, [1.0]]) for q in t]}[kind]
+    for light in ((0, (2.0, -1.0, 3.0)), (1, (1.0, 0.7, -0.6))):
+        s = dataclasses.replace(scenes.small(52, n=9, image=40, m=7, kind="noise"), dims=dims, light_steps=steps,
+                                array=rng.uniform(0, 1, dims[::-1]).astype(np.float32), sample_distance=2.0 / steps,
+                                light_kind=light[0], light=light[1])
+        s.coords = tuple(np.float32(c) for c in coords)
+        for name, dt in DTYPES[:2]:
+            o = oracle(s, name)
+            om, _ = o.light_march()
+            oimg, lit = o.view_march(om)
+            with renderer(s, dt) as r:
+                img, m, n = frame(r, s)
+                assert np.array_equal(m, om.ravel()) and n[1] == lit, (light, name)
+                check(img, oimg)
+        cells = s.array[:-1, :-1, :-1].copy()
+        oimg, lit = Oracle(s, field=cells).view_march_cells()
+        with B.Renderer(0) as r:
+            r.set_volume(cells, dims=dims, origin=s.origin, spacing=s.spacing, value_range=s.value_range, assoc=B.ASSOC_CELLS)
+            r.set_volume_coordinates(*s.coords)
+            s.configure(r)
+            r.set_use_shadow_map(False)
+            img, t = r.render(s.camera())
+            assert t["lit_samples"] == lit
+            check(img, oimg)
