@@ -409,13 +409,22 @@ cudaError_t launch_view_march_mlp(const ExactGeo& g, const float4* quads, const 
                                   cudaStream_t st) {
   if (knot < 1 || knot > kKnotMax) return cudaErrorInvalidValue;
   if (pass.probes_only && (probe.P < 1 || !probe.rec || !probe.count)) return cudaErrorInvalidValue;
-  const size_t smem = (size_t)g.max_off[0] * sizeof(float4) + (size_t)g.tf_n * sizeof(float4) +
-                      (size_t)kPacked * sizeof(uint2) + (size_t)((kAux + 3) & ~3) * sizeof(float) +
-                      (size_t)8 * knot * 32 * sizeof(unsigned short);
+  const size_t tables = (size_t)g.max_off[0] * sizeof(float4) + (size_t)g.tf_n * sizeof(float4) +
+                        (size_t)kPacked * sizeof(uint2) + (size_t)((kAux + 3) & ~3) * sizeof(float);
+  // Eight warps a block; seven where the axes' closing table entries push the eight warps'
+  // indices past a block's shared memory (a knot of 64 and the longest axes)
+  int warps = 8;
+  size_t smem = tables + (size_t)warps * knot * 32 * sizeof(unsigned short);
   cudaError_t e = cudaFuncSetAttribute(k_view_march_mlp<float4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaErrorInvalidValue) {
+    cudaGetLastError();
+    warps = 7;
+    smem = tables + (size_t)warps * knot * 32 * sizeof(unsigned short);
+    e = cudaFuncSetAttribute(k_view_march_mlp<float4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  }
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_view_march_mlp<float4>, 256, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_view_march_mlp<float4>, 32 * warps, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   int dev = 0, sms = 148;
@@ -423,10 +432,10 @@ cudaError_t launch_view_march_mlp(const ExactGeo& g, const float4* quads, const 
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int ntiles = pass.probes_only ? (probe.nqx * probe.nqy + 31) / 32 : ((g.width + 7) >> 3) * ((g.height + 3) >> 2);
   int grid = sms * per_sm;
-  const int need = (ntiles + 7) / 8;
+  const int need = (ntiles + warps - 1) / warps;
   if (grid > need) grid = need;
   if (grid < 1) return cudaSuccess;
-  k_view_march_mlp<float4><<<grid, 256, smem, st>>>(g, quads, tab, tf, W, aux, enc, lf[0], lf[1], lf[2], knot, out,
+  k_view_march_mlp<float4><<<grid, 32 * warps, smem, st>>>(g, quads, tab, tf, W, aux, enc, lf[0], lf[1], lf[2], knot, out,
                                                     cnt, probe, pass);
   return cudaGetLastError();
 }

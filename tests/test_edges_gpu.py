@@ -146,6 +146,27 @@ def test_hidden_units_that_are_not_numbers_are_off(cuda_device, value):
     assert np.isfinite(out[0]).all() and np.array_equal(out[1], out[0])
 
 
+@pytest.mark.parametrize("ny", [745, 748])
+def test_learned_form_on_the_longest_axes(cuda_device, ny):
+    """A knot of 64 fits beside 9,963 table entries (cells and colours), the axes' closing ones not
+    counted. Bar: on rays of fewer lit samples than the knot, the image of a knot of 63 (which
+    leaves room to spare), bit for bit."""
+    dims = (8192, ny, 2)
+    s = dataclasses.replace(scenes.small(53, n=24, image=40, m=8, kind="noise"), dims=dims, sample_distance=0.03,
+                            array=np.random.default_rng(53).random(dims[::-1], np.float32))
+    s.tf = np.repeat(s.tf, -(-1024 // len(s.tf)), axis=0)[:1024]
+    assert len(s.tf) + sum(dims) - 3 in (9960, 9963)
+    P = np.random.default_rng(53).normal(0, 0.08, M.N_PARAMS).astype(np.float32)
+    out = []
+    with renderer(s) as r:
+        r.mlp_set_params(P)
+        for knot in (63, 64):
+            r.set_form(B.FORM_MLP, B.mlp_options(knot=knot, probe_fraction=0.0))
+            out.append(r.render(s.camera()))
+    assert np.max(out[0][0][..., 3]) > 0 and out[0][1]["lit_samples"] == out[1][1]["lit_samples"]
+    assert np.array_equal(out[1][0], out[0][0])
+
+
 @pytest.mark.parametrize("name,dt", DTYPES[:2], ids=lambda d: str(d))
 @pytest.mark.parametrize("org", [(3.0e5, 0.0, 1.0e3), (4.0e6, 2.5e6, 0.0), (0.0, 3.0e7, 5.0e6)], ids=str)
 def test_positions_rounded_onto_faces(cuda_device, org, name, dt):
