@@ -95,6 +95,34 @@ __device__ __forceinline__ unsigned find_cell_rect(unsigned first, unsigned last
   return a;
 }
 
+// The view march's cells of p among explicit coordinates when a sample leaves its cell: a,
+// the previous cell's entries, become p's and e what they hold. A look at the previous cell
+// and the next one along the step, without a branch; what that does not settle is searched
+// (512^2 views of 160^3 noise, evenly spaced: 1.13 ms walking from the previous cell, 1.03 so).
+__device__ __forceinline__ void locate_view_cell_rect(const ExactGeo& g, const CellTables& C, const float p[3],
+                                                      const float step[3], unsigned a[3], float4 e[3]) {
+  unsigned first[3], last[3];
+  bool off = false;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    first[k] = C.tab[k] + (kGuessBias << 4);
+    last[k] = first[k] + ((unsigned)(g.n[k] - 2) << 4);
+    const bool up = step[k] > 0.f;
+    const unsigned next = up ? min(a[k] + 16u, last[k]) : max(a[k] - 16u, first[k]);
+    e[k] = ld_shared4(a[k]);
+    const float4 f = ld_shared4(next);
+    if (up ? p[k] >= e[k].y : p[k] < e[k].x) {
+      a[k] = next;
+      e[k] = f;
+    }
+    off = off | (p[k] < e[k].x) | (p[k] >= e[k].y);
+  }
+  if (off) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) a[k] = find_cell_rect<true>(first[k], last[k], a[k], p[k], e[k]);
+  }
+}
+
 // The view march's cell location on a uniform grid when a sample leaves its cell
 // (RectilinearLocator::LocateCell, LightedVolumeRenderer.cxx:119-165: the unique
 // c with coord(c) <= p < coord(c+1)), from the guesses b: sets the cell's lower

@@ -295,10 +295,11 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<LIST, RECT>()) k_li
 // ---------------------------------------------------------------------------
 // Four blocks a SM (64 registers): left to itself the compiler takes 78 and three
 // blocks run (1024^2 view of 384^3 bfloat16 3.25 -> 2.86 ms, 512^2 of 128^3 blobs 0.33
-// -> 0.31 ms; five blocks spill: 3.05 and 0.34 ms).
+// -> 0.31 ms; five blocks spill: 3.05 and 0.34 ms). Explicit coordinates need
+// more: at four blocks a 512^2 view of 160^3 noise takes 0.94 ms, at three 0.87.
 template <typename QuadT, bool USE_MAP, typename MapT, bool LIST = false, bool SKIP = false, bool MULTI = false,
           bool RECT = false>
-__global__ void __launch_bounds__(kThreads, 4) k_view_march(const ExactGeo g, const QuadT* __restrict__ quads,
+__global__ void __launch_bounds__(kThreads, RECT ? 3 : 4) k_view_march(const ExactGeo g, const QuadT* __restrict__ quads,
                                                          const float4* __restrict__ tab,
                                                          const float4* __restrict__ tf,
                                                          const MapT* __restrict__ map,
@@ -394,7 +395,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_mark_view_cells(const ExactGeo 
 // ---------------------------------------------------------------------------
 // K2c (cell field, unlit)
 // ---------------------------------------------------------------------------
-template <typename FieldT>
+template <typename FieldT, bool RECT>
 __global__ void __launch_bounds__(kThreads) k_view_march_cells(const ExactGeo g,
                                                                const FieldT* __restrict__ field,
                                                                const float4* __restrict__ tab,
@@ -441,19 +442,14 @@ __global__ void __launch_bounds__(kThreads) k_view_march_cells(const ExactGeo g,
       while (inside_vol(g, p) && dist < maxD && budget-- > 0) {
         if (!(min3(tx, ty, tz) >= 0.f && max3(tx, ty, tz) <= 1.f)) {
           unsigned cid = 0;  // the quads' strides are the cells'
-          if (g.rect) {
+          if (RECT) {
+            float4 e[3];
+            locate_view_cell_rect(g, cells, p, d, a, e);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-              const unsigned first = cells.tab[k] + (kGuessBias << 4), last = first + ((unsigned)(g.n[k] - 2) << 4);
-              float4 e = ld_shared4(a[k]);
-              if (p[k] == g.maxp[k]) {
-                e = ld_shared4(a[k] = last);
-              } else {
-                a[k] = find_cell_rect<true>(first, last, a[k], p[k], e);
-                inv[k] = e.z;
-              }
-              bl[k] = e.x;
-              cid += ((a[k] - first) >> 4) * g.fs[k];
+              if (p[k] != g.maxp[k]) inv[k] = e[k].z;
+              bl[k] = e[k].x;
+              cid += ((a[k] - cells.tab[k] - (kGuessBias << 4)) >> 4) * g.fs[k];
             }
             tx = (p[0] - bl[0]) * inv[0];
             ty = (p[1] - bl[1]) * inv[1];
@@ -967,9 +963,10 @@ cudaError_t launch_view_march_f32(const ExactGeo& g, const float* field, const f
   int grid = 0;
   cudaError_t e;
   if (g.assoc_cells) {
-    e = persistent_grid(k_view_march_cells<float>, smem, ntiles, grid);
+    const auto kernel = g.rect ? k_view_march_cells<float, true> : k_view_march_cells<float, false>;
+    e = persistent_grid(kernel, smem, ntiles, grid);
     if (e != cudaSuccess) return e;
-    k_view_march_cells<float><<<grid, kThreads, smem, st>>>(g, field, tab, tf, out, cnt);
+    kernel<<<grid, kThreads, smem, st>>>(g, field, tab, tf, out, cnt);
   } else if (g.rect && g.n_lights > 1) {
     return cudaErrorInvalidValue;
   } else if (g.use_map && g.n_lights > 1) {

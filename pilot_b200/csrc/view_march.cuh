@@ -337,18 +337,13 @@ __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT*
     for (;;) {
       if (!(min3(t[0], t[1], t[2]) >= 0.f && max3(t[0], t[1], t[2]) <= 1.f)) {
         unsigned off = 0;
+        float4 e[3];
+        locate_view_cell_rect(g, T.cells, p, sd, a, e);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          const unsigned first = T.cells.tab[k] + (kGuessBias << 4), last = first + ((unsigned)(g.n[k] - 2) << 4);
-          float4 e = ld_shared4(a[k]);
-          if (p[k] == g.maxp[k]) {
-            e = ld_shared4(a[k] = last);  // the reference leaves invSpacing[k] unchanged here
-          } else {
-            a[k] = find_cell_rect<true>(first, last, a[k], p[k], e);
-            inv[k] = e.z;  // 1.f / (coord(c+1) - coord(c)), IEEE
-          }
-          bl[k] = e.x;
-          off += ((a[k] - first) >> 4) * g.fs[k];
+          if (p[k] != g.maxp[k]) inv[k] = e[k].z;  // 1.f / (coord(c+1) - coord(c)), IEEE; kept on a max face
+          bl[k] = e[k].x;
+          off += ((a[k] - T.cells.tab[k] - (kGuessBias << 4)) >> 4) * g.fs[k];
           t[k] = (p[k] - bl[k]) * inv[k];
         }
         QuadLoad<QuadT>::cell(quads, off, g.fs[1], g.fs[2], v);
