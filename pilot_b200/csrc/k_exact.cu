@@ -295,11 +295,12 @@ __global__ void __launch_bounds__(kThreads, k1_blocks_per_sm<LIST, RECT>()) k_li
 // ---------------------------------------------------------------------------
 // Four blocks a SM (64 registers): left to itself the compiler takes 78 and three
 // blocks run (1024^2 view of 384^3 bfloat16 3.25 -> 2.86 ms, 512^2 of 128^3 blobs 0.33
-// -> 0.31 ms; five blocks spill: 3.05 and 0.34 ms). Explicit coordinates need
-// more: at four blocks a 512^2 view of 160^3 noise takes 0.94 ms, at three 0.87.
+// -> 0.31 ms; five blocks spill: 3.05 and 0.34 ms). Several lights and explicit coordinates
+// need more: at four blocks 8 lights on 160^3 noise take 2.28 ms and explicit coordinates
+// 0.94, at three 2.14 and 0.87.
 template <typename QuadT, bool USE_MAP, typename MapT, bool LIST = false, bool SKIP = false, bool MULTI = false,
           bool RECT = false>
-__global__ void __launch_bounds__(kThreads, RECT ? 3 : 4) k_view_march(const ExactGeo g, const QuadT* __restrict__ quads,
+__global__ void __launch_bounds__(kThreads, MULTI || RECT ? 3 : 4) k_view_march(const ExactGeo g, const QuadT* __restrict__ quads,
                                                          const float4* __restrict__ tab,
                                                          const float4* __restrict__ tf,
                                                          const MapT* __restrict__ map,
