@@ -402,11 +402,11 @@ __device__ __forceinline__ void view_march_pixel(const ExactGeo& g, const QuadT*
           const unsigned b[3] = {b0, b1, b2};
           const ViewFace f = view_cell_at_face(g, T.cells, cell, p, b);
           cell = f.cell;
-          off = cell.off;
           tx = f.t[0];
           ty = f.t[1];
           tz = f.t[2];
-          QuadLoad<QuadT>::cell(quads, off, g.fs[1], g.fs[2], v);
+          // (512^2 of 160^3 noise 4e6 cells from the origin: 1.03 ms loading again in any case, 1.01 so)
+          if (cell.off != off) QuadLoad<QuadT>::cell(quads, off = cell.off, g.fs[1], g.fs[2], v);
         }
         cell.off = off;
         shade_sample<USE_MAP, MapT, Rec, MULTI>(g, T, s_tab, map, p, view_interp(v, tx, ty, tz), wild, color, lit, rec);
