@@ -65,21 +65,24 @@ __device__ void stage_tables(const ExactGeo& g, int n, float4* s_tab) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) s_tab[i] = table_entry(g, i);
 }
 
-// Vertices are marched in the light-aligned order of k_light_march, columns of
-// 2^kBrickLog2 x 2^kBrickLog2 vertices.
-// A frame of a 128^3 field and map takes 1.19 ms (in row order 1.67), of a 200^3 field
-// with a 100^3 map 1.12 (1.46).
+// COLUMNS: vertices are marched in the light-aligned order of k_light_march, columns of
+// 2^kBrickLog2 x 2^kBrickLog2 vertices, else in rows. The plain field's eight loads a cell
+// take fewer lines with a warp's rays side by side along x, unless the map is about as fine
+// as the field: columns for unsplit maps of at least half as many vertices as the field has
+// points. Light march, mean of six lights, rows and columns: 160^3 field, map cells 64 123
+// and 150 us, 100 291 and 304, 128 536 and 514; 64^3 field, 64 104 and 102, 100 248 and 214.
 constexpr int kBrickLog2 = 3;
-// SPLIT: kSplit lanes a ray, in maps of at most kSplitSlots slots (k_light_march's
-// split, for the same reason): a frame of a 64^3 field with a 32^3 map takes 0.15 ms
-// (unsplit 0.20), one with a 100^3 map, too large, 1.23 (1.13).
+// SPLIT: kSplit lanes a ray, in maps of at most kSplitVertices vertices (k_light_march's
+// split, for the same reason) and in rows: the light march of a 160^3 field with a 40^3
+// map takes 50 us (in columns 63, unsplit 74); a frame with a 100^3 map, too large, of a
+// 64^3 field takes 1.23 ms (unsplit 1.13).
 constexpr int kSplit = 4;
-constexpr unsigned kSplitSlots = 160000;
+constexpr unsigned kSplitVertices = 160000;
 
-// K1: a thread, or kSplit lanes, per slot of the light-aligned vertex order, the
+// K1: a thread, or kSplit lanes, per slot of the vertex order, the
 // light march of k_light_march (light_march, TransmittanceMap.h:279-332) on the
 // plain field, into the scratch map. Alpha / max alpha as GetMaxAlpha (TransmittanceMap.h:515-525).
-template <bool SPLIT>
+template <bool SPLIT, bool COLUMNS>
 __global__ void __launch_bounds__(256) k_noalloc_light_march(const ExactGeo g, const FieldF32* __restrict__ field,
                                                              const float4* __restrict__ tf,
                                                              float* __restrict__ map, unsigned nslots) {
@@ -89,7 +92,7 @@ __global__ void __launch_bounds__(256) k_noalloc_light_march(const ExactGeo g, c
   __shared__ float s_max;
   __shared__ int s_lo[8];
   if (threadIdx.x == 0) {
-    light_order_setup(g, s_lo);
+    if (COLUMNS) light_order_setup(g, s_lo);
     float m = 0.f;
     for (int i = 0; i < g.tf_n; ++i) m = mx(m, tf[i].w);
     s_max = m;
@@ -100,7 +103,15 @@ __global__ void __launch_bounds__(256) k_noalloc_light_march(const ExactGeo g, c
   __syncthreads();
   const unsigned thread = blockIdx.x * blockDim.x + threadIdx.x, slot = SPLIT ? thread / kSplit : thread;
   int x = 0, y = 0, z = 0;
-  const bool active = slot < nslots && light_slot_vertex(slot, kBrickLog2, s_lo, x, y, z);
+  bool active = slot < nslots;
+  if (COLUMNS) {
+    active = active && light_slot_vertex(slot, kBrickLog2, s_lo, x, y, z);
+  } else {
+    const unsigned row = slot / g.pd[0];
+    x = slot % g.pd[0];
+    y = row % g.pd[1];
+    z = row / g.pd[1];
+  }
   if (!SPLIT && !active) return;
   const float V[3] = {vtx_coord(g, 0, x), vtx_coord(g, 1, y), vtx_coord(g, 2, z)};
   float L[3], dir[3];
@@ -273,11 +284,14 @@ extern "C" beams_status beams_render_noalloc(const beams_volume* vol, const floa
   }
   cudaStream_t st = (cudaStream_t)cuda_stream;
   geo_light_order(g, g.light_kind, light_pos);
-  const unsigned nslots = light_slots(g, kBrickLog2);
+  const unsigned nvert = (unsigned)g.pd[0] * (unsigned)g.pd[1] * (unsigned)g.pd[2];
+  const bool split = nvert <= kSplitVertices;
+  const bool columns = !split && 2.0 * nvert >= (double)g.n[0] * g.n[1] * g.n[2];
+  const unsigned nslots = columns ? light_slots(g, kBrickLog2) : nvert;
   const size_t smem1 = (size_t)g.max_off[0] * sizeof(float4) + (size_t)tf_n * sizeof(float);
   const size_t smem2 = ((size_t)g.ntab + (size_t)tf_n) * sizeof(float4);
-  const bool split = nslots <= kSplitSlots;
-  const auto light_march_kernel = split ? k_noalloc_light_march<true> : k_noalloc_light_march<false>;
+  const auto light_march_kernel = split ? k_noalloc_light_march<true, false>
+                                        : (columns ? k_noalloc_light_march<false, true> : k_noalloc_light_march<false, false>);
   e = cudaFuncSetAttribute(light_march_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_noalloc_view_march, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);

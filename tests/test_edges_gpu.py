@@ -16,6 +16,7 @@ from pilot_b200 import beams as B
 from pilot_b200 import scenes
 from test_marches_gpu import DTYPES, LIGHTS, frame, oracle, renderer, same, sparse
 from test_rectilinear_gpu import check
+from test_zz_no_alloc import _render_noalloc, _render_regular
 
 pytestmark = pytest.mark.gpu
 
@@ -239,3 +240,19 @@ def test_coordinate_searches_over_short_and_long_steps(cuda_device, kind, dims, 
             img, t = r.render(s.camera())
             assert t["lit_samples"] == lit
             check(img, oimg)
+
+
+# split rays below 160,000 vertices; else columns where twice the vertices are the field's points
+@pytest.mark.parametrize("dims,m", [((80, 80, 80), 53), ((80, 80, 80), 54), ((53, 71, 97), 55), ((41, 90, 95), 55),
+                                    ((42, 90, 95), 55), ((9, 300, 70), 56), ((90, 90, 90), 70)], ids=str)
+def test_allocation_free_frames_in_each_vertex_order(cuda_device, dims, m):
+    """Bar: the regular entry point's image, bit for bit."""
+    import torch
+    rng = np.random.default_rng(sum(dims))
+    for light in ((2.0, 0.4, 0.5), (0.3, -2.0, 0.9), (0.45, 0.5, 0.4)):
+        s = dataclasses.replace(scenes.small(54, n=9, image=40, m=m, kind="noise"), dims=dims, light_kind=0, light=light,
+                                array=rng.uniform(0, 1, dims[::-1]).astype(np.float32))
+        fd, tf = torch.from_numpy(s.array).cuda(), torch.from_numpy(np.ascontiguousarray(s.tf, np.float32)).cuda()
+        out = torch.full((s.height, s.width, 4), -1.0, device="cuda")
+        assert _render_noalloc(s, fd, tf, out) == 0
+        assert np.array_equal(out.cpu().numpy(), _render_regular(s))
