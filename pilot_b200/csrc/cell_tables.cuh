@@ -53,9 +53,9 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return r;
 }
 
-// Distance in macro-cells (Chebyshev, at most 255) from the macro-cell of the
+// Distance in macro-cells (Chebyshev, at most kMacroFar = 15) from the macro-cell of the
 // guess b to the nearest one that is not empty; 0: it is not empty itself. A
-// macro-cell's emptiness covers a guess off by one cell (k_build_occupancy), and
+// macro-cell's emptiness covers a guess off by one cell (k_macro_empty), and
 // a step count that moves less than 8 (distance - 1) cells on every axis stays in
 // empty macro-cells.
 __device__ __forceinline__ int macro_distance(const ExactGeo& g, const unsigned char* __restrict__ occ, unsigned b0,

@@ -219,7 +219,7 @@ __device__ __forceinline__ int trunc_small(float x) {
 __device__ __forceinline__ float div_field(float x, const float4& e) { return fmaf(x, e.z, x * e.w); }
 
 // The view march's walk (the unique c with coord(c) <= p < coord(c+1)) that
-// settles seeded guesses off by a face, out of line like walk_cells_bsearch.
+// settles seeded guesses off by a face, out of line so that its registers are not the march's.
 static __device__ __noinline__ int walk_cell_view(const float4* T, int cmax, float p, int c) {
   c = min(c, cmax);
   while (c > 0 && p < T[c].x) --c;

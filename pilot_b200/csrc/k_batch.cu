@@ -53,12 +53,9 @@ __device__ __forceinline__ int find_request(const int* off, int n, int item) {
 }
 
 // MODE 0: map and view items in one launch; 1: map items only; 2: view items only.
-// Four blocks per SM in every mode. The one-launch kernel (MODE 0) holds both
-// marches' registers, so its light march issues one sample at a time (no
-// two-sample pipeline, which it would otherwise use with SKIP): 64 registers,
-// 8 bytes of spills with SKIP. On 64 mixed requests that took the one-launch
-// plan from 98.0 ms (three blocks per SM, the pipelined skipping march) to
-// 86.7 ms, below one render at a time (88.1 ms).
+// Four blocks per SM in every mode (64 registers; the one-launch kernel, MODE 0, holds
+// both marches). 64 mixed requests: 54.0 ms in one launch, 51.7 in two, 50.6 as single
+// renders one after the other.
 template <bool SKIP, int MODE>
 __global__ void __launch_bounds__(kBatchThreads, 4) k_batch(const ExactGeo* __restrict__ geos,
                                                             const BatchDesc* __restrict__ descs,

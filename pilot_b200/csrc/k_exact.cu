@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256) k_mark_cell_blocks(const ExactGeo g, cons
 }
 
 // The work list of a masked map build: the vertices of marked cells
-// (vertex_in_marked_cell) in the light march's vertex order, list[1 + i] their
+// (vertex_in_marked_cell) by 8^3 vertex bricks along the light, list[1 + i] their
 // ids, list[0] their count (zeroed before the launch). A masked build over this
 // list takes one tile-counter atomic per 32 listed vertices, where testing every
 // vertex took one per 32 vertices of the whole map (the 257^3-vertex map of a

@@ -32,13 +32,13 @@ struct NoRecord {
 };
 
 // A view-march observer that marks, for every lit sample of premultiplied
-// alpha above 0, the map cell that the shading looks up (the cell of
-// map_interp_t: truncate min(max((p - origin) / spacing, 0), pd - 2) per axis),
-// one byte per cell, skipping repeats of the previous sample's cell. A sample
-// of alpha 0 adds exactly 0 times its shading, so the map value it reads only
-// has to be finite (the masked builds zero a newly allocated map). A masked map build then lists every vertex with a marked cell
-// around it (the same vertex set as marking the 8 corners, with one store per
-// cell).
+// alpha above 0, the map cell that the shading looks up (map_cell's: truncate
+// min(max((p - origin) / spacing, 0), pd - 2) per axis), one byte per cell,
+// skipping repeats of the previous sample's cell. A sample of alpha 0 adds
+// exactly 0 times its shading, so the map value it reads only has to be finite
+// (the masked builds zero a newly allocated map). A masked map build then lists
+// every vertex with a marked cell around it (the same vertex set as marking the
+// 8 corners, with one store per cell).
 struct CellMarker {
   float morig[3], minv[3];
   int pd[3];
